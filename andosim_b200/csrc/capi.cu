@@ -71,7 +71,6 @@ struct ando_ctx_s {
   double mu = 0, thickness = 0, density = 0;
   int el_semantics = -1;
   bool mesh_ready = false, state_ready = false;
-  int pcg_grid = 1;
 
   DevBuf<int> tris, rowptr, cols, slot_row, diag_slot, face_slot, slot_cptr, slot_contrib, vf_ptr, vf;
   DevBuf<double> rest_area, dm_inv, mass, el_a, el_b, g_el, mesh_x;
@@ -84,7 +83,7 @@ struct ando_ctx_s {
   DevBuf<unsigned char> sflags;
   DevBuf<StrainSV> sv;
   DevBuf<Ctrl> ctrl;
-  DevBuf<double> partials;
+  DevBuf<XrSlot> xr_slots;         // reduction slots of the PCG kernels (common.cuh)
   Ctrl* ctrl_host = nullptr;
 
   // block-scaled system of the CORRECTED step (L = chol(A_ii), A^ = L^-1 A L^-T)
@@ -136,6 +135,10 @@ struct ando_ctx_s {
   int nx_raw = 0;
   DevBuf<ContactEntry> ents, ents_sorted, xent;
   DevBuf<float> xval;
+  // SELL-32 copy of the scaled contact blocks (resident PCG)
+  DevBuf<int> xs_width, xs_off, xs_col;
+  DevBuf<float> xs_val;
+  bool xs_ready = false;
   int nx = 0, nent = 0;
   DevBuf<unsigned char> cub_tmp;
 
@@ -445,6 +448,7 @@ int prepare_contacts(ando_ctx c, const StepParams& sp, const double* g_base, con
   Phase ph(c, ANDO_PHASE_SETUP);
   MeshDev m = c->mesh_dev();
   int nc = c->ncontacts, V = c->V;
+  c->xs_ready = false;
   if (nc) { launch_contact_prep(m, c->contacts.p, nc, sp, c->stream); ph.launched(); }
   int ne = 16 * nc;
   c->nent = ne;
@@ -513,6 +517,11 @@ int prepare_contacts(ando_ctx c, const StepParams& sp, const double* g_base, con
   c->nx = nu;
   launch_vertex_ranges(c->xrow.p, nu, V, c->xbegin.p, c->xend.p, c->stream);
   ph.launched();
+  if (nu && sp.semantics == ANDO_SEMANTICS_CORRECTED && pcg_resident(V)) {
+    CK(c->xs_width.reserve((V + 31) / 32)); CK(c->xs_off.reserve((V + 31) / 32 + 1));
+    launch_x_layout(V, c->xbegin.p, c->xend.p, 6ll * nu + 65536, c->xs_width.p, c->xs_off.p, c->ctrl.p, c->stream);
+    ph.launched(2);
+  }
   CK(cudaGetLastError());
   return ANDO_OK;
 }
@@ -562,7 +571,7 @@ int inner_newton(ando_ctx c, const ando_params& p, const StepParams& sp, ando_st
   pa.V = c->V; pa.rowptr = c->rowptr.p; pa.cols = c->cols.p; pa.val = c->val.p;
   pa.xbegin = c->nx ? c->xbegin.p : nullptr; pa.xend = c->nx ? c->xend.p : nullptr; pa.xcols = c->xcols.p; pa.xval = c->xval.p;
   pa.P = c->precond.p; pa.b = c->b.p; pa.x = c->d.p; pa.r = c->r.p; pa.z = c->z.p; pa.p0 = c->p0.p; pa.p1 = c->p1.p; pa.Ap = c->Ap.p;
-  pa.partials = c->partials.p; pa.ctrl = c->ctrl.p; pa.tol = float(p.pcg_tol); pa.max_iters = p.pcg_max_iters;
+  pa.slots = c->xr_slots.p; pa.ctrl = c->ctrl.p; pa.tol = float(p.pcg_tol); pa.max_iters = p.pcg_max_iters;
   for (int it = 0; it < max_it; ++it) {
     if (sp.enable_strain) {
       Phase ph(c, ANDO_PHASE_STRAIN);
@@ -586,7 +595,7 @@ int inner_newton(ando_ctx c, const ando_params& p, const StepParams& sp, ando_st
     }
     {
       Phase ph(c, ANDO_PHASE_PCG);
-      CK(launch_pcg(pa, c->pcg_grid, c->stream));
+      CK(launch_pcg(pa, c->stream));
       ph.launched();
     }
     {
@@ -809,7 +818,8 @@ void enqueue_scaled_assembly_tpb(ando_ctx c, const StepParams& sp, cudaStream_t 
                          tpb, c->chunk_off.p, c->sell_wmax);
 }
 
-void enqueue_scaled_assembly(ando_ctx c, const StepParams& sp, cudaStream_t s) {
+// Reads the control block's host copy (xs_blocks of this Newton iteration).
+int enqueue_scaled_assembly(ando_ctx c, const StepParams& sp, cudaStream_t s) {
   if (c->asm_V != c->V) {
     c->asm_V = c->V;
     c->asm_tpb = c->asm_choice >= 0 ? ASM_TPB[c->asm_choice] : 256;
@@ -833,14 +843,27 @@ void enqueue_scaled_assembly(ando_ctx c, const StepParams& sp, cudaStream_t s) {
     if (e1) cudaEventDestroy(e1);
   }
   enqueue_scaled_assembly_tpb(c, sp, s, c->asm_tpb);
-  if (c->nx) launch_extra_merge(c->contacts.p, c->xent.p, c->xk1.p, c->xi1.p, c->xheads.p, c->nx, c->nx_raw, c->fixed.p, sp, c->Linv.p,
-                                nullptr, nullptr, nullptr, c->xvalh.p, s);
+  if (!c->nx) return ANDO_OK;
+  // the layout's size came with the control block of this Newton iteration
+  XsLayout xs;
+  const int places = c->ctrl_host->xs_blocks;
+  c->xs_ready = pcg_resident(c->V) && places > 0;
+  if (c->xs_ready) {
+    CK(c->xs_col.reserve(places)); CK(c->xs_val.reserve(9ull * places));
+    CK(cudaMemsetAsync(c->xs_col.p, 0xff, sizeof(int) * size_t(places), s));
+    xs.off = c->xs_off.p; xs.begin = c->xbegin.p; xs.col = c->xs_col.p; xs.val = c->xs_val.p;
+  }
+  launch_extra_merge(c->contacts.p, c->xent.p, c->xk1.p, c->xi1.p, c->xheads.p, c->nx, c->nx_raw, c->fixed.p, sp, c->Linv.p,
+                     nullptr, nullptr, nullptr, c->xvalh.p, s, xs);
+  return ANDO_OK;
 }
 
 PcgScaledArgs scaled_args(ando_ctx c, const ando_params& p) {
   PcgScaledArgs a;
   a.V = c->V; a.chunk_off = c->chunk_off.p; a.sell_col = c->sell_col.p; a.valh = c->valh_sell.p;
   a.xbegin = c->nx ? c->xbegin.p : nullptr; a.xend = c->nx ? c->xend.p : nullptr; a.xcols = c->xcols.p; a.xvalh = c->xvalh.p;
+  a.xs_off = c->nx && c->xs_ready ? c->xs_off.p : nullptr; a.xs_col = c->xs_col.p; a.xs_val = c->xs_val.p;
+  a.wmax = c->sell_wmax; a.slots_red = c->xr_slots.p;
   a.coef = nullptr; a.Sdiag = nullptr; a.Linv = c->Linv.p; a.Lf = c->Lf.p; a.bhat = c->bhat.p; a.d = c->d.p;
   a.xh = c->xh.p; a.r = c->r.p; a.r2 = c->r2.p; a.z = c->z.p; a.p0 = c->p0.p; a.p1 = c->p1.p; a.Ap = c->Ap.p;
   a.partials = c->spart.p; a.ctrl = c->ctrl.p; a.tol = float(p.pcg_tol); a.max_iters = p.pcg_max_iters; a.stall_window = 50;
@@ -867,7 +890,7 @@ int ensure_learned(ando_ctx c) {
   }
   CK(c->Sval.reserve(9ull * c->nnzb));
   CK(c->S_coef.reserve(c->sell_blocks));
-  CK(c->S_diag.reserve(9ull * c->V));
+  CK(c->S_diag.reserve(288ull * ((c->V + 31) / 32)));
   return ANDO_OK;
 }
 
@@ -1002,7 +1025,8 @@ int inner_newton_corrected(ando_ctx c, const ando_params& p, const StepParams& s
       Phase ph(c, ANDO_PHASE_ASSEMBLE);
       c->write_val = c->keep_system;                       // unscaled copy only for ando_last_system
       c->write_valh = p.precond == ANDO_PRECOND_LEARNED;   // CSR-ordered scaled copy: the network's features
-      enqueue_scaled_assembly(c, sp, s);
+      rc = enqueue_scaled_assembly(c, sp, s);
+      if (rc) return rc;
       ph.launched(c->nx ? 3 : 2);
     }
     rc = scaled_solve(c, p, st);
@@ -1102,7 +1126,7 @@ void enqueue_reference_iteration(ando_ctx c, const ando_params& p, const StepPar
                   c->ebegin.p, c->eend.p, sp, nullptr, c->g.p, c->b.p, c->diag_extra.p, c->ctrl.p, s);
   launch_check(c->ctrl.p, p.pcg_tol, s);
   launch_assemble(m, c->sflags.p, c->sv.p, c->diag_extra.p, sp.enable_strain, nullptr, c->val.p, c->precond.p, c->ctrl.p, s);
-  cudaError_t e = launch_pcg(pa, c->pcg_grid, s);
+  cudaError_t e = launch_pcg(pa, s);
   if (e != cudaSuccess && err == cudaSuccess) err = e;
   if (ls_wall) launch_ls_wall(c->V, c->x.p, c->d.p, wall, c->ctrl.p, s);
   launch_update(c->V, c->x.p, c->d.p, c->ctrl.p, s);
@@ -1123,7 +1147,7 @@ int capture_frame(ando_ctx c, const ando_params& p, const StepParams& sp, bool l
   pa.V = c->V; pa.rowptr = c->rowptr.p; pa.cols = c->cols.p; pa.val = c->val.p;
   pa.xbegin = nullptr; pa.xend = nullptr; pa.xcols = c->xcols.p; pa.xval = c->xval.p;
   pa.P = c->precond.p; pa.b = c->b.p; pa.x = c->d.p; pa.r = c->r.p; pa.z = c->z.p; pa.p0 = c->p0.p; pa.p1 = c->p1.p; pa.Ap = c->Ap.p;
-  pa.partials = c->partials.p; pa.ctrl = c->ctrl.p; pa.tol = float(p.pcg_tol); pa.max_iters = p.pcg_max_iters;
+  pa.slots = c->xr_slots.p; pa.ctrl = c->ctrl.p; pa.tol = float(p.pcg_tol); pa.max_iters = p.pcg_max_iters;
   MeshDev m = c->mesh_dev();
   cudaGraph_t full = nullptr, tmp = nullptr;
   int depth = 0;   // open captures, closed on failure
@@ -1377,8 +1401,7 @@ int32_t ando_ctx_create(int32_t device, ando_ctx* out) {
   if (e == cudaSuccess) e = c->ctrl.reserve(1);
   if (e == cudaSuccess) e = cudaMemset(c->ctrl.p, 0, sizeof(Ctrl));
   if (e != cudaSuccess) { delete c; return fail(ANDO_ERR_CUDA, cudaGetErrorString(e)); }
-  c->pcg_grid = pcg_grid_size(device);
-  e = c->partials.reserve(3ull * std::max(c->pcg_grid, 1));
+  e = c->xr_slots.reserve(XR_SLOTS);
   if (e != cudaSuccess) { delete c; return fail(ANDO_ERR_CUDA, cudaGetErrorString(e)); }
   *out = c;
   return ANDO_OK;
@@ -1822,7 +1845,12 @@ int32_t ando_eval_system(ando_ctx c, const ando_params* params, const ando_pin* 
     c->solve_first = false;
     if (rc) return rc;
     c->write_val = c->write_valh = true;   // the system is read back (tests, training data)
-    enqueue_scaled_assembly(c, sp, s);
+    if (c->nx) {
+      CK(cudaMemcpyAsync(c->ctrl_host, c->ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+    }
+    rc = enqueue_scaled_assembly(c, sp, s);
+    if (rc) return rc;
     c->val_valid = true;
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));

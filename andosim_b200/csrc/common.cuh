@@ -125,13 +125,13 @@ struct Ctrl {
   double pcg_rel;
   double alpha;
   int strain_active;
-  unsigned int bar_count, bar_gen; int bar_err;
+  int bar_err;                    // a bounded wait of the PCG gave up
   int tc_err;                     // a tensor-core GEMM's bounded wait gave up (sticky)
   int toi_overflow;               // > 0: a time-of-impact candidate list needed this many slots; the move was not applied
   int learned_iters;              // iterations of this Newton iteration's learned solve
   int fallback_ran;               // block-Jacobi redid this Newton iteration's learned solve
-  int pad_;
-  unsigned long long bar_arrivals;  // grid_sync_ar: arrivals since the launcher zeroed it
+  int xs_blocks;                  // block places of the contact blocks' SELL-32 copy (-1: too uneven)
+  unsigned long long bar_arrivals;  // xr_reduce (and grid_sync_ar): arrivals since the launcher zeroed it
 };
 
 // PCG_PRECOND: the learned preconditioner lost positive definiteness
@@ -149,43 +149,11 @@ struct StepCtl {
   int iterations_run, inner_steps;    // Newton bodies and inner steps executed (launch accounting)
 };
 
-// Bounded grid barrier for cooperative launches. All CTAs of the grid must be
-// co-resident (cudaLaunchCooperativeKernel guarantees it). A CTA that waits
-// more than `limit` polls sets *err and every CTA leaves; callers check the
-// return value and bail out uniformly.
-__device__ inline bool grid_sync(unsigned int* count, unsigned int* gen, int* err, unsigned int nblocks) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned int* vgen = gen;
-    volatile int* verr = err;
-    unsigned int g = *vgen;
-    __threadfence();
-    unsigned int arrived = atomicAdd(count, 1u);
-    if (arrived == nblocks - 1) {
-      atomicExch(count, 0u);
-      __threadfence();
-      atomicAdd(gen, 1u);
-    } else {
-      long long polls = 0;
-      const long long limit = 1ll << 24;  // ~seconds with backoff
-      while (*vgen == g) {
-        if (*verr) break;
-        if (++polls > limit) { atomicExch(err, 1); break; }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  volatile int* verr = err;
-  return *verr == 0;
-}
-
 // Bounded grid barrier with acquire/release atomics: every CTA adds one
 // arrival to a 64-bit counter that the launcher zeroed (release: the CTA's
 // writes, ordered before the arrival by __syncthreads, are published) and
 // polls with acquire loads until all nblocks CTAs have arrived `epoch` times.
-// About half the cost of grid_sync's full fences. The polling thread hands
+// The polling thread hands
 // its verdict to the CTA through shared memory, so the other threads leave
 // the barrier without another L2 round trip. A CTA that passed a barrier
 // while another CTA was giving up on it meets the error flag in the poll of
@@ -212,6 +180,162 @@ __device__ inline bool grid_sync_ar(unsigned long long* arrivals, unsigned int n
   }
   __syncthreads();
   return passed != 0;
+}
+
+// ------------------------------------------------ PCG reductions across CTAs
+// A PCG iteration is two dot products with a barrier each. These reductions
+// are the barrier: every CTA hands over its partial sum (and maximum) with its
+// arrival and leaves with the total of one partial per CTA.
+//
+// Grid form (cooperative launch, at most XR_MAX_CTAS CTAs): a CTA writes its
+// partial and adds one arrival to a 64-bit counter that the launcher zeroed
+// (release: the CTA's writes, ordered before the arrival by __syncthreads, are
+// published); one thread polls the counter (acquire) and its warp then reads
+// all partials. They alternate between two sets: a CTA writes set s again only
+// after a reduction that every CTA has entered, so nobody still reads it. The
+// polls are bounded; on timeout the error flag makes the other CTAs leave
+// their next wait, and the host reads the flag after the launch. Measured
+// alone, 148 CTAs of 896 threads: 2.25 us; polling one flagged slot per CTA
+// instead of the counter 3.4 us (148 x 148 reads of the same lines), two
+// levels of such slots 2.0 us without and 2.8 us with the publication,
+// clusters of 8 handing one partial each 2.6 us.
+//
+// Cluster form (cl_reduce, the whole launch is one cluster of at most 16
+// CTAs): each CTA leaves its partial in its own shared memory, the cluster
+// barrier follows, and one warp of each CTA reads the others'. The barrier's
+// release waits for every outstanding store of the thread: 360 to 500 cycles
+// with shared-memory stores, 900 to 2,000 behind global ones; with a release
+// restricted to the CTA's own shared memory it takes 100 to 280. So the
+// cluster form publishes its vectors in shared memory and writes no global
+// memory between its barriers.
+//
+// In both forms one thread of each CTA turns the total into the iteration's
+// scalar (`tail`) and the others read that from shared memory: the FP64
+// divisions and the state of the stopping test take no registers of theirs.
+// The partials are added in an order that depends on the numbers of CTAs and
+// slices only.
+constexpr int XR_MAX_CTAS = 160;
+constexpr int XR_MAX_SLICES = 96;   // 32-row slices of one CTA whose partials fit its shared array
+struct alignas(16) XrSlot { double v; unsigned m, pad; };
+constexpr size_t XR_SLOTS = 2ull * XR_MAX_CTAS;
+
+struct XrSmem {
+  double part[XR_MAX_SLICES];
+  unsigned pmax[XR_MAX_SLICES];
+  XrSlot mine[2];                   // cluster form: this CTA's partial
+};
+
+__device__ inline double xr_warp_sum(double v) {
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// |v| as bits whose unsigned order is the order of the magnitudes; a NaN
+// counts as 0 (fmax drops it)
+__device__ inline unsigned xr_mag(float v) { return v == v ? __float_as_uint(fabsf(v)) : 0u; }
+
+// Sum of part[0, n) and max of pmax[0, n) over the calling warp's lanes; the
+// total is lane 0's. (Lanes past n hold zeros, so up to 32 entries need only
+// log2(n) exchanges.)
+__device__ inline void xr_block_total(const XrSmem& sh, int n, double& v, unsigned& m) {
+  const int l = threadIdx.x & 31;
+  v = 0.0; m = 0u;
+  for (int k = l; k < n; k += 32) { v += sh.part[k]; m = max(m, sh.pmax[k]); }
+  for (int o = n > 16 ? 16 : n > 8 ? 8 : n > 4 ? 4 : n > 2 ? 2 : n > 1 ? 1 : 0; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  m = __reduce_max_sync(0xffffffffu, m);
+}
+
+// Total over all CTAs of the partials that the warps left in sh.part / sh.pmax
+// (n slices of this CTA; written before this call, no barrier needed). Writes
+// to global memory made by any thread of the grid before the call are visible
+// to every thread after it. `epoch`: this is the epoch-th reduction of the
+// launch, from 1. One thread calls tail(ok, sum, max); what it writes to
+// shared memory is visible to the CTA afterwards. ok: no wait gave up. Called
+// by all threads.
+template <class Tail>
+__device__ inline void xr_reduce(XrSmem& sh, int n, unsigned epoch, XrSlot* slots, unsigned long long* arrivals, int* err, Tail tail) {
+  __syncthreads();
+  const int nb = gridDim.x;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    double v; unsigned m;
+    xr_block_total(sh, n, v, m);
+    XrSlot* set = slots + (epoch & 1u) * XR_MAX_CTAS;
+    bool good = true;
+    if (lane == 0) {
+      *reinterpret_cast<uint4*>(set + blockIdx.x) = make_uint4((unsigned)__double2loint(v), (unsigned)__double2hiint(v), m, 0u);
+      const unsigned long long target = (unsigned long long)epoch * (unsigned)nb;
+      asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(arrivals) : "memory");
+      long long polls = 0;
+      while (true) {
+        unsigned long long c;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(arrivals) : "memory");
+        if (c >= target) break;
+        if ((++polls & 1023) == 0) {
+          if (*(volatile int*)err) { good = false; break; }
+          if (polls > (1ll << 24)) { atomicExch(err, 1); good = false; break; }
+        }
+      }
+    }
+    __syncwarp();
+    v = 0.0; m = 0u;
+#pragma unroll
+    for (int k = 0; k < XR_MAX_CTAS / 32; ++k) {
+      const int s = lane + 32 * k;
+      if (s < nb) {
+        const uint4 q = __ldcg(reinterpret_cast<const uint4*>(set + s));   // written by other CTAs: read from L2
+        v += __hiloint2double((int)q.y, (int)q.x);
+        m = max(m, q.z);
+      }
+    }
+    v = xr_warp_sum(v);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) tail(good, v, m);
+  }
+  __syncthreads();
+}
+
+__device__ inline unsigned cl_size() { unsigned r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
+// Cluster barrier that orders the CTAs' own shared-memory writes before it with any CTA's reads of them after it.
+__device__ inline void cl_sync_shared() {
+  asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\t"
+               "barrier.cluster.arrive.relaxed;\n\t"
+               "barrier.cluster.wait.acquire;\n\t"
+               "fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+}
+// shared::cluster address of a location of this CTA's shared memory in CTA `rank`
+__device__ inline unsigned cl_map(unsigned addr, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// xr_reduce over a cluster: shared-memory writes of any thread of the cluster
+// before the call are visible to every thread after it. No CTA may leave the
+// kernel before a further cl_sync_shared (others still read its partial).
+template <class Tail>
+__device__ inline void cl_reduce(XrSmem& sh, int n, unsigned epoch, Tail tail) {
+  __syncthreads();
+  const int lane = threadIdx.x & 31, par = epoch & 1u;
+  if (threadIdx.x < 32) {
+    double v; unsigned m;
+    xr_block_total(sh, n, v, m);
+    if (lane == 0) sh.mine[par] = XrSlot{v, m, 0u};
+  }
+  cl_sync_shared();
+  if (threadIdx.x < 32) {
+    const int C = (int)cl_size();
+    double v = 0.0;
+    unsigned m = 0u;
+    if (lane < C) {
+      unsigned lo, hi, z;
+      const unsigned at = cl_map((unsigned)__cvta_generic_to_shared(&sh.mine[par]), lane);
+      asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(lo), "=r"(hi), "=r"(m), "=r"(z) : "r"(at) : "memory");
+      v = __hiloint2double((int)hi, (int)lo);
+    }
+    for (int o = C > 8 ? 8 : C > 4 ? 4 : C > 2 ? 2 : C > 1 ? 1 : 0; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) tail(true, v, m);
+  }
+  __syncthreads();
 }
 
 }  // namespace ando

@@ -415,7 +415,7 @@ __global__ void k_extra_flags(const ContactEntry* ents, const int* keys, int n, 
 __global__ void k_ctrl_reset(Ctrl* c) {
   c->gnorm_bits = 0ull; c->ls_mask = (1u << 20) - 1u; c->converged = 0;
   c->pcg_iters = 0; c->pcg_converged = 0; c->pcg_status = PCG_SKIPPED; c->pcg_rel = 0.0;
-  c->alpha = 0.0; c->strain_active = 0; c->bar_count = 0; c->bar_err = 0;
+  c->alpha = 0.0; c->strain_active = 0; c->bar_err = 0; c->bar_arrivals = 0ull;
   c->learned_iters = 0; c->fallback_ran = 0;
 }
 
@@ -1024,9 +1024,38 @@ __global__ void k_run_heads(const unsigned long long* key, int n, int* flags) {
   if (k >= n) return;
   flags[k] = (k == 0 || key[k] != key[k - 1]) ? 1 : 0;
 }
+// SELL-32 layout of the merged blocks for the resident PCG: a slice of 32 rows
+// is as wide as its row with the most blocks. The scan of the slice widths is
+// one CTA (a mesh of the resident form has at most 4,736 slices). A layout
+// whose padding would exceed `limit` block places (a few rows with very many
+// contacts) is reported as -1 and not used.
+__global__ void k_x_widths(int V, const int* begin, const int* end, int* width) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = __reduce_max_sync(0xffffffffu, v < V ? end[v] - begin[v] : 0);
+  if ((threadIdx.x & 31) == 0 && v < V) width[v >> 5] = n;
+}
+__global__ void __launch_bounds__(1024) k_x_scan(int ns, const int* width, long long limit, int* off, Ctrl* ctrl) {
+  __shared__ long long part[32];
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  long long carry = 0;
+  for (int base = 0; base < ns; base += 1024) {
+    const int i = base + threadIdx.x;
+    const long long mine = i < ns ? 32ll * width[i] : 0;
+    long long v = mine;
+    for (int o = 1; o < 32; o <<= 1) { const long long u = __shfl_up_sync(0xffffffffu, v, o); if (l >= o) v += u; }
+    if (l == 31) part[w] = v;
+    __syncthreads();
+    long long before = carry, all = 0;
+    for (int k = 0; k < 32; ++k) { if (k < w) before += part[k]; all += part[k]; }
+    if (i < ns) off[i] = int(min(before + v - mine, limit));
+    carry += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) { off[ns] = int(min(carry, limit)); ctrl->xs_blocks = carry <= limit ? int(carry) : -1; }
+}
 __global__ void k_extra_merge(const ContactDev* cs, const ContactEntry* xent, const unsigned long long* key, const int* idx, const int* heads,
                               int nu, int n, const unsigned char* fixed, StepParams p, const double* Linv, int* xrow, int* xcols,
-                              float* xval, float* xvalh) {
+                              float* xval, float* xvalh, XsLayout xs) {
   int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= nu) return;
   int k0 = heads[u], k1 = u + 1 < nu ? heads[u + 1] : n;
@@ -1054,6 +1083,12 @@ __global__ void k_extra_merge(const ContactDev* cs, const ContactEntry* xent, co
     if (zero) for (int q = 0; q < 9; ++q) R[q] = 0.0;
     else scale_block(ld_tri(Linv, row), H, ld_tri(Linv, col), R);
     for (int q = 0; q < 9; ++q) xvalh[9 * (long long)u + q] = float(R[q]);
+    if (xs.off) {
+      const long long base = xs.off[row >> 5] + 32 * (u - xs.begin[row]);
+      const int l = row & 31;
+      xs.col[base + l] = col;
+      for (int q = 0; q < 9; ++q) xs.val[9 * base + 32 * q + l] = float(R[q]);
+    }
   }
 }
 
@@ -1465,10 +1500,14 @@ void launch_extra_key64(const ContactEntry* xent, const int* xkeys, int n, unsig
 void launch_run_heads(const unsigned long long* key, int n, int* flags, cudaStream_t s) {
   if (n) k_run_heads<<<nblk(n), TPB, 0, s>>>(key, n, flags);
 }
+void launch_x_layout(int V, const int* begin, const int* end, long long limit, int* width, int* off, Ctrl* ctrl, cudaStream_t s) {
+  k_x_widths<<<nblk(V), TPB, 0, s>>>(V, begin, end, width);
+  k_x_scan<<<1, 1024, 0, s>>>((V + 31) / 32, width, limit, off, ctrl);
+}
 void launch_extra_merge(const ContactDev* c, const ContactEntry* xent, const unsigned long long* key, const int* idx, const int* heads, int nu,
                         int n, const unsigned char* fixed, const StepParams& p, const double* Linv, int* xrow, int* xcols, float* xval,
-                        float* xvalh, cudaStream_t s) {
-  if (nu) k_extra_merge<<<nblk(nu), TPB, 0, s>>>(c, xent, key, idx, heads, nu, n, fixed, p, Linv, xrow, xcols, xval, xvalh);
+                        float* xvalh, cudaStream_t s, XsLayout xs) {
+  if (nu) k_extra_merge<<<nblk(nu), TPB, 0, s>>>(c, xent, key, idx, heads, nu, n, fixed, p, Linv, xrow, xcols, xval, xvalh, xs);
 }
 void launch_ls_wall(int V, const double* x, const float* d, WallDev w, Ctrl* ctrl, cudaStream_t s) {
   if (V) k_ls_wall<<<nblk(V), TPB, 0, s>>>(V, x, d, w, ctrl);

@@ -66,9 +66,15 @@ void launch_assemble_scaled(const MeshDev& m, const unsigned char* sflags, const
                             const int* chunk_off = nullptr, int wmax = 0);
 void launch_extra_key64(const ContactEntry* xent, const int* xkeys, int n, unsigned long long* key, int* idx, cudaStream_t s);
 void launch_run_heads(const unsigned long long* key, int n, int* flags, cudaStream_t s);
+// SELL-32 copy of the merged scaled blocks for the resident PCG: slice offsets
+// (32 x width), columns (-1: padding, set by the caller) and 9 planes of 32
+// lanes per slot; begin = first block of each row
+struct XsLayout { const int* off = nullptr; const int* begin = nullptr; int* col = nullptr; float* val = nullptr; };
+// its slice widths and offsets; ctrl->xs_blocks = places in all, -1 when over `limit`
+void launch_x_layout(int V, const int* begin, const int* end, long long limit, int* width, int* off, Ctrl* ctrl, cudaStream_t s);
 void launch_extra_merge(const ContactDev* c, const ContactEntry* xent, const unsigned long long* key, const int* idx, const int* heads, int nu,
                         int n, const unsigned char* fixed, const StepParams& p, const double* Linv, int* xrow, int* xcols, float* xval,
-                        float* xvalh, cudaStream_t s);
+                        float* xvalh, cudaStream_t s, XsLayout xs = XsLayout{});
 void launch_ls_wall(int V, const double* x, const float* d, WallDev w, Ctrl* ctrl, cudaStream_t s);
 void launch_ls_contacts(const ContactDev* c, int nc, const double* x, const float* d, Ctrl* ctrl, cudaStream_t s);
 void launch_update(int V, double* x, const float* d, Ctrl* ctrl, cudaStream_t s);
@@ -110,12 +116,17 @@ struct PcgArgs {
   const int* xbegin; const int* xend; const int* xcols; const float* xval;  // extra contact segment
   const float* P;     // block-Jacobi inverse, 9V
   const float* b;
+  // z, p0 and p1: float4 rows (4V floats, 16-byte aligned) up to the largest
+  // system whose rows' state fits the registers, packed rows (3V) above it,
+  // where r and Ap (3V each) are used as well (pcg_packed_rows)
   float *x, *r, *z, *p0, *p1, *Ap;
-  double* partials;   // 3 * grid
-  Ctrl* ctrl;
+  XrSlot* slots;      // XR_SLOTS
+  Ctrl* ctrl;         // its arrival counter zeroed before the launch
   float tol; int max_iters;
+  int smem = 0;       // dynamic shared memory (set by the launch)
 };
-int pcg_grid_size(int device);
+// true: the solve of V rows keeps its rows' state in r and Ap and uses packed z, p0, p1
+bool pcg_packed_rows(int V);
 
 // CG on the block-scaled system (pcg.cu): identity (= block-Jacobi on A) or
 // the learned approximate inverse S of the scaled system.
@@ -123,8 +134,13 @@ struct PcgScaledArgs {
   int V;
   const int* chunk_off; const int* sell_col; const float* valh;               // A^ on the static pattern (SELL-32, pcg.cu)
   const int* xbegin; const int* xend; const int* xcols; const float* xvalh;  // A^ extra contact segment
+  // its SELL-32 copy (offsets per slice, columns with -1 pads, 9 planes); null: walked through xbegin / xend
+  const int* xs_off; const int* xs_col; const float* xs_val;
+  int wmax;             // column slots of the widest SELL-32 slice
+  XrSlot* slots_red;    // XR_SLOTS
+  int slots = 0;        // resident form: blocks of a row kept in shared memory (set by the launch)
   // learned solves only: S_ij = coef * A^_ij off the diagonal (coef per SELL
-  // slot, at the positions of sell_col) and S_ii = Sdiag (9 per vertex)
+  // slot, at the positions of sell_col) and S_ii = Sdiag (per slice 9 planes of 32)
   const float* coef; const float* Sdiag;
   const double* Linv;   // 6V packed L^-1
   const float* Lf;      // 6V packed L
@@ -141,12 +157,15 @@ struct PcgScaledArgs {
   // on the stream; returns at once when that solve ended PCG_OK (or timed out)
   int fallback = 0;
 };
-// Launch shape of the scaled PCG (threads per CTA, CTAs, column slots loaded
-// ahead per thread). A tuning knob only: every shape gives the same bits.
+// Launch shape of the scaled PCG: threads per CTA, CTAs, and the block slots
+// of a row kept in shared memory (resident form: KiB of it) or loaded ahead per
+// thread (looping form). A tuning knob only: every shape gives the same bits.
 struct PcgShape { int tpb = 0, grid = 0, unroll = 1; };
 size_t pcg_scaled_partials(int V);
+bool pcg_resident(int V);   // the scaled PCG of V rows runs in its resident form (reads xs_*)
+constexpr int PCG_NEAR_SLOTS = 7;   // static slots of a row whose neighbours' p the resident form keeps itself
 int pcg_scaled_shapes(int device, int V, bool learned, PcgShape* out, int max);
 cudaError_t launch_pcg_scaled(const PcgScaledArgs& a, bool learned, const PcgShape& sh, cudaStream_t s);
-cudaError_t launch_pcg(const PcgArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_pcg(const PcgArgs& a, cudaStream_t s);
 
 }  // namespace ando

@@ -427,7 +427,7 @@ __global__ void k_build_S(LsView s, const float* zv, const float* ab, float* S, 
     }
   }
   if (kd >= 0 && S) for (int q = 0; q < 9; ++q) S[9ll * kd + q] = D[q];
-  if (pcg.diag) for (int q = 0; q < 9; ++q) pcg.diag[9ll * i + q] = D[q];
+  if (pcg.diag) for (int q = 0; q < 9; ++q) pcg.diag[288ll * (i >> 5) + 32 * q + (i & 31)] = D[q];
 }
 
 // ------------------------------------------------------- training loss

@@ -87,7 +87,8 @@ void launch_net_prepare(const float* master, NetDev n, unsigned short* bf16, cud
 
 // S in the form the PCG applies it: off the diagonal S_ij = coef * A^_ij, so
 // one coefficient per SELL-32 slot (at slot position chunk_off + 32 k + lane,
-// like sell_col) and the 3x3 diagonal blocks (9 per vertex, row-major).
+// like sell_col) and the 3x3 diagonal blocks in the same order (per slice of
+// 32 vertices 9 planes of 32 lanes).
 struct SPcg { float* coef = nullptr; float* diag = nullptr; };
 
 // Inference: features, network, S (9 floats per static slot when S is not

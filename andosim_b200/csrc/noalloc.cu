@@ -12,9 +12,9 @@
 // What it runs: the persistent cooperative PCG kernel of pcg.cu (the same
 // iteration as PCGSolver::solve, pcg_solver.cpp:8-146), preceded by a kernel
 // that forms the block-Jacobi inverse from the matrix's diagonal blocks
-// exactly as the assembly kernel does. The kernel's per-CTA reduction
-// partials and its grid-barrier control words, which the context-based path
-// keeps in context buffers, live here in one file-scope static device array.
+// exactly as the assembly kernel does. The kernel's control block and
+// reduction slots, which the context-based path keeps in context buffers,
+// live here in one file-scope static device array.
 // Vectors live in the caller's work buffer.
 #include <cuda_runtime.h>
 
@@ -31,12 +31,11 @@ using namespace ando;
 
 namespace {
 
-// Scratch layout: [Ctrl control block, padded to 256 B][3 x kMaxCtas FP64 partials].
+// Scratch layout: [Ctrl control block, padded to 256 B][reduction slots].
 constexpr int kCtrlBytes = 256;
-constexpr int kMaxCtas = 640;
 constexpr size_t kScratchBytes = 16384;
 static_assert(sizeof(Ctrl) <= kCtrlBytes, "control block does not fit its slot");
-static_assert(kCtrlBytes + 3ull * kMaxCtas * sizeof(double) <= kScratchBytes, "partials do not fit the scratch");
+static_assert(kCtrlBytes + XR_SLOTS * sizeof(XrSlot) <= kScratchBytes, "reduction slots do not fit the scratch");
 
 // One 16 KiB scratch per device (the array is instantiated in every device's
 // copy of the module). It starts zeroed at module load; each call zeroes the
@@ -46,7 +45,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
 void* g_scratch_ptr[kMaxDevices] = {};
-int g_grid[kMaxDevices] = {};
 
 // Block-Jacobi inverse from the diagonal blocks, the same arithmetic as the
 // assembly kernel (pcg_solver.cpp:77-114): FP64 cofactors of the FP32 block,
@@ -80,7 +78,7 @@ __global__ void k_noalloc_jacobi(int V, const int* rowptr, const int* cols, cons
 
 // Device-side address of this device's scratch, looked up once per device
 // with that device current (the host-side symbol is not a device address).
-int scratch_for(int device, void** ptr, int* grid) {
+int scratch_for(int device, void** ptr) {
   std::lock_guard<std::mutex> lock(g_setup_mu);
   if (!g_scratch_ptr[device]) {
     void* p = nullptr;
@@ -89,12 +87,9 @@ int scratch_for(int device, void** ptr, int* grid) {
       cudaGetLastError();
       return set_last_error(ANDO_ERR_CUDA, "ando_pcg_solve_noalloc: cudaGetSymbolAddress of the scratch failed");
     }
-    int g = pcg_grid_size(device);
-    g_grid[device] = g < 1 ? 1 : (g > kMaxCtas ? kMaxCtas : g);
     g_scratch_ptr[device] = p;
   }
   *ptr = g_scratch_ptr[device];
-  *grid = g_grid[device];
   return ANDO_OK;
 }
 
@@ -108,31 +103,36 @@ int solve(int32_t device, cudaStream_t s, int32_t V, const int32_t* rowptr, cons
   if (work_floats < 24ll * V)
     return set_last_error(ANDO_ERR_CAPACITY, "ando_pcg_solve_noalloc: work buffer smaller than 24 * num_rows floats");
   void* scratch = nullptr;
-  int grid = 1;
-  int rc = scratch_for(device, &scratch, &grid);
+  int rc = scratch_for(device, &scratch);
   if (rc) return rc;
-  if (kCtrlBytes + 3ull * grid * sizeof(double) > kScratchBytes)
-    return set_last_error(ANDO_ERR_CAPACITY, "ando_pcg_solve_noalloc: grid needs more partials than the scratch holds");
   Ctrl* ctrl = reinterpret_cast<Ctrl*>(scratch);
   PcgArgs a{};
   a.V = V;
   a.rowptr = rowptr; a.cols = cols; a.val = vals;
   a.xbegin = nullptr; a.xend = nullptr; a.xcols = nullptr; a.xval = nullptr;
+  // P (9V), then z, p0 and p1 as 16-byte aligned float4 rows (12V and at most
+  // 3 floats of padding), or packed rows with r and Ap (15V): 24V holds either
   a.P = work;
   a.b = rhs;
   a.x = x;
-  a.r = work + 9ll * V; a.z = work + 12ll * V; a.p0 = work + 15ll * V; a.p1 = work + 18ll * V; a.Ap = work + 21ll * V;
-  a.partials = reinterpret_cast<double*>(static_cast<unsigned char*>(scratch) + kCtrlBytes);
+  float* vec = work + 9ll * V;
+  if (pcg_packed_rows(V)) {
+    a.z = vec; a.p0 = vec + 3ll * V; a.p1 = vec + 6ll * V; a.r = vec + 9ll * V; a.Ap = vec + 12ll * V;
+  } else {
+    vec = reinterpret_cast<float*>((reinterpret_cast<size_t>(vec) + 15) & ~size_t(15));
+    a.z = vec; a.p0 = vec + 4ll * V; a.p1 = vec + 8ll * V; a.r = a.Ap = nullptr;
+  }
+  a.slots = reinterpret_cast<XrSlot*>(static_cast<unsigned char*>(scratch) + kCtrlBytes);
   a.ctrl = ctrl;
   a.tol = float(tol);
   a.max_iters = max_iters;
-  // zero the control block (barrier words, error flag, converged flag)
+  // zero the control block (arrival counter, error flag, converged flag)
   cudaError_t e = cudaMemsetAsync(ctrl, 0, sizeof(Ctrl), s);
   if (e == cudaSuccess) {
     k_noalloc_jacobi<<<(V + 255) / 256, 256, 0, s>>>(V, rowptr, cols, vals, work);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = launch_pcg(a, grid, s);
+  if (e == cudaSuccess) e = launch_pcg(a, s);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_last_error(ANDO_ERR_CUDA, cudaGetErrorString(e));

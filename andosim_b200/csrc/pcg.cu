@@ -7,196 +7,420 @@
 // product and norm is accumulated in FP64 and reduced in a fixed order, so
 // results are bitwise reproducible run to run.
 //
-// Per iteration there are two grid barriers:
+// Per iteration there are two barriers over the launch's CTAs:
 //   A: p_new = z + beta p_old (recomputed on the fly for gathered columns),
-//      Ap = A p_new with one warp per block row, partial p^T Ap
+//      Ap = A p_new, partial p^T Ap
 //   B: x += alpha p, r -= alpha Ap, z = P r, partial r^T z and |r|_inf
-// The barrier is bounded (common.cuh): on timeout the kernel reports
+// The barriers are bounded (common.cuh): on timeout the kernel reports
 // PCG_TIMEOUT instead of spinning forever.
+#include <algorithm>
+#include <mutex>
+#include <type_traits>
+#include <utility>
+#include <vector>
+
 #include "kernels.cuh"
 
 namespace ando {
 
 namespace {
 
-constexpr int PCG_TPB = 512;
-constexpr int PCG_WARPS = PCG_TPB / 32;
+// ---------------------------------------------------------- unscaled PCG
+// What bounds it: a small system by the two dependent reductions of an
+// iteration, a large one by reading the matrix from L2. So
+//  - each warp owns whole 32-row slices, one thread per row, and the row's
+//    r, z, p, A p and x stay in registers for the whole solve; only z and p
+//    are published, for the neighbours' products;
+//  - a warp copies a slice's blocks and columns, contiguous in the CSR arrays,
+//    into its own shared-memory buffer with 16-byte asynchronous copies. A
+//    warp with one slice (RPT = 1) copies it once per solve; a warp with two
+//    or three walks them up and down in turn, so that one of them is always
+//    still there. The row stride of 9 x 7 floats reads without bank conflicts;
+//  - the barrier of each dot product carries the sum (xr_reduce).
+// RPT = 0 keeps the rows' state in the caller's vectors, for any size.
+constexpr int PCG_WARPS = 24;                 // 24 x 9.4 KB of shared memory: a slice of 32 rows of 7 blocks each
+constexpr int PCG_TPB = 32 * PCG_WARPS;
+constexpr int PCG_CLUSTER_TPB = 512;
+constexpr int PCG_SMEM = 224 * 1024;          // all warps' buffers
 
-__device__ inline double block_sum(double v, double* sh) {
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (w == 0) {
-    r = l < PCG_WARPS ? sh[l] : 0.0;
-    for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-    if (l == 0) sh[0] = r;
+// The solve's scalars, in shared memory: written by the thread that ends a
+// reduction, read by the CTA after it (coef: alpha after phase A, beta after
+// phase B).
+struct PcgScalars {
+  double rz, binf, rel, best;
+  int status, iters, since;
+  float coef;
+  // max |b| and r^T z of the initial residual
+  __device__ void start(bool ok, double rz0, unsigned mx, float tol, bool learned) {
+    rz = rz0; binf = double(__uint_as_float(mx)); rel = 0.0; iters = 0; since = 0; coef = 0.f; status = PCG_MAXIT;
+    if (!ok) { status = PCG_TIMEOUT; return; }
+    best = rel = binf < 1e-16 ? binf : 1.0;
+    if (rel < double(tol)) status = PCG_OK;
+    else if (learned && !(rz > 0.0)) status = PCG_PRECOND;
   }
-  __syncthreads();
-  r = sh[0];
-  __syncthreads();
-  return r;
-}
-__device__ inline double block_max(double v, double* sh) {
-  for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sh[w] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (w == 0) {
-    r = l < PCG_WARPS ? sh[l] : 0.0;
-    for (int o = 16; o; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
-    if (l == 0) sh[0] = r;
+  __device__ void after_product(bool ok, double pap) {
+    if (!ok) { status = PCG_TIMEOUT; return; }
+    ++iters;
+    if (fabs(pap) < 1e-16) status = PCG_NOT_SPD;
+    else coef = float(rz / pap);
   }
-  __syncthreads();
-  r = sh[0];
-  __syncthreads();
-  return r;
-}
-// Every CTA reduces the per-CTA partials in the same order -> identical scalars everywhere.
-__device__ inline double grid_sum(const double* part, int n, double* sh) {
-  double v = 0.0;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) v += part[k];
-  return block_sum(v, sh);
-}
-__device__ inline double grid_max(const double* part, int n, double* sh) {
-  double v = 0.0;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) v = fmax(v, part[k]);
-  return block_max(v, sh);
-}
-
-__device__ inline void p_at(const float* z, const float* pold, float beta, bool first, int j, float& p0, float& p1, float& p2) {
-  float z0 = z[3 * j], z1 = z[3 * j + 1], z2 = z[3 * j + 2];
-  if (first) { p0 = z0; p1 = z1; p2 = z2; return; }
-  p0 = z0 + beta * pold[3 * j]; p1 = z1 + beta * pold[3 * j + 1]; p2 = z2 + beta * pold[3 * j + 2];
-}
-
-__global__ void __launch_bounds__(PCG_TPB) k_pcg(PcgArgs a) {
-  Ctrl* ctrl = a.ctrl;
-  if (ctrl->converged) return;
-  __shared__ double sh[PCG_WARPS + 1];
-  const int V = a.V;
-  const unsigned nb = gridDim.x;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
-  double* part_pap = a.partials;
-  double* part_rz = a.partials + nb;
-  double* part_rinf = a.partials + 2 * nb;
-
-  // init: x = 0, r = b, z = P r
-  double rz_loc = 0.0, binf_loc = 0.0;
-  for (int i = tid; i < V; i += nthreads) {
-    float r0 = a.b[3 * i], r1 = a.b[3 * i + 1], r2 = a.b[3 * i + 2];
-    const float* P = a.P + 9 * (long long)i;
-    float z0 = P[0] * r0 + P[1] * r1 + P[2] * r2, z1 = P[3] * r0 + P[4] * r1 + P[5] * r2, z2 = P[6] * r0 + P[7] * r1 + P[8] * r2;
-    a.x[3 * i] = 0.f; a.x[3 * i + 1] = 0.f; a.x[3 * i + 2] = 0.f;
-    a.r[3 * i] = r0; a.r[3 * i + 1] = r1; a.r[3 * i + 2] = r2;
-    a.z[3 * i] = z0; a.z[3 * i + 1] = z1; a.z[3 * i + 2] = z2;
-    rz_loc += double(r0) * z0 + double(r1) * z1 + double(r2) * z2;
-    binf_loc = fmax(binf_loc, fmax(fabs(double(r0)), fmax(fabs(double(r1)), fabs(double(r2)))));
-  }
-  rz_loc = block_sum(rz_loc, sh);
-  binf_loc = block_max(binf_loc, sh);
-  if (threadIdx.x == 0) { part_rz[blockIdx.x] = rz_loc; part_rinf[blockIdx.x] = binf_loc; }
-  bool ok = grid_sync(&ctrl->bar_count, &ctrl->bar_gen, &ctrl->bar_err, nb);
-  int status = PCG_MAXIT, iters = 0;
-  double rel = 0.0;
-  if (!ok) status = PCG_TIMEOUT;
-  double rz = ok ? grid_sum(part_rz, nb, sh) : 0.0;
-  double binf = ok ? grid_max(part_rinf, nb, sh) : 0.0;
-  if (ok) {
-    rel = binf < 1e-16 ? binf : 1.0;
-    if (rel < double(a.tol)) status = PCG_OK;
-  }
-  float* pold = a.p0;
-  float* pnew = a.p1;
-  float beta = 0.f;
-  bool first = true;
-  const int lane = threadIdx.x & 31;
-  const int gwarp = tid >> 5, nwarps = nthreads >> 5;
-  const int comp = lane >> 3, bi = lane & 7;
-  for (int it = 0; ok && status == PCG_MAXIT && it < a.max_iters; ++it) {
-    // ---- phase A: p_new, Ap = A p_new, p^T Ap
-    double pap_loc = 0.0;
-    for (int row = gwarp; row < V; row += nwarps) {
-      float acc = 0.f;
-      int s0 = a.rowptr[row], s1 = a.rowptr[row + 1];
-      for (int k0 = s0; k0 < s1; k0 += 8) {
-        int k = k0 + bi;
-        if (comp < 3 && k < s1) {
-          int col = a.cols[k];
-          const float* h = a.val + 9 * (long long)k + 3 * comp;
-          float q0, q1, q2; p_at(a.z, pold, beta, first, col, q0, q1, q2);
-          acc += h[0] * q0 + h[1] * q1 + h[2] * q2;
-        }
-      }
-      if (a.xbegin) {
-        int e0 = a.xbegin[row], e1 = a.xend[row];
-        for (int k0 = e0; k0 < e1; k0 += 8) {
-          int k = k0 + bi;
-          if (comp < 3 && k < e1) {
-            int col = a.xcols[k];
-            const float* h = a.xval + 9 * (long long)k + 3 * comp;
-            float q0, q1, q2; p_at(a.z, pold, beta, first, col, q0, q1, q2);
-            acc += h[0] * q0 + h[1] * q1 + h[2] * q2;
-          }
-        }
-      }
-      acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-      float y0 = __shfl_sync(0xffffffffu, acc, 0), y1 = __shfl_sync(0xffffffffu, acc, 8), y2 = __shfl_sync(0xffffffffu, acc, 16);
-      if (lane == 0) {
-        float q0, q1, q2; p_at(a.z, pold, beta, first, row, q0, q1, q2);
-        pnew[3 * row] = q0; pnew[3 * row + 1] = q1; pnew[3 * row + 2] = q2;
-        a.Ap[3 * row] = y0; a.Ap[3 * row + 1] = y1; a.Ap[3 * row + 2] = y2;
-        pap_loc += double(q0) * y0 + double(q1) * y1 + double(q2) * y2;
-      }
-    }
-    pap_loc = block_sum(pap_loc, sh);
-    if (threadIdx.x == 0) part_pap[blockIdx.x] = pap_loc;
-    ok = grid_sync(&ctrl->bar_count, &ctrl->bar_gen, &ctrl->bar_err, nb);
-    if (!ok) { status = PCG_TIMEOUT; break; }
-    double pap = grid_sum(part_pap, nb, sh);
-    iters = it + 1;
-    if (fabs(pap) < 1e-16) { status = PCG_NOT_SPD; break; }
-    float alpha = float(rz / pap);
-    // ---- phase B: x, r, z, r^T z, |r|_inf
-    double rz_new_loc = 0.0, rinf_loc = 0.0;
-    for (int i = tid; i < V; i += nthreads) {
-      float p0 = pnew[3 * i], p1 = pnew[3 * i + 1], p2 = pnew[3 * i + 2];
-      float q0 = a.Ap[3 * i], q1 = a.Ap[3 * i + 1], q2 = a.Ap[3 * i + 2];
-      a.x[3 * i] += alpha * p0; a.x[3 * i + 1] += alpha * p1; a.x[3 * i + 2] += alpha * p2;
-      float r0 = a.r[3 * i] - alpha * q0, r1 = a.r[3 * i + 1] - alpha * q1, r2 = a.r[3 * i + 2] - alpha * q2;
-      a.r[3 * i] = r0; a.r[3 * i + 1] = r1; a.r[3 * i + 2] = r2;
-      const float* P = a.P + 9 * (long long)i;
-      float z0 = P[0] * r0 + P[1] * r1 + P[2] * r2, z1 = P[3] * r0 + P[4] * r1 + P[5] * r2, z2 = P[6] * r0 + P[7] * r1 + P[8] * r2;
-      a.z[3 * i] = z0; a.z[3 * i + 1] = z1; a.z[3 * i + 2] = z2;
-      rz_new_loc += double(r0) * z0 + double(r1) * z1 + double(r2) * z2;
-      rinf_loc = fmax(rinf_loc, fmax(fabs(double(r0)), fmax(fabs(double(r1)), fabs(double(r2)))));
-    }
-    rz_new_loc = block_sum(rz_new_loc, sh);
-    rinf_loc = block_max(rinf_loc, sh);
-    if (threadIdx.x == 0) { part_rz[blockIdx.x] = rz_new_loc; part_rinf[blockIdx.x] = rinf_loc; }
-    ok = grid_sync(&ctrl->bar_count, &ctrl->bar_gen, &ctrl->bar_err, nb);
-    if (!ok) { status = PCG_TIMEOUT; break; }
-    double rz_new = grid_sum(part_rz, nb, sh);
-    double rinf = grid_max(part_rinf, nb, sh);
+  __device__ void after_update(bool ok, double rz_new, unsigned mx, float tol, int stall_window) {
+    if (!ok) { status = PCG_TIMEOUT; return; }
+    const double rinf = double(__uint_as_float(mx));
     rel = binf < 1e-16 ? rinf : rinf / binf;
-    if (rel < double(a.tol)) { status = PCG_OK; break; }
-    beta = float(rz_new / rz);
+    if (rel < double(tol)) { status = PCG_OK; return; }
+    if (stall_window > 0) {   // learned preconditioner
+      if (!(rz_new > 0.0)) { status = PCG_PRECOND; return; }
+      if (rel < best) { best = rel; since = 0; }
+      else if (++since >= stall_window) { status = PCG_STALL; return; }
+    }
+    coef = float(rz_new / rz);
     rz = rz_new;
-    first = false;
-    float* t = pold; pold = pnew; pnew = t;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  __device__ void report(Ctrl* ctrl) const {
     ctrl->pcg_iters = iters;
     ctrl->pcg_status = status;
     ctrl->pcg_converged = status == PCG_OK ? 1 : 0;
     ctrl->pcg_rel = rel;
   }
+};
+
+// Row stride of z and p: float4 rows where the state is in registers, packed
+// rows where the caller's work buffer also holds r and A p.
+template <int S> __device__ inline float4 ld4(const float* v, int j) {
+  if (S == 4) return reinterpret_cast<const float4*>(v)[j];
+  return make_float4(v[3 * j], v[3 * j + 1], v[3 * j + 2], 0.f);
+}
+template <int S> __device__ inline void st4(float* v, int j, float a, float b, float c) {
+  if (S == 4) reinterpret_cast<float4*>(v)[j] = make_float4(a, b, c, 0.f);
+  else { v[3 * j] = a; v[3 * j + 1] = b; v[3 * j + 2] = c; }
+}
+
+// Asynchronous copy of n 4-byte elements from src into 16-byte aligned shared
+// memory, by the calling warp, in whole 16-byte pieces of global memory (a
+// piece holds at least one of the elements, so it is readable). Returns the
+// element offset of src[0] in dst.
+__device__ inline int warp_copy_async(void* dst, const void* src, int n) {
+  const size_t a = reinterpret_cast<size_t>(src);
+  const int off = int(a & 15) >> 2;
+  const char* g = reinterpret_cast<const char*>(a & ~size_t(15));
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int pieces = (off + n + 3) >> 2;
+  for (int q = threadIdx.x & 31; q < pieces; q += 32)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * q), "l"(g + 16ll * q) : "memory");
+  return off;
+}
+
+template <int RPT>
+__global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
+  Ctrl* ctrl = a.ctrl;
+  if (ctrl->converged) return;
+  extern __shared__ __align__(16) unsigned char pcg_dyn[];
+  __shared__ XrSmem sh;
+  __shared__ PcgScalars st;
+  constexpr int N = RPT > 0 ? RPT : 1, S = RPT > 0 ? 4 : 3, U = 4;
+  const int V = a.V, ns = (V + 31) >> 5, spc = (ns + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int w = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+  const int s0 = blockIdx.x * spc, sn = max(0, min(spc, ns - s0));   // slices [s0, s0 + sn)
+  const int wbuf = (a.smem / nw) & ~15, cap = (wbuf - 64) / 40;      // blocks that a warp's buffer holds
+  unsigned char* buf = pcg_dyn + (size_t)w * wbuf;
+  float* bval = reinterpret_cast<float*>(buf);
+  int* bcol = reinterpret_cast<int*>(buf + ((36 * cap + 16 + 15) & ~15));
+  float r[N][3], z[N][3], p[N][3], q[N][3], x[N][3], Pm[9];
+  int kb[N], cnt[N];
+  int held = -1, vo = 0, co = 0, hk0 = 0;   // slice in the buffer, element offsets of its first block and column, that block
+  auto row_of = [&](int j) { return 32 * (s0 + j) + lane; };
+  auto load_P = [&](int row, float (&m)[9]) {
+    for (int e = 0; e < 9; ++e) m[e] = a.P[9ll * row + e];
+  };
+  auto apply_P = [&](const float (&m)[9], const float (&v)[3], float (&o)[3]) {
+    o[0] = m[0] * v[0] + m[1] * v[1] + m[2] * v[2];
+    o[1] = m[3] * v[0] + m[4] * v[1] + m[5] * v[2];
+    o[2] = m[6] * v[0] + m[7] * v[1] + m[8] * v[2];
+  };
+  // slice j's partials of the next reduction
+  auto hand_over = [&](int j, double v, float m0, float m1, float m2) {
+    v = xr_warp_sum(v);
+    const unsigned m = __reduce_max_sync(0xffffffffu, max(xr_mag(m0), max(xr_mag(m1), xr_mag(m2))));
+    if (RPT > 0) { if (lane == 0) { sh.part[j] = v; sh.pmax[j] = m; } }
+    else if (lane == 0) { sh.part[w] += v; sh.pmax[w] = max(sh.pmax[w], m); }   // any number of slices: one partial per warp
+  };
+  auto begin = [&]() { if (RPT == 0 && lane == 0) { sh.part[w] = 0.0; sh.pmax[w] = 0u; } __syncwarp(); };
+  const int nparts = RPT > 0 ? sn : nw;
+  auto reduce = [&](unsigned epoch, auto tail) { xr_reduce(sh, nparts, epoch, a.slots, &ctrl->bar_arrivals, &ctrl->bar_err, tail); };
+
+  // init: x = 0, r = b, z = P r
+  begin();
+  auto init = [&](int k, int j) {
+    const int row = row_of(j);
+    double rz_loc = 0.0;
+    float b[3] = {0.f, 0.f, 0.f}, zz[3];
+    kb[k] = 0; cnt[k] = 0;
+    if (row < V) {
+      for (int e = 0; e < 3; ++e) b[e] = a.b[3 * row + e];
+      float m[9];
+      load_P(row, m);
+      apply_P(m, b, zz);
+      st4<S>(a.z, row, zz[0], zz[1], zz[2]);
+      rz_loc = double(b[0]) * zz[0] + double(b[1]) * zz[1] + double(b[2]) * zz[2];
+      if (RPT == 1) for (int e = 0; e < 9; ++e) Pm[e] = m[e];
+      if (RPT > 0) {
+        kb[k] = a.rowptr[row]; cnt[k] = a.rowptr[row + 1] - kb[k];
+        for (int e = 0; e < 3; ++e) { r[k][e] = b[e]; z[k][e] = zz[e]; x[k][e] = 0.f; p[k][e] = 0.f; }
+      } else {
+        for (int e = 0; e < 3; ++e) { a.x[3 * row + e] = 0.f; a.r[3 * row + e] = b[e]; }
+      }
+    }
+    hand_over(j, rz_loc, b[0], b[1], b[2]);
+  };
+  if constexpr (RPT > 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) if (w + nw * k < sn) init(k, w + nw * k);
+  } else {
+    for (int j = w; j < sn; j += nw) init(0, j);
+  }
+  reduce(1, [&](bool ok, double rz, unsigned mx) { st.start(ok, rz, mx, a.tol, false); });
+  float beta = 0.f;
+  float* pold = a.p0;
+  float* pnew = a.p1;
+  bool first = true;
+  for (int it = 0; st.status == PCG_MAXIT && it < a.max_iters; ++it) {
+    // ---- phase A: p_new = z + beta p_old, Ap = A p_new, p^T Ap
+    begin();
+    auto product = [&](int k, int j) {
+      const int row = row_of(j);
+      int k0 = 0, n = 0;
+      if (RPT > 0) { k0 = kb[k]; n = cnt[k]; }
+      else if (row < V) { k0 = a.rowptr[row]; n = a.rowptr[row + 1] - k0; }
+      if (held != j) {
+        const int first_block = __shfl_sync(0xffffffffu, k0, 0);
+        const int nb = __reduce_max_sync(0xffffffffu, n > 0 ? k0 + n - first_block : 0);
+        __syncwarp();
+        hk0 = first_block;
+        vo = warp_copy_async(bval, a.val + 9ll * first_block, 9 * min(nb, cap));
+        co = warp_copy_async(bcol, a.cols + first_block, min(nb, cap));
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        held = j;
+      }
+      float y[3] = {0.f, 0.f, 0.f};
+      const int lo = k0 - hk0, inbuf = max(0, min(n, cap - lo));
+      const int* bc = bcol + co + lo;
+      const float* bv = bval + vo + 9 * lo;
+      auto fma3 = [&](const float* h, const float4& zz, const float4& pp) {
+        const float q0 = first ? zz.x : zz.x + beta * pp.x, q1 = first ? zz.y : zz.y + beta * pp.y, q2 = first ? zz.z : zz.z + beta * pp.z;
+        y[0] += h[0] * q0 + h[1] * q1 + h[2] * q2;
+        y[1] += h[3] * q0 + h[4] * q1 + h[5] * q2;
+        y[2] += h[6] * q0 + h[7] * q1 + h[8] * q2;
+      };
+      for (int e = 0; e < inbuf; e += U) {
+        float4 zz[U], pp[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (e + u < inbuf) {
+            const int c = bc[e + u];
+            zz[u] = ld4<S>(a.z, c);
+            pp[u] = first ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4<S>(pold, c);
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (e + u < inbuf) fma3(bv + 9 * (e + u), zz[u], pp[u]);
+      }
+      auto outside = [&](int c, const float* h) {
+        fma3(h, ld4<S>(a.z, c), first ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4<S>(pold, c));
+      };
+      for (int e = inbuf; e < n; ++e) outside(a.cols[k0 + e], a.val + 9ll * (k0 + e));
+      if (a.xbegin && row < V)
+        for (int e = a.xbegin[row]; e < a.xend[row]; ++e) outside(a.xcols[e], a.xval + 9ll * e);
+      double pap_loc = 0.0;
+      if (row < V) {
+        float pv[3];
+        if (RPT > 0) {
+          for (int e = 0; e < 3; ++e) pv[e] = p[k][e] = first ? z[k][e] : z[k][e] + beta * p[k][e];
+          for (int e = 0; e < 3; ++e) q[k][e] = y[e];
+        } else {
+          const float4 zz = ld4<S>(a.z, row), pp = first ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4<S>(pold, row);
+          pv[0] = first ? zz.x : zz.x + beta * pp.x; pv[1] = first ? zz.y : zz.y + beta * pp.y; pv[2] = first ? zz.z : zz.z + beta * pp.z;
+          for (int e = 0; e < 3; ++e) a.Ap[3 * row + e] = y[e];
+        }
+        st4<S>(pnew, row, pv[0], pv[1], pv[2]);
+        pap_loc = double(pv[0]) * y[0] + double(pv[1]) * y[1] + double(pv[2]) * y[2];
+      }
+      hand_over(j, pap_loc, 0.f, 0.f, 0.f);
+    };
+    const bool up = (it & 1) == 0;
+    if constexpr (RPT > 0) {
+      if (RPT == 1 || up) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) if (w + nw * k < sn) product(k, w + nw * k);
+      } else {
+#pragma unroll
+        for (int k = N - 1; k >= 0; --k) if (w + nw * k < sn) product(k, w + nw * k);
+      }
+    } else {
+      const int m = w < sn ? (sn - 1 - w) / nw + 1 : 0;
+      for (int t = 0; t < m; ++t) product(0, w + nw * (up ? t : m - 1 - t));
+    }
+    reduce(2 + 2 * it, [&](bool ok, double pap, unsigned) { st.after_product(ok, pap); });
+    if (st.status != PCG_MAXIT) break;
+    const float alpha = st.coef;
+    // ---- phase B: x, r, z, r^T z, |r|_inf
+    begin();
+    auto update = [&](int k, int j) {
+      const int row = row_of(j);
+      double rz_loc = 0.0;
+      float rv[3] = {0.f, 0.f, 0.f}, zv[3], m[9];
+      if (row < V) {
+        if (RPT != 1) load_P(row, m);
+        if (RPT > 0) {
+          for (int e = 0; e < 3; ++e) { x[k][e] += alpha * p[k][e]; r[k][e] -= alpha * q[k][e]; rv[e] = r[k][e]; }
+        } else {
+          const float4 pp = ld4<S>(pnew, row);
+          const float pv[3] = {pp.x, pp.y, pp.z};
+          for (int e = 0; e < 3; ++e) {
+            a.x[3 * row + e] += alpha * pv[e];
+            rv[e] = a.r[3 * row + e] - alpha * a.Ap[3 * row + e];
+            a.r[3 * row + e] = rv[e];
+          }
+        }
+        if (RPT == 1) apply_P(Pm, rv, zv); else apply_P(m, rv, zv);
+        if (RPT > 0) for (int e = 0; e < 3; ++e) z[k][e] = zv[e];
+        st4<S>(a.z, row, zv[0], zv[1], zv[2]);
+        rz_loc = double(rv[0]) * zv[0] + double(rv[1]) * zv[1] + double(rv[2]) * zv[2];
+      }
+      hand_over(j, rz_loc, rv[0], rv[1], rv[2]);
+    };
+    if constexpr (RPT > 0) {
+#pragma unroll
+      for (int k = 0; k < N; ++k) if (w + nw * k < sn) update(k, w + nw * k);
+    } else {
+      for (int j = w; j < sn; j += nw) update(0, j);
+    }
+    reduce(3 + 2 * it, [&](bool ok, double rz, unsigned mx) { st.after_update(ok, rz, mx, a.tol, 0); });
+    if (st.status != PCG_MAXIT) break;
+    beta = st.coef;
+    first = false;
+    float* t = pold; pold = pnew; pnew = t;
+  }
+  if constexpr (RPT > 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const int row = row_of(w + nw * k);
+      if (w + nw * k < sn && row < V) for (int e = 0; e < 3; ++e) a.x[3 * row + e] = x[k][e];
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) st.report(ctrl);
+}
+
+// The same solve for a small system, as one cluster of at most 16 CTAs with
+// one row per thread (512 rows to a CTA): z and p are published in shared
+// memory and read from the CTA that owns the row, so an iteration touches no
+// global memory and its two barriers are the cluster's. A row's first PCG_KQ
+// neighbours' p stay in registers (p_new_j = z_j + beta p_j is what the
+// thread computed for them one iteration ago). 1,024 rows: 34.9 us per
+// iteration with a warp per row and two grid barriers through L2.
+constexpr int PCG_KQ = 8;
+
+__device__ inline float4 cl_ld4(unsigned addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(PCG_CLUSTER_TPB, 1) k_pcg_cluster(PcgArgs a) {
+  Ctrl* ctrl = a.ctrl;
+  if (ctrl->converged) return;
+  extern __shared__ __align__(16) unsigned char pcg_dyn[];   // z, p, p' of the CTA's rows (float4), then each warp's matrix buffer
+  __shared__ XrSmem sh;
+  __shared__ PcgScalars st;
+  const int V = a.V, rows = blockDim.x, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int row = blockIdx.x * rows + threadIdx.x;
+  const bool live = row < V;
+  float4* const pub = reinterpret_cast<float4*>(pcg_dyn);
+  const unsigned pub0 = (unsigned)__cvta_generic_to_shared(pub);
+  const unsigned array = 16u * rows;                         // bytes of one published vector: z, then the two p
+  const int wbuf = ((a.smem - 48 * rows) / nw) & ~15, cap = (wbuf - 64) / 40;
+  unsigned char* buf = pcg_dyn + 48 * rows + (size_t)w * wbuf;
+  float* bval = reinterpret_cast<float*>(buf);
+  int* bcol = reinterpret_cast<int*>(buf + ((36 * cap + 16 + 15) & ~15));
+  auto handle = [&](int col) { const int c = col / rows; return cl_map(pub0 + 16u * (col - c * rows), c); };   // z of row col
+
+  const int kb = live ? a.rowptr[row] : 0, n = live ? a.rowptr[row + 1] - kb : 0;
+  const int k0 = __shfl_sync(0xffffffffu, kb, 0), nb = __reduce_max_sync(0xffffffffu, n > 0 ? kb + n - k0 : 0);
+  const int vo = warp_copy_async(bval, a.val + 9ll * k0, 9 * min(nb, cap));
+  const int co = warp_copy_async(bcol, a.cols + k0, min(nb, cap));
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+  const int lo = kb - k0, inbuf = max(0, min(n, cap - lo));
+  int* const bc = bcol + co + lo;
+  const float* const bv = bval + vo + 9 * lo;
+  for (int e = 0; e < inbuf; ++e) bc[e] = (int)handle(bc[e]);   // columns -> addresses of their z
+
+  float P[9], r[3] = {0.f, 0.f, 0.f}, z[3] = {0.f, 0.f, 0.f}, p[3] = {0.f, 0.f, 0.f}, x[3] = {0.f, 0.f, 0.f}, q[PCG_KQ][3];
+  for (int e = 0; e < 9; ++e) P[e] = live ? a.P[9ll * row + e] : 0.f;
+  for (int e = 0; e < PCG_KQ; ++e) q[e][0] = q[e][1] = q[e][2] = 0.f;
+  if (live) for (int e = 0; e < 3; ++e) r[e] = a.b[3 * row + e];
+  auto put = [&](unsigned off, const float (&v)[3]) { *reinterpret_cast<float4*>(pcg_dyn + off + 16 * threadIdx.x) = make_float4(v[0], v[1], v[2], 0.f); };
+  auto apply_P = [&]() {
+    z[0] = P[0] * r[0] + P[1] * r[1] + P[2] * r[2];
+    z[1] = P[3] * r[0] + P[4] * r[1] + P[5] * r[2];
+    z[2] = P[6] * r[0] + P[7] * r[1] + P[8] * r[2];
+    put(0, z);
+    return double(r[0]) * z[0] + double(r[1]) * z[1] + double(r[2]) * z[2];
+  };
+  auto mag = [&]() { return max(xr_mag(r[0]), max(xr_mag(r[1]), xr_mag(r[2]))); };
+  auto reduce = [&](unsigned epoch, double v, unsigned m, auto tail) {
+    v = xr_warp_sum(v);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) { sh.part[w] = v; sh.pmax[w] = m; }
+    cl_reduce(sh, nw, epoch, tail);
+  };
+  double rz0 = apply_P();
+  reduce(1, rz0, mag(), [&](bool ok, double rz, unsigned mx) { st.start(ok, rz, mx, a.tol, false); });
+  unsigned pold = array, pnew = 2 * array;
+  float beta = 0.f;
+  for (int it = 0; st.status == PCG_MAXIT && it < a.max_iters; ++it) {
+    // ---- phase A: p_new = z + beta p_old, Ap = A p_new, p^T Ap
+    float y[3] = {0.f, 0.f, 0.f};
+    auto fma3 = [&](const float* h, float q0, float q1, float q2) {
+      y[0] += h[0] * q0 + h[1] * q1 + h[2] * q2;
+      y[1] += h[3] * q0 + h[4] * q1 + h[5] * q2;
+      y[2] += h[6] * q0 + h[7] * q1 + h[8] * q2;
+    };
+    float4 zz[PCG_KQ];
+#pragma unroll
+    for (int e = 0; e < PCG_KQ; ++e) if (e < inbuf) zz[e] = cl_ld4((unsigned)bc[e]);
+#pragma unroll
+    for (int e = 0; e < PCG_KQ; ++e)
+      if (e < inbuf) {
+        q[e][0] = zz[e].x + beta * q[e][0]; q[e][1] = zz[e].y + beta * q[e][1]; q[e][2] = zz[e].z + beta * q[e][2];
+        fma3(bv + 9 * e, q[e][0], q[e][1], q[e][2]);
+      }
+    auto far = [&](unsigned at, const float* h) {
+      const float4 zf = cl_ld4(at), pf = it ? cl_ld4(at + pold) : make_float4(0.f, 0.f, 0.f, 0.f);
+      fma3(h, zf.x + beta * pf.x, zf.y + beta * pf.y, zf.z + beta * pf.z);
+    };
+    for (int e = PCG_KQ; e < inbuf; ++e) far((unsigned)bc[e], bv + 9 * e);
+    for (int e = inbuf; e < n; ++e) far(handle(a.cols[kb + e]), a.val + 9ll * (kb + e));
+    if (a.xbegin && live)
+      for (int e = a.xbegin[row]; e < a.xend[row]; ++e) far(handle(a.xcols[e]), a.xval + 9ll * e);
+    for (int e = 0; e < 3; ++e) p[e] = z[e] + beta * p[e];
+    put(pnew, p);
+    reduce(2 + 2 * it, double(p[0]) * y[0] + double(p[1]) * y[1] + double(p[2]) * y[2], 0u,
+           [&](bool ok, double pap, unsigned) { st.after_product(ok, pap); });
+    if (st.status != PCG_MAXIT) break;
+    const float alpha = st.coef;
+    // ---- phase B: x, r, z, r^T z, |r|_inf
+    for (int e = 0; e < 3; ++e) { x[e] += alpha * p[e]; r[e] -= alpha * y[e]; }
+    rz0 = apply_P();
+    reduce(3 + 2 * it, rz0, mag(), [&](bool ok, double rz, unsigned mx) { st.after_update(ok, rz, mx, a.tol, 0); });
+    if (st.status != PCG_MAXIT) break;
+    beta = st.coef;
+    const unsigned t = pold; pold = pnew; pnew = t;
+  }
+  if (live) for (int e = 0; e < 3; ++e) a.x[3 * row + e] = x[e];
+  if (row == 0) st.report(ctrl);
+  cl_sync_shared();   // the others have read this CTA's last partial
 }
 
 // ------------------------------------------------------------ scaled PCG
@@ -236,15 +460,6 @@ __global__ void __launch_bounds__(PCG_TPB) k_pcg(PcgArgs a) {
 // larger vectors measured slower (19.5 against 18.7 us per iteration at
 // C4). Each solve initialises its vectors, so the two layouts share buffers
 // of 4V floats.
-template <int S> __device__ inline float4 ld4(const float* v, int j) {
-  if (S == 4) return reinterpret_cast<const float4*>(v)[j];
-  return make_float4(v[3 * j], v[3 * j + 1], v[3 * j + 2], 0.f);
-}
-template <int S> __device__ inline void st4(float* v, int j, float a, float b, float c) {
-  if (S == 4) reinterpret_cast<float4*>(v)[j] = make_float4(a, b, c, 0.f);
-  else { v[3 * j] = a; v[3 * j + 1] = b; v[3 * j + 2] = c; }
-}
-
 template <int S> struct GatherP {  // p = z + beta p_old
   const float* z; const float* pold; float beta; bool first;
   __device__ void operator()(int j, float& q0, float& q1, float& q2) const {
@@ -402,7 +617,7 @@ __device__ inline void sell_row_S(int row, const int* chunk_off, const int* sell
     }
   }
   float g0, g1, g2; vec(row, g0, g1, g2);
-  block_fma<1>(Sdiag + 9ll * row, g0, g1, g2, a0, a1, a2);
+  block_fma<32>(Sdiag + 288ll * (row >> 5) + (row & 31), g0, g1, g2, a0, a1, a2);
   y0 = a0; y1 = a1; y2 = a2;
 }
 
@@ -588,6 +803,283 @@ __global__ void __launch_bounds__(SCALED_MAX_TPB) k_pcg_scaled(PcgScaledArgs a) 
   }
 }
 
+// ------------------------------------------- scaled PCG, resident form
+// The same solve, bit for bit in its vectors, for meshes of at most one row
+// per thread of the GPU (1,024 rows per CTA, one CTA on each SM): each warp
+// owns one 32-row slice, one thread per row, for the whole solve.
+//  - r^, p, A^ p and x^ of a row are registers; r^ (learned: z, r^ and A^ p)
+//    is published as float4 rows for the neighbours' products.
+//  - With KQ > 0 the neighbours' p of a row's first KQ slots stay in registers
+//    too: p_new_j = z_j + beta p_j is what the thread computed for column j
+//    one iteration ago, so a product gathers one vector instead of two. The
+//    shapes whose registers do not hold them (KQ = 0) publish p as well.
+//  - A^ is constant over the solve, so a slice's blocks are copied into shared
+//    memory once, in the SELL-32 order (9 planes of 32 lanes: no bank
+//    conflicts). A row's own block is exactly I unless its factorisation was
+//    shifted, so in CTAs of more than 512 threads it takes no space: a
+//    curtain's 6 remaining blocks at 886 rows per SM just fit. FAR: meshes with
+//    wider rows and systems with contact blocks; slots past the capacity
+//    (`slots` per row) are read from L2.
+//  - The barrier of each dot product carries the sum: one partial per CTA
+//    through L2 (xr_reduce), or, for systems of at most 16,384 rows, one
+//    cluster whose CTAs publish everything through shared memory (cl_reduce).
+// Contact blocks come in a SELL-32 copy of their own (xs_*), so a warp reads
+// them as whole lines; without one (rows of very uneven contact counts) they
+// are walked row by row.
+constexpr int RES_KQ = PCG_NEAR_SLOTS;
+constexpr int RES_SMEM = 224 * 1024;   // dynamic shared memory of a CTA, at most
+// float4 vectors that a CTA of the cluster form publishes in shared memory
+constexpr int res_vectors(bool learned, bool far, int kq) { return (learned ? 4 : 1) + (far || kq == 0 ? 2 : 0); }
+// CTAs of more than 512 threads have no room for the rows' own blocks
+constexpr bool res_compact(bool far, int max_threads) { return !far && max_threads > 512; }
+inline int res_warp_bytes(int slots) { return slots * 1152 + (slots + 1) * 128; }
+
+template <bool LEARNED, bool FAR, bool CLUSTER, int KQ, int NB, int U, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) k_pcg_res(const __grid_constant__ PcgScaledArgs a) {
+  Ctrl* const ctrl = a.ctrl;
+  if (ctrl->converged) return;
+  if (!LEARNED && a.fallback) {
+    // every CTA reads the learned solve's status before the first barrier; it
+    // is rewritten only after one
+    const int st = ctrl->pcg_status;
+    if (st == PCG_OK || st == PCG_TIMEOUT) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->fallback_ran = 1;
+  }
+  constexpr bool COMPACT = res_compact(FAR, MAXT);
+  constexpr int PUB = CLUSTER ? res_vectors(LEARNED, FAR, KQ) : 0;
+  constexpr bool PUB_P = FAR || KQ == 0;
+  extern __shared__ __align__(16) float res_dyn[];   // cluster form: the published vectors; then each warp's blocks and columns
+  __shared__ XrSmem sh;
+  __shared__ PcgScalars st;
+  const int V = a.V, ns = (V + 31) >> 5, nw = blockDim.x >> 5, rows = blockDim.x;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sn = max(0, min(nw, ns - (int)blockIdx.x * nw));   // slices of this CTA
+  const int slice = blockIdx.x * nw + w, row = 32 * slice + lane;
+  const bool own = w < sn, live = own && row < V;
+  const int Kc = a.slots;
+  float* const sm = res_dyn + 4 * PUB * rows + w * (Kc * 288 + (Kc + 1) * 32) + lane;   // the lane's entries of the warp's blocks
+  int* const smc = reinterpret_cast<int*>(sm + Kc * 288);                                // and columns
+
+  // Published vectors: global float4 rows, or this CTA's shared memory. A
+  // column's handle is its row, or the address of its row's first vector in
+  // the CTA that owns it; -1: padding.
+  using Vec = std::conditional_t<CLUSTER, unsigned, float*>;
+  const unsigned pub0 = (unsigned)__cvta_generic_to_shared(res_dyn), array = 16u * rows;
+  auto vec_z = [&]() -> Vec { if constexpr (CLUSTER) return 0u; else return LEARNED ? a.z : a.r; };
+  auto vec_r = [&](int odd) -> Vec { if constexpr (CLUSTER) return (odd ? 2u : 1u) * array; else return odd ? a.r2 : a.r; };
+  auto vec_ap = [&]() -> Vec { if constexpr (CLUSTER) return 3u * array; else return a.Ap; };
+  auto vec_p = [&](int odd) -> Vec { if constexpr (CLUSTER) return ((LEARNED ? 4u : 1u) + (odd ? 1u : 0u)) * array; else return odd ? a.p1 : a.p0; };
+  auto get = [&](Vec v, int h) -> float4 {
+    if constexpr (CLUSTER) return cl_ld4((unsigned)h + v);
+    else return ld4<4>(v, h);
+  };
+  auto put = [&](Vec v, const float (&f)[3]) {
+    if constexpr (CLUSTER) *reinterpret_cast<float4*>(reinterpret_cast<unsigned char*>(res_dyn) + v + 16 * threadIdx.x) = make_float4(f[0], f[1], f[2], 0.f);
+    else if (live) st4<4>(v, row, f[0], f[1], f[2]);
+  };
+  auto handle = [&](int col) -> int {
+    if constexpr (CLUSTER) {
+      if (col < 0) return -1;
+      const int c = col / rows;
+      return (int)cl_map(pub0 + 16u * (col - c * rows), c);
+    } else return col;
+  };
+
+  // The slice's columns and blocks: static slots, then contact blocks. In the
+  // compact layout the row's own block (slot kd) takes no place and the blocks
+  // after it move up one.
+  const int b0 = own ? a.chunk_off[slice] : 0, wd = own ? (a.chunk_off[slice + 1] - b0) >> 5 : 0;
+  const int xb0 = FAR && own && a.xs_off ? a.xs_off[slice] : 0, xw = FAR && own && a.xs_off ? (a.xs_off[slice + 1] - xb0) >> 5 : 0;
+  const int nk = wd + xw, own_h = handle(min(row, V - 1));   // a row past the end reads the last one's vectors, unused
+  const float* const gv = a.valh + 9ll * b0 + lane;   // slot k: 288 k floats on
+  auto global_block = [&](int k) -> const float* {
+    return !FAR || k < wd ? gv + 288 * k : a.xs_val + 9ll * (xb0 + 32 * (k - wd)) + lane;
+  };
+  auto global_col = [&](int k) { return handle(!FAR || k < wd ? a.sell_col[b0 + 32 * k + lane] : a.xs_col[xb0 + 32 * (k - wd) + lane]); };
+  int kd = 1 << 20;
+  bool ident = true;
+  for (int k = 0; k < min(nk, Kc + 1); ++k) {
+    const int h = global_col(k);
+    smc[32 * k] = h;
+    if (COMPACT && h == own_h) kd = k;
+  }
+  for (int k = 0; k < min(nk, Kc + 1); ++k) {
+    const float* g = global_block(k);
+    const int t = COMPACT ? k - (k > kd) : k;
+    if (COMPACT && k == kd) { for (int e = 0; e < 9; ++e) ident = ident && g[32 * e] == ((e & 3) == 0 ? 1.f : 0.f); }
+    else if (t < Kc) for (int e = 0; e < 9; ++e) sm[288 * t + 32 * e] = g[32 * e];
+  }
+  // h = block k (on chip), entries of a lane without that slot undefined
+  auto near_block = [&](int k, float (&h)[9]) {
+    const float* s = sm + 288 * min(COMPACT ? k - (k > kd) : k, Kc - 1);
+#pragma unroll
+    for (int e = 0; e < 9; ++e) h[e] = s[32 * e];
+    if (COMPACT && k == kd) {
+      if (ident) { for (int e = 0; e < 9; ++e) h[e] = (e & 3) == 0 ? 1.f : 0.f; }
+      else { for (int e = 0; e < 9; ++e) h[e] = gv[288 * k + 32 * e]; }
+    }
+  };
+  auto fma9 = [&](const float (&h)[9], float q0, float q1, float q2, float (&y)[3]) { block_fma<1>(h, q0, q1, q2, y[0], y[1], y[2]); };
+  auto reduce = [&](unsigned epoch, double v, float m0, float m1, float m2, auto tail) {
+    v = xr_warp_sum(v);
+    const unsigned m = __reduce_max_sync(0xffffffffu, max(xr_mag(m0), max(xr_mag(m1), xr_mag(m2))));
+    if (lane == 0 && own) { sh.part[w] = v; sh.pmax[w] = m; }
+    if constexpr (CLUSTER) cl_reduce(sh, sn, epoch, tail);
+    else xr_reduce(sh, sn, epoch, a.slots_red, &ctrl->bar_arrivals, &ctrl->bar_err, tail);
+  };
+
+  // init: x^ = 0, r = b^, z = S b^, max |b^|
+  float r[3] = {0.f, 0.f, 0.f}, z[3] = {0.f, 0.f, 0.f}, p[3] = {0.f, 0.f, 0.f}, q[KQ > 0 ? KQ : 1][3];
+  double x[3] = {0.0, 0.0, 0.0};
+  for (int k = 0; k < KQ; ++k) q[k][0] = q[k][1] = q[k][2] = 0.f;
+  if (live) for (int e = 0; e < 3; ++e) r[e] = a.bhat[3 * row + e];
+  if (LEARNED) {
+    for (int k = 0; k < wd; ++k) {
+      const int c = a.sell_col[b0 + 32 * k + lane];
+      if (c < 0 || c == row) continue;
+      const float cf = a.coef[b0 + 32 * k + lane];
+      block_fma<32>(gv + 288 * k, cf * a.bhat[3 * c], cf * a.bhat[3 * c + 1], cf * a.bhat[3 * c + 2], z[0], z[1], z[2]);
+    }
+    if (live) block_fma<32>(a.Sdiag + 288ll * slice + lane, r[0], r[1], r[2], z[0], z[1], z[2]);
+    put(vec_r(0), r);
+  } else {
+    for (int e = 0; e < 3; ++e) z[e] = r[e];
+    if (live && a.snap_r && a.snap_max > 0)
+      for (int e = 0; e < 3; ++e) { a.snap_r[3 * row + e] = r[e]; a.snap_x[3 * row + e] = 0.0; }
+  }
+  put(vec_z(), z);
+  reduce(1, double(r[0]) * z[0] + double(r[1]) * z[1] + double(r[2]) * z[2], r[0], r[1], r[2],
+         [&](bool ok, double rz, unsigned mx) { st.start(ok, rz, mx, a.tol, LEARNED); });
+  float beta = 0.f;
+  int it = 0;
+  for (; st.status == PCG_MAXIT && it < a.max_iters; ++it) {
+    // ---- phase A: p_new = z + beta p_old, Ap = A^ p_new, p^T Ap
+    float y[3] = {0.f, 0.f, 0.f};
+    // slots whose neighbours' p the thread keeps. Loads are unconditional (a
+    // lane without the slot reads its own row), so a batch's are all in flight
+    // together; only the products are predicated.
+#pragma unroll
+    for (int k0 = 0; k0 < KQ; k0 += NB) {
+      if (k0 >= nk) break;
+      int c[NB];
+      float4 zz[NB];
+#pragma unroll
+      for (int u = 0; u < NB; ++u)
+        if (k0 + u < KQ) {
+          c[u] = k0 + u < nk ? (!FAR || k0 + u <= Kc ? smc[32 * (k0 + u)] : global_col(k0 + u)) : -1;
+          zz[u] = get(vec_z(), c[u] != -1 ? c[u] : own_h);
+        }
+#pragma unroll
+      for (int u = 0; u < NB; ++u)
+        if (k0 + u < KQ) {
+          float (&qk)[3] = q[KQ > 0 ? k0 + u : 0];
+          qk[0] = zz[u].x + beta * qk[0]; qk[1] = zz[u].y + beta * qk[1]; qk[2] = zz[u].z + beta * qk[2];
+          float h[9];
+          if (!FAR || k0 + u < Kc) near_block(k0 + u, h);
+          else if (k0 + u < nk) for (int e = 0; e < 9; ++e) h[e] = global_block(k0 + u)[32 * e];
+          if (c[u] != -1) fma9(h, qk[0], qk[1], qk[2], y);
+        }
+    }
+    if (PUB_P) {   // further slots: both vectors gathered
+      const Vec pold = vec_p(it & 1);
+#pragma unroll 1
+      for (int k0 = KQ; k0 < nk; k0 += U) {
+        int c[U];
+        float4 zz[U], pp[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          c[u] = k0 + u < nk ? (!FAR || k0 + u <= Kc ? smc[32 * (k0 + u)] : global_col(k0 + u)) : -1;
+          const int at = c[u] != -1 ? c[u] : own_h;
+          zz[u] = get(vec_z(), at);
+          pp[u] = it ? get(pold, at) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          float h[9];
+          if (!FAR || k0 + u < Kc) near_block(min(k0 + u, nk - 1), h);
+          else if (k0 + u < nk) for (int e = 0; e < 9; ++e) h[e] = global_block(k0 + u)[32 * e];
+          if (c[u] != -1) fma9(h, zz[u].x + beta * pp[u].x, zz[u].y + beta * pp[u].y, zz[u].z + beta * pp[u].z, y);
+        }
+      }
+      if (FAR && a.xbegin && !a.xs_off && live)
+        for (int e = a.xbegin[row]; e < a.xend[row]; ++e) {
+          const int c = handle(a.xcols[e]);
+          const float4 zf = get(vec_z(), c), pf = it ? get(pold, c) : make_float4(0.f, 0.f, 0.f, 0.f);
+          block_fma<1>(a.xvalh + 9ll * e, zf.x + beta * pf.x, zf.y + beta * pf.y, zf.z + beta * pf.z, y[0], y[1], y[2]);
+        }
+    }
+    for (int e = 0; e < 3; ++e) p[e] = z[e] + beta * p[e];
+    if (PUB_P) put(vec_p(~it & 1), p);
+    if (LEARNED) put(vec_ap(), y);
+    reduce(2 + 2 * it, double(p[0]) * y[0] + double(p[1]) * y[1] + double(p[2]) * y[2], 0.f, 0.f, 0.f,
+           [&](bool ok, double pap, unsigned) { st.after_product(ok, pap); });
+    if (st.status != PCG_MAXIT) break;
+    const float alpha = st.coef;
+    // ---- phase B: x^ += alpha p, r -= alpha Ap, z = S r, r^T z, |r|_inf
+    for (int e = 0; e < 3; ++e) { x[e] += double(alpha) * p[e]; r[e] = r[e] - alpha * y[e]; }
+    if (LEARNED) {
+      z[0] = z[1] = z[2] = 0.f;
+#pragma unroll 1
+      for (int k0 = 0; k0 < wd; k0 += U) {
+        int c[U];
+        float cf[U];
+        float4 rr[U], aa[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          c[u] = k0 + u < wd ? (!FAR || k0 + u <= Kc ? smc[32 * (k0 + u)] : global_col(k0 + u)) : -1;
+          if (c[u] == own_h) c[u] = -1;
+          const int at = c[u] != -1 ? c[u] : own_h;
+          cf[u] = c[u] != -1 ? a.coef[b0 + 32 * (k0 + u) + lane] : 0.f;
+          rr[u] = get(vec_r(it & 1), at);
+          aa[u] = get(vec_ap(), at);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          float h[9];
+          if (!FAR || k0 + u < Kc) near_block(min(k0 + u, wd - 1), h);
+          else if (k0 + u < wd) for (int e = 0; e < 9; ++e) h[e] = gv[288 * (k0 + u) + 32 * e];
+          const float g0 = rr[u].x - alpha * aa[u].x, g1 = rr[u].y - alpha * aa[u].y, g2 = rr[u].z - alpha * aa[u].z;
+          if (c[u] != -1) fma9(h, cf[u] * g0, cf[u] * g1, cf[u] * g2, z);
+        }
+      }
+      if (live) block_fma<32>(a.Sdiag + 288ll * slice + lane, r[0], r[1], r[2], z[0], z[1], z[2]);
+      put(vec_r(~it & 1), r);   // neighbours still read the old r
+    } else {
+      for (int e = 0; e < 3; ++e) z[e] = r[e];
+      if (live && a.snap_r) {
+        // snapshot k of (r^, x^) after 2^k - 1 iterations (training probes)
+        const int done = it + 1, snap = (done & (done + 1)) == 0 ? __ffs(done + 1) - 1 : -1;
+        if (snap >= 0 && snap < a.snap_max)
+          for (int e = 0; e < 3; ++e) {
+            a.snap_r[3ll * V * snap + 3 * row + e] = r[e];
+            a.snap_x[3ll * V * snap + 3 * row + e] = x[e];
+          }
+      }
+    }
+    put(vec_z(), z);
+    reduce(3 + 2 * it, double(r[0]) * z[0] + double(r[1]) * z[1] + double(r[2]) * z[2], r[0], r[1], r[2],
+           [&](bool ok, double rz, unsigned mx) { st.after_update(ok, rz, mx, a.tol, LEARNED ? a.stall_window : 0); });
+    if (st.status != PCG_MAXIT) break;
+    beta = st.coef;
+  }
+  // d = L^-T x^; x^ is FP64: rounding it to FP32 would cost up to cond(L_i) x
+  // 6e-8 of d_i at stiff vertices
+  if (live) {
+    for (int e = 0; e < 3; ++e) a.xh[3 * row + e] = x[e];
+    if (st.status != PCG_TIMEOUT) {
+      const double* l = a.Linv + 6 * (long long)row;
+      a.d[3 * row] = float(l[0] * x[0] + l[1] * x[1] + l[3] * x[2]);
+      a.d[3 * row + 1] = float(l[2] * x[1] + l[4] * x[2]);
+      a.d[3 * row + 2] = float(l[5] * x[2]);
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (LEARNED) ctrl->learned_iters = st.iters;
+    st.report(ctrl);
+  }
+  if constexpr (CLUSTER) cl_sync_shared();   // the others have read this CTA's last partial
+}
+
 using ScaledKernel = void (*)(PcgScaledArgs);
 ScaledKernel scaled_kernel(bool learned, int unroll) {
   if (learned) return unroll >= 2 ? k_pcg_scaled<true, 2> : k_pcg_scaled<true, 1>;
@@ -596,25 +1088,94 @@ ScaledKernel scaled_kernel(bool learned, int unroll) {
 
 }  // namespace
 
-int pcg_grid_size(int device) {
-  int sms = 0, per_sm = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg, PCG_TPB, 0);
-  if (per_sm < 1) per_sm = 1;
-  int co = sms * per_sm;
-  int want = 2 * sms;
-  return co < want ? co : want;
-}
-
 size_t pcg_scaled_partials(int V) { return 3ull * (size_t)((V + 31) / 32 + 1); }
 
-// Candidate launch shapes of the scaled PCG for V rows on `device`; shape 0
-// is the default. Every shape gives the same result bits.
+namespace {
+using PcgKernel = void (*)(PcgArgs);
+PcgKernel pcg_kernel(int rpt) { return rpt == 1 ? k_pcg<1> : rpt == 2 ? k_pcg<2> : rpt == 3 ? k_pcg<3> : k_pcg<0>; }
+
+// Resident kernel of a shape: threads per CTA rounded up to a compiled bound,
+// and with it the registers, which decide how many neighbours' p are kept
+// and how many slots are gathered at once.
+struct ResKernel { const void* f; int kq; bool compact; };
+template <bool L, bool F, bool C> ResKernel res_pick(int tpb) {
+  constexpr int KW = F ? 24 : RES_KQ;   // 256 threads leave registers for contact blocks' neighbours as well
+  if (tpb <= 256) return {(const void*)k_pcg_res<L, F, C, KW, F ? 8 : RES_KQ, 4, 256>, KW, res_compact(F, 256)};
+  if (tpb <= 512) return {(const void*)k_pcg_res<L, F, C, RES_KQ, 4, L ? 3 : 4, 512>, RES_KQ, res_compact(F, 512)};
+  if constexpr (!C) {   // a cluster's CTAs have at most 512
+    if constexpr (!F) if (tpb <= 896) return {(const void*)k_pcg_res<L, F, C, L ? 0 : RES_KQ, 4, L ? 2 : 3, 896>, L ? 0 : RES_KQ, res_compact(F, 896)};
+    return {(const void*)k_pcg_res<L, F, C, 0, 1, 2, 1024>, 0, res_compact(F, 1024)};
+  }
+  return {nullptr, 0, false};
+}
+ResKernel res_kernel(bool learned, bool far, bool cluster, int tpb) {
+  if (cluster) {
+    if (learned) return far ? res_pick<true, true, true>(tpb) : res_pick<true, false, true>(tpb);
+    return far ? res_pick<false, true, true>(tpb) : res_pick<false, false, true>(tpb);
+  }
+  if (learned) return far ? res_pick<true, true, false>(tpb) : res_pick<true, false, false>(tpb);
+  return far ? res_pick<false, true, false>(tpb) : res_pick<false, false, false>(tpb);
+}
+
+// Shared-memory and cluster attributes of a kernel, set on its first launch on
+// a device: setting them loads the kernel, and a process uses few of them.
+// Host-side calls only, so a first launch may be under stream capture.
+cudaError_t kernel_ready(const void* f, int smem, bool cluster) {
+  static std::mutex mu;
+  static std::vector<std::pair<int, const void*>> ready;
+  int d = 0;
+  cudaGetDevice(&d);
+  std::lock_guard<std::mutex> lock(mu);
+  for (const auto& r : ready) if (r.first == d && r.second == f) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (!e && cluster) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (!e) ready.push_back({d, f});
+  return e;
+}
+
+// SMs of the current device, and whether a cluster of 16 CTAs of the cluster
+// kernels' size (one to an SM) can run on it.
+struct PcgDevice { int sms = 0; bool cluster = false; };
+PcgDevice pcg_device() {
+  static std::mutex mu;
+  static PcgDevice dev[64];
+  int d = 0, sms = 0, n = 0;
+  cudaGetDevice(&d);
+  std::lock_guard<std::mutex> lock(mu);
+  PcgDevice& D = dev[d & 63];
+  if (D.sms) return D;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d);
+  const void* f = (const void*)k_pcg_cluster;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 16; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(16); cfg.blockDim = dim3(PCG_CLUSTER_TPB); cfg.dynamicSmemBytes = RES_SMEM; cfg.attrs = at; cfg.numAttrs = 1;
+  D.cluster = kernel_ready(f, RES_SMEM, true) == cudaSuccess && cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n >= 1;
+  cudaGetLastError();
+  D.sms = sms > 0 ? sms : 148;
+  return D;
+}
+
+// One cluster of `ctas` CTAs, or a cooperative grid of them.
+cudaError_t launch_ctas(const void* f, bool cluster, int ctas, int tpb, int smem, int smem_max, void** args, cudaStream_t s) {
+  cudaError_t e = kernel_ready(f, smem_max, cluster);
+  if (e) return e;
+  if (!cluster) return cudaLaunchCooperativeKernel(f, dim3(ctas), dim3(tpb), args, smem, s);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(ctas); cfg.blockDim = dim3(tpb); cfg.dynamicSmemBytes = smem; cfg.stream = s; cfg.attrs = at; cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, f, args);
+}
+
+// Launch shapes of the looping form (more rows than the resident form takes):
 //  - balanced: the 32-row slices spread evenly over the SMs (one or two
 //    CTAs per SM, each warp one slice per pass);
 //  - fixed CTA sizes of 256 and 512 threads up to the co-resident grid;
 // each with one and two column slots loaded ahead per thread.
-int pcg_scaled_shapes(int device, int V, bool learned, PcgShape* out, int max) {
+int streamed_shapes(int device, int V, bool learned, PcgShape* out, int max) {
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (sms < 1) sms = 1;
@@ -656,20 +1217,102 @@ int pcg_scaled_shapes(int device, int V, bool learned, PcgShape* out, int max) {
   return n;
 }
 
-cudaError_t launch_pcg_scaled(const PcgScaledArgs& a, bool learned, const PcgShape& sh, cudaStream_t s) {
-  if (sh.tpb < 32 || sh.tpb > SCALED_MAX_TPB || (sh.tpb & 31) || sh.grid < 1) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaMemsetAsync(&a.ctrl->bar_arrivals, 0, sizeof(unsigned long long), s);
-  if (e != cudaSuccess) return e;
-  void* args[] = {(void*)&a};
-  return cudaLaunchCooperativeKernel((void*)scaled_kernel(learned, sh.unroll), dim3(sh.grid), dim3(sh.tpb), args, 0, s);
+// CTAs and slices per CTA of the resident form; false when V has more rows
+// than it takes.
+//  - Up to 8,192 rows without contact blocks (1,024 with): one cluster. Its
+//    barriers cost a third of the grid's, but a row of another CTA is read at
+//    an eighth of the local shared-memory rate, which many-block rows or more
+//    rows to a CTA make the longer part.
+//  - Above: CTAs of 16 slices (8 with contact blocks, whose registers then
+//    hold 24 neighbours' p), so that a small system leaves SMs to other
+//    contexts' solves, and more slices once every SM has a CTA.
+bool res_layout(int V, bool far, bool& cluster, int& ctas, int& spc) {
+  const PcgDevice D = pcg_device();
+  const int ns = std::max(1, (V + 31) / 32), sms = std::min(D.sms, XR_MAX_CTAS);
+  cluster = D.cluster && ns <= (far ? 32 : 256);
+  if (cluster) {
+    ctas = 1;
+    while (ctas < 16 && ctas * 4 < ns) ctas *= 2;   // four warps to an SM while there are CTAs left
+    spc = (ns + ctas - 1) / ctas;
+    return true;
+  }
+  const int wide = far ? 8 : 16;
+  spc = std::max(std::min(wide, ns), (ns + sms - 1) / sms);
+  ctas = (ns + spc - 1) / spc;
+  return spc <= 32;
 }
 
-cudaError_t launch_pcg(const PcgArgs& a, int grid, cudaStream_t s) {
-  int need = (a.V + PCG_TPB - 1) / PCG_TPB;  // enough CTAs for one vertex per thread
-  if (need < 1) need = 1;
-  if (grid > need) grid = need;
-  void* args[] = {(void*)&a};
-  return cudaLaunchCooperativeKernel((void*)k_pcg, dim3(grid), dim3(PCG_TPB), args, 0, s);
+}  // namespace
+
+bool pcg_resident(int V) {
+  bool cluster; int ctas, spc;
+  return res_layout(V, true, cluster, ctas, spc) && res_layout(V, false, cluster, ctas, spc);
+}
+
+// Candidate launch shapes of the scaled PCG for V rows on `device`; shape 0
+// is the default. Every shape gives the same result bits. The resident form's
+// CTAs and warps follow from V and whether there are contact blocks; its
+// candidates are the shared memory (KiB) for the blocks of a system that does
+// not fit whole: all of it, or less, which leaves more to the L1 for the
+// gathers.
+int pcg_scaled_shapes(int device, int V, bool learned, PcgShape* out, int max) {
+  bool cluster; int ctas, spc;
+  if (!pcg_resident(V)) return streamed_shapes(device, V, learned, out, max);
+  res_layout(V, false, cluster, ctas, spc);
+  int n = 0;
+  for (int kb : {RES_SMEM / 1024, 160, 96})
+    if (n < max) out[n++] = PcgShape{32 * spc, ctas, kb};
+  return n;
+}
+
+cudaError_t launch_pcg_scaled(const PcgScaledArgs& args, bool learned, const PcgShape& sh, cudaStream_t s) {
+  if (sh.tpb < 32 || sh.tpb > SCALED_MAX_TPB || (sh.tpb & 31) || sh.grid < 1) return cudaErrorInvalidConfiguration;
+  cudaError_t e = cudaMemsetAsync(&args.ctrl->bar_arrivals, 0, sizeof(unsigned long long), s);
+  if (e != cudaSuccess) return e;
+  PcgScaledArgs a = args;
+  void* p[] = {(void*)&a};
+  if (!pcg_resident(a.V)) return cudaLaunchCooperativeKernel((void*)scaled_kernel(learned, sh.unroll), dim3(sh.grid), dim3(sh.tpb), p, 0, s);
+  bool cluster, far = a.xbegin || a.wmax > RES_KQ;
+  int ctas, spc, pub = 0;
+  ResKernel k;
+  int near = 0;
+  while (true) {   // a mesh without contact blocks keeps all its blocks on chip, or is treated as one with
+    res_layout(a.V, far, cluster, ctas, spc);
+    k = res_kernel(learned, far, cluster, 32 * spc);
+    near = std::max(a.wmax - (k.compact ? 1 : 0), 1);
+    pub = cluster ? 16 * 32 * spc * res_vectors(learned, far, k.kq) : 0;
+    if (far || pub + spc * res_warp_bytes(near) <= RES_SMEM) break;
+    far = true;
+  }
+  const int room = std::max(std::min(sh.unroll * 1024, RES_SMEM) - pub - 128 * spc, 0);
+  a.slots = far ? std::min(room / (1280 * spc), 64) : near;
+  const int smem = pub + spc * res_warp_bytes(a.slots);
+  return launch_ctas(k.f, cluster, ctas, 32 * spc, smem, RES_SMEM, p, s);
+}
+
+bool pcg_packed_rows(int V) {
+  const int ns = (V + 31) / 32, ctas = std::min(pcg_device().sms, XR_MAX_CTAS);
+  return (ns + ctas - 1) / ctas > 3 * PCG_WARPS;
+}
+
+cudaError_t launch_pcg(const PcgArgs& args, cudaStream_t s) {
+  const PcgDevice D = pcg_device();
+  PcgArgs a = args;
+  const int ns = (a.V + 31) / 32;
+  if (D.cluster && a.V <= 16 * PCG_CLUSTER_TPB) {
+    int C = 1;
+    while (C < 16 && C * 4 < ns) C *= 2;   // four warps to an SM while there are CTAs left
+    const int spc = (ns + C - 1) / C;
+    a.smem = 48 * 32 * spc + spc * std::min((RES_SMEM - 48 * 32 * spc) / spc, 16 * 1024);
+    void* p[] = {(void*)&a};
+    return launch_ctas((const void*)k_pcg_cluster, true, C, 32 * spc, a.smem, RES_SMEM, p, s);
+  }
+  const int ctas = std::min(D.sms, XR_MAX_CTAS);
+  const int spc = (ns + ctas - 1) / ctas, grid = (ns + spc - 1) / spc;
+  const int nw = std::min(spc, PCG_WARPS), rpt = (spc + nw - 1) / nw;
+  a.smem = nw * std::min(PCG_SMEM / nw, 24 * 1024);
+  void* p[] = {(void*)&a};
+  return launch_ctas((const void*)pcg_kernel(rpt <= 3 ? rpt : 0), false, grid, 32 * nw, a.smem, PCG_SMEM, p, s);
 }
 
 }  // namespace ando
