@@ -13,9 +13,9 @@
 // Pipeline: primitive boxes -> scene bounds -> 30-bit Morton codes of box
 // centres (index appended, so keys are unique) -> radix sort -> Karras
 // hierarchy (one thread per internal node) -> bottom-up refit in shared
-// memory (cut subtrees, then the nodes above the cut) -> one thread per query with an explicit stack; hits are compacted
-// with a warp ballot (one atomic per warp) and the pair list is then sorted so
-// its order does not depend on scheduling.
+// memory (cut subtrees, then the nodes above the cut) -> one thread per query with an explicit stack; overlapping
+// leaves are queued per warp and appended in batches, and the pair list is then
+// sorted so its order does not depend on scheduling.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
@@ -448,8 +448,22 @@ __device__ inline void emit(bool hit, int q, int prim, int2* out, int* count, in
 // pad), prims = triangles, skip incident triangles. kind 1: query = edge,
 // prims = edges, keep e1 < e2 without shared vertex. kind 2: query = edge,
 // prims = triangles, skip triangles that hold either end of the edge.
-__global__ void k_query(const double* x, const double* x1, const int* qprims, const int* qorder, int kind, int nq, float pad, int n,
+//
+// A query is a chain of dependent node loads, and there are only about 30
+// warps of them to an SM, so what a step waits for is the time. Overlapping
+// leaves therefore go into a shared-memory queue of the warp (ballots, no
+// memory round trip); only when it fills does the warp turn to them, 32 at
+// once: load the leaf, drop incident primitives, close the gaps, and append
+// what is left with one atomic. Testing each leaf where it is met and appending
+// each step's hits with an atomic of its own put two trips through L2 into
+// every step that met a leaf, all of them on the one counter.
+constexpr int QUEUE = 256;   // entries per warp; a step adds at most 128
+__global__ void __launch_bounds__(TPB) k_query(const double* x, const double* x1, const int* qprims, const int* qorder, int kind, int nq, float pad, int n,
                         const int4* leafv, const int* rank, const LbvhWide* wide, const Box* nodes, int2* out, int* count, int cap) {
+  __shared__ int2 queue[TPB / 32][QUEUE];
+  int2* const qu = queue[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  int held = 0;   // entries in the queue (uniform over the warp)
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   bool active = t < nq;
   const int q = active && qorder ? qorder[t] : t;
@@ -478,7 +492,7 @@ __global__ void k_query(const double* x, const double* x1, const int* qprims, co
   }
   // Depth-first traversal of the four-wide hierarchy: each step loads one
   // 128-byte node and tests its (up to) four child boxes; an overlapping leaf
-  // child is reported at once, the first overlapping internal child is entered
+  // child is queued, the first overlapping internal child is entered
   // and the others go on the stack. The binary hierarchy is at most 64 levels
   // deep with unique 64-bit keys, the four-wide one half that, so three
   // pushes per level fit 96 slots; an overflow would be reported through
@@ -495,23 +509,42 @@ __global__ void k_query(const double* x, const double* x1, const int* qprims, co
   const int qpos = active && kind == 1 ? rank[q] : -1;
   const bool single = active && n == 1;  // one primitive: the root (node 0) is its leaf
   int node = active && n > 1 ? 0 : -1;
-  auto accept = [&](int pos) {
-    const int4 lv = leafv[pos];
-    bool hit;
-    if (kind == 0) hit = lv.y != q && lv.z != q && lv.w != q;
-    else if (kind == 2) hit = lv.y != qa && lv.y != qc && lv.z != qa && lv.z != qc && lv.w != qa && lv.w != qc;
-    else hit = pos > qpos && lv.y != qa && lv.y != qc && lv.z != qa && lv.z != qc;
-    return hit ? lv.x : -1;
+  auto push = [&](bool hit, int pos) {
+    const unsigned mask = __ballot_sync(0xffffffffu, hit);
+    if (hit) qu[held + __popc(mask & ((1u << lane) - 1u))] = make_int2(q, pos);
+    held += __popc(mask);
   };
-  auto emit_pair = [&](int prim) {  // (lower, higher) edge index for the self query
-    const bool hit = prim >= 0;
-    const int a = kind == 1 && hit ? min(q, prim) : q, b = kind == 1 && hit ? max(q, prim) : prim;
-    emit(hit, a, b, out, count, cap);
+  auto flush = [&]() {
+    int kept = 0;
+    __syncwarp();
+    for (int k0 = 0; k0 < held; k0 += 32) {
+      bool hit = false;
+      int2 pr = make_int2(0, 0);
+      if (k0 + lane < held) {
+        pr = qu[k0 + lane];
+        const int4 lv = leafv[pr.y];
+        if (kind == 0) hit = lv.y != pr.x && lv.z != pr.x && lv.w != pr.x;
+        else {
+          const int a = qprims[2 * pr.x], b = qprims[2 * pr.x + 1];
+          hit = lv.y != a && lv.y != b && lv.z != a && lv.z != b && (kind == 1 || (lv.w != a && lv.w != b));
+        }
+        // (lower, higher) edge index for the self query
+        pr = kind == 1 ? make_int2(min(pr.x, lv.x), max(pr.x, lv.x)) : make_int2(pr.x, lv.x);
+      }
+      const unsigned mask = __ballot_sync(0xffffffffu, hit);
+      if (hit) qu[kept + __popc(mask & ((1u << lane) - 1u))] = pr;   // kept <= k0: only entries already read
+      kept += __popc(mask);
+      __syncwarp();
+    }
+    int base = 0;
+    if (lane == 0 && kept) base = atomicAdd(count, kept);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (int k = lane; k < kept; k += 32)
+      if (base + k < cap) out[base + k] = qu[k];
+    held = 0;
+    __syncwarp();
   };
-  if (__any_sync(0xffffffffu, single)) {
-    int prim = single && overlap(qb, nodes[0]) ? accept(0) : -1;
-    emit_pair(prim);
-  }
+  push(single && overlap(qb, nodes[0]), 0);
   while (__any_sync(0xffffffffu, node >= 0)) {
     int h[4] = {-1, -1, -1, -1};
     if (node >= 0) {
@@ -522,7 +555,7 @@ __global__ void k_query(const double* x, const double* x1, const int* qprims, co
       auto slot = [&](float lox, float loy, float loz, float hix, float hiy, float hiz, int c, int m, int& hk) {
         if (!(m > qpos && qb.lo[0] <= hix && qb.hi[0] >= lox && qb.lo[1] <= hiy && qb.hi[1] >= loy && qb.lo[2] <= hiz && qb.hi[2] >= loz))
           return;
-        if (c < 0) hk = accept(-c - 1);
+        if (c < 0) hk = -c - 1;
         else if (next < 0) next = c;
         else if (sp < STACK) stack[sp++] = c;
         else atomicAdd(count + 1, 1);
@@ -533,11 +566,11 @@ __global__ void k_query(const double* x, const double* x1, const int* qprims, co
       slot(f4.z, f4.w, f5.x, f5.y, f5.z, f5.w, ch.w, cm.w, h[3]);
       node = next >= 0 ? next : (sp > 0 ? stack[--sp] : -1);
     }
-    emit_pair(h[0]);
-    emit_pair(h[1]);
-    emit_pair(h[2]);
-    emit_pair(h[3]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) push(h[k] >= 0 && h[k] > qpos, h[k]);
+    if (held > QUEUE - 128) flush();
   }
+  if (held) flush();
 }
 
 // The four vertices of candidate pair (q, prim): kind 0 vertex q against
