@@ -12,6 +12,7 @@
 #include <atomic>
 #include <thread>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <numeric>
@@ -126,6 +127,7 @@ struct ando_ctx_s {
   // contacts
   DevBuf<int> det_counts, det_offsets;
   DevBuf<ContactDev> contacts;
+  DevBuf<unsigned char> contact_out;   // contacts as public records, for ando_compute_contacts*
   int ncontacts = 0, n_pe = 0;
   int* ctrl_host_count = nullptr;  // pinned int for small device -> host counts
   DevBuf<int> ekeys, ekeys_sorted, ebegin, eend, xflags, xkeys, xcols, xbegin, xend, nsel;
@@ -1973,19 +1975,16 @@ int contacts_out(ando_ctx c, ando_contact* out, int32_t capacity, int32_t* num_o
   *num_out = c->ncontacts;
   if (c->ncontacts == 0) return ANDO_OK;
   if (capacity == 0) return fail(ANDO_ERR_CAPACITY, "contact buffer too small");  // a size query: nothing to copy
-  std::vector<ContactDev> h(c->ncontacts);
-  CK(cudaMemcpyAsync(h.data(), c->contacts.p, sizeof(ContactDev) * c->ncontacts, cudaMemcpyDeviceToHost, c->stream));
+  // packed on the device, so the copy is the caller's records and nothing else
+  static_assert(sizeof(ando_contact) == CONTACT_OUT_BYTES && offsetof(ando_contact, gap) == offsetof(ContactDev, gap) &&
+                    offsetof(ando_contact, weights) == offsetof(ContactDev, w) && offsetof(ContactDev, kbar) == CONTACT_OUT_BYTES,
+                "ando_contact is the head of ContactDev");
+  const int n = std::min(capacity, c->ncontacts);
+  CK(c->contact_out.reserve(size_t(CONTACT_OUT_BYTES) * n));
+  launch_contacts_out(c->contacts.p, n, c->contact_out.p, c->stream);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(out, c->contact_out.p, size_t(CONTACT_OUT_BYTES) * n, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  int n = std::min(capacity, c->ncontacts);
-  for (int k = 0; k < n; ++k) {
-    const ContactDev& C = h[k];
-    ando_contact& o = out[k];
-    std::memset(&o, 0, sizeof(o));
-    o.type = C.type; o.idx0 = C.idx[0]; o.idx1 = C.idx[1]; o.idx2 = C.idx[2]; o.idx3 = C.idx[3];
-    o.rigid_body_index = C.rigid; o.vertex_count = C.count; o.gap = C.gap;
-    for (int q = 0; q < 3; ++q) { o.normal[q] = C.n[q]; o.witness_p[q] = C.wp[q]; o.witness_q[q] = C.wq[q]; o.barycentric[q] = C.bary[q]; }
-    for (int q = 0; q < 4; ++q) o.weights[q] = C.w[q];
-  }
   return c->ncontacts > capacity ? fail(ANDO_ERR_CAPACITY, "contact buffer too small") : ANDO_OK;
 }
 }  // namespace

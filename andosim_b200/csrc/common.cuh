@@ -76,6 +76,9 @@ struct ContactDev {
   int in_dom;
 };
 
+// The fields up to the weights, as the public ando_contact holds them.
+constexpr int CONTACT_OUT_BYTES = 168;
+
 // Contact contribution entry (contact c, local i, local j), sorted by row vertex.
 struct ContactEntry { int contact, li, lj, col; };
 

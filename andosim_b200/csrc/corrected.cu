@@ -173,6 +173,20 @@ __global__ void k_update_toi(int V, double* x, const double* ext, double ext_sca
 
 __global__ void k_toi_reset(unsigned long long* toi) { *toi = (unsigned long long)__double_as_longlong(1.0); }
 
+// The public record of a contact: the leading CONTACT_OUT_BYTES of ContactDev
+// with the alignment gap after its seven integers zeroed. One thread per
+// 8-byte word, so both sides move whole lines.
+__global__ void k_contacts_out(const ContactDev* cs, int n, unsigned long long* out) {
+  constexpr int W = CONTACT_OUT_BYTES / 8;
+  static_assert(sizeof(ContactDev) % 8 == 0 && CONTACT_OUT_BYTES % 8 == 0, "contact records are whole words");
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= (long long)n * W) return;
+  const int c = int(k / W), w = int(k - (long long)c * W);
+  unsigned long long v = reinterpret_cast<const unsigned long long*>(cs + c)[w];
+  if (w == 3) v &= 0xffffffffull;   // {count, gap}
+  out[k] = v;
+}
+
 }  // namespace
 
 void launch_drive_extent(const int* pin_vertex, const double* pin_target, int num_pins, const double* x, const double* v, int V, double dt,
@@ -205,6 +219,11 @@ void launch_toi_rigid(int V, const double* x, const double* ext, const RigidDev*
 void launch_update_toi(int V, double* x, const double* ext, double scale, const unsigned char* fixed, Ctrl* ctrl,
                        const unsigned long long* toi, cudaStream_t s) {
   k_update_toi<<<nblk(V > 0 ? 3ll * V : 1), TPB, 0, s>>>(V, x, ext, scale, fixed, ctrl, toi);
+}
+
+void launch_contacts_out(const ContactDev* cs, int n, void* out, cudaStream_t s) {
+  const long long words = (long long)n * (CONTACT_OUT_BYTES / 8);
+  if (n) k_contacts_out<<<(unsigned)((words + TPB - 1) / TPB), TPB, 0, s>>>(cs, n, static_cast<unsigned long long*>(out));
 }
 
 }  // namespace ando

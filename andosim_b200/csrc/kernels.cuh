@@ -101,6 +101,8 @@ void launch_pin_gather(const int* pin_vertex, int num_pins, const double* x, dou
 void launch_pin_interp(int num_pins, const double* start, const double* fin, double f, double* target, cudaStream_t s);
 void launch_pairs_to_contacts(const int2* vt, int nvt, const int2* ee, int nee, const int* tris, const int* edges, const double* x,
                               double gap_max, ContactDev* out, cudaStream_t s);
+// the n contacts as packed public records (ando_contact, CONTACT_OUT_BYTES each)
+void launch_contacts_out(const ContactDev* cs, int n, void* out, cudaStream_t s);
 void launch_swept_end(int V, const double* x, const float* d, const unsigned char* fixed, double scale, double lmax,
                       double* x1, double* ext, cudaStream_t s);
 void launch_toi_reset(unsigned long long* toi, cudaStream_t s);
