@@ -714,8 +714,8 @@ int detect_corrected(ando_ctx c, int nb, double gap_max, bool reuse = false) {
         CK(cudaStreamSynchronize(s));
       }
     }
-    CK(c->bvh_tri.contacts_finish(h, c->pairs, c->pk0, c->pk1, c->cub_tmp, &nvt, s));
-    CK(c->bvh_edge.contacts_finish(h + 3, c->pairs_ee, c->pk0, c->pk1, c->cub_tmp, &nee, s));
+    CK(c->bvh_tri.contacts_finish(h, c->V, c->pairs, c->pk0, c->pk1, c->cub_tmp, &nvt, s));
+    CK(c->bvh_edge.contacts_finish(h + 3, c->E, c->pairs_ee, c->pk0, c->pk1, c->cub_tmp, &nee, s));
     ph.launched(int(c->bvh_tri.launches + c->bvh_edge.launches - b0));
   }
   int nr = 0;

@@ -30,19 +30,21 @@ struct Lbvh {
   // nq queries, device; null: identity). A spatially coherent order keeps the
   // 32 traversals of a warp on similar paths; results do not depend on it.
   const int* qorder = nullptr;
-  DevBuf<LbvhBox> boxes, nodes; // primitive boxes; node boxes (internal [0,n-1), leaves [n-1, 2n-1))
+  DevBuf<LbvhBox> nodes;        // node boxes (internal [0,n-1), leaves [n-1, 2n-1))
   DevBuf<LbvhInner> inner;      // n-1 internal nodes: children and their last leaves (the build's topology)
   DevBuf<LbvhWide> wide;        // four-wide nodes: topology at build time, boxes by every refit
-  DevBuf<int> wflag, widx;      // per internal node: 1 at even depth (a four-wide node), its four-wide index
   DevBuf<int> wslot;            // per node: 4 * four-wide index + slot where its box is kept, -1 if nowhere
-  DevBuf<unsigned long long> keys, keys_sorted;
+  DevBuf<unsigned> codes, codes_sorted;   // Morton codes
+  // per internal node, low half: top node (above the refit's cut) or not, its
+  // number; high half: at even depth (a four-wide node), its four-wide index
+  DevBuf<unsigned long long> nflag, nnum;
   DevBuf<int> idx, order, parent, arrive, bounds;
   DevBuf<int> rank;             // sorted leaf position of each primitive (inverse of order)
   DevBuf<int4> topo;            // per internal node: first leaf, split, last leaf, parent
   DevBuf<int4> leafv;           // per sorted leaf: primitive and its vertices (-1 past the arity)
-  // refit schedule made at build time: nodes above the cut (flags, numbers,
-  // records), the cut subtrees as leaf ranges, meta = {top nodes, cut entries}
-  DevBuf<int> topflag, topnum, meta;
+  // refit schedule made at build time: records of the nodes above the cut, the
+  // cut subtrees as leaf ranges, meta = {top nodes, cut entries}
+  DevBuf<int> meta;
   DevBuf<int4> toprec;
   DevBuf<int2> cuts;
   DevBuf<int2> surv;            // candidates kept by the narrow phase of contacts_launch
@@ -75,7 +77,8 @@ struct Lbvh {
   // scratch.n at launch) must be grown and launched again before finishing.
   cudaError_t contacts_launch(const double* x, int kind, const int* qprims, int nq, float pad, double gap, DevBuf<int2>& scratch,
                               DevBuf<int>& counter, cudaStream_t s);
-  cudaError_t contacts_finish(const int count[3], DevBuf<int2>& out, DevBuf<unsigned long long>& k0, DevBuf<unsigned long long>& k1,
+  // (nq: number of queries, as at the launch)
+  cudaError_t contacts_finish(const int count[3], int nq, DevBuf<int2>& out, DevBuf<unsigned long long>& k0, DevBuf<unsigned long long>& k1,
                               DevBuf<unsigned char>& tmp, int* npairs, cudaStream_t s);
   // min over the swept-box candidates (x -> x1 = x + ext) of the pair's
   // conservative time of impact, min-reduced into *toi (IEEE bits of a

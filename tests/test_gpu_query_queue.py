@@ -21,3 +21,18 @@ def test_dense_overlap(oracle, abi, n, pad):
         assert len(vo) == len(x) * sc.num_triangles - 3 * sc.num_triangles
     np.testing.assert_array_equal(vg, vo)
     np.testing.assert_array_equal(eg, eo)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 9, 64, 65])
+def test_index_ranges(oracle, abi, k):
+    """Strips of k triangles: the sorted keys hold just the bits that the two index ranges need."""
+    v = np.array([[0.02 * i, 0.01 * (i % 2), 0.0] for i in range(k + 2)] + [[0.013, 0.004, 5e-5]])
+    t = np.array([[i, i + 1, i + 2] for i in range(k)], dtype=np.int32)
+    mat = dict(youngs_modulus=1e5, poisson_ratio=0.3, density=200.0, thickness=1e-3)
+    sc = scenes.Scene("strip", v, t, mat, scenes.cloth_params(), [], [])
+    x = v.astype(np.float32).astype(np.float64)
+    for pad in (0.0, 0.5):
+        vo, eo = oracle_pairs(oracle, sc, x, pad)
+        vg, eg = gpu_pairs(abi, sc, x, pad)
+        np.testing.assert_array_equal(vg, vo)
+        np.testing.assert_array_equal(eg, eo)
