@@ -18,7 +18,8 @@ using namespace net;
 
 constexpr int TPB = 256;
 constexpr int GRID = 296;          // fixed grid of the reducing kernels (2 CTAs per SM on 148 SMs)
-constexpr int PART = H * 2 * H + H;  // largest per-CTA partial (update layer: 64 x 128 weights + 64 bias)
+// floats of one CTA's weight-gradient partials over a whole backward pass
+constexpr int PART = NL * (H * 2 * H + H + H * FE + H + H * H + H) + (H + 1 + 2 * DE_IN + 2) + (H * FN + H);
 inline int nblk(long long n, int tpb = TPB) { return int((n + tpb - 1) / tpb); }
 
 // transposed (forward) layout of the dense matrices inside NetDev::wt
@@ -107,114 +108,177 @@ __global__ void k_node_feats(LsView s, const float* Ef, float* X) {
 }
 
 // --------------------------------------------------------------- row GEMM
-// Y[r, :N] = act(X[r, :] M + bias) + R1[r, :N] + R2[r, :N], X = [X1 | X2]
-// (K = K1 + K2 <= 128), M row-major [K][N], N in {64, 128}; Q gets the
-// pre-activation. 64 rows per CTA (M is staged in shared memory once per 64
-// rows), each thread 4 rows x N/16 outputs held in registers (N is a template
-// parameter so the accumulators never spill to local memory).
+// Y[r, :N] = act(X[r, :] M + bias) + R1[r, :N] + R2[r, :N], X an FP32 matrix of
+// K <= 64 columns (with `mask`, entries whose mask entry is not positive read
+// as zero: the relu's backward), M row-major [K][N], N in {64, 128}; Q gets the
+// pre-activation. 64 rows per CTA, each thread 4 rows x N/16 outputs in
+// registers. Both operands sit in shared memory so that a step of k takes
+// N/64 + 1 16-byte reads without bank conflicts for its 4 N/16 products: X
+// transposed, a thread's outputs as groups of 4 columns 64 apart. With scalar
+// reads of X and M shared memory bound it.
 template <int N>
-__global__ void __launch_bounds__(TPB) k_gemm(int V, const float* X1, int ld1, int K1, const float* X2, int ld2, int K2, const float* M,
-                                              const float* bias, const float* R1, int ldr1, const float* R2, int ldr2, float* Q,
-                                              float* Y, int relu) {
-  constexpr int ROWS = 64, PER = N / 16;
-  extern __shared__ float sm[];
-  const int K = K1 + K2, XS = K + 1;
+__global__ void __launch_bounds__(TPB) k_gemm(int V, const float* X, int ldx, const float* mask, int K, const float* M, const float* bias,
+                                              const float* R1, int ldr1, const float* R2, int ldr2, float* Q, float* Y, int relu) {
+  constexpr int ROWS = 64, PER = N / 16, XS = ROWS + 4;
+  extern __shared__ __align__(16) float sm[];
   float* Ms = sm;                // K x N
-  float* Xs = sm + K * N;        // ROWS x XS
+  float* Xt = sm + K * N;        // K x XS, transposed
   const int r0 = blockIdx.x * ROWS;
-  for (int i = threadIdx.x; i < K * N; i += TPB) Ms[i] = M[i];
-  for (int i = threadIdx.x; i < ROWS * K; i += TPB) {
-    int r = i / K, k = i % K, row = r0 + r;
-    float v = 0.f;
-    if (row < V) v = k < K1 ? X1[(long long)row * ld1 + k] : X2[(long long)row * ld2 + (k - K1)];
-    Xs[r * XS + k] = v;
+  for (int i = threadIdx.x; i < K * N / 4; i += TPB) reinterpret_cast<float4*>(Ms)[i] = reinterpret_cast<const float4*>(M)[i];
+  for (int i = threadIdx.x; i < ROWS * K / 4; i += TPB) {
+    const int r = i % ROWS, k = 4 * (i / ROWS), row = r0 + r;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row < V) {
+      v = *reinterpret_cast<const float4*>(X + (long long)row * ldx + k);
+      if (mask) {
+        const float4 q = *reinterpret_cast<const float4*>(mask + (long long)row * ldx + k);
+        v = make_float4(q.x > 0.f ? v.x : 0.f, q.y > 0.f ? v.y : 0.f, q.z > 0.f ? v.z : 0.f, q.w > 0.f ? v.w : 0.f);
+      }
+    }
+    Xt[k * XS + r] = v.x; Xt[(k + 1) * XS + r] = v.y; Xt[(k + 2) * XS + r] = v.z; Xt[(k + 3) * XS + r] = v.w;
   }
   __syncthreads();
-  // 16 row groups of 4 rows x 16 column groups of PER columns
-  const int r = (threadIdx.x / 16) * 4, c0 = (threadIdx.x % 16) * PER;
+  const int r = (threadIdx.x / 16) * 4, c0 = (threadIdx.x % 16) * 4;   // columns c0.. and, N = 128, c0 + 64..
   float acc[4][PER];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int j = 0; j < PER; ++j) acc[a][j] = 0.f;
+#pragma unroll 4
   for (int k = 0; k < K; ++k) {
-    float xv[4];
+    const float4 xv4 = *reinterpret_cast<const float4*>(Xt + k * XS + r);
+    const float xv[4] = {xv4.x, xv4.y, xv4.z, xv4.w};
 #pragma unroll
-    for (int a = 0; a < 4; ++a) xv[a] = Xs[(r + a) * XS + k];
-    const float* mr = Ms + k * N + c0;
+    for (int g = 0; g < PER / 4; ++g) {
+      const float4 m4 = *reinterpret_cast<const float4*>(Ms + k * N + 64 * g + c0);
+      const float m[4] = {m4.x, m4.y, m4.z, m4.w};
 #pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      float m = mr[j];
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int a = 0; a < 4; ++a) acc[a][j] += xv[a] * m;
+        for (int a = 0; a < 4; ++a) acc[a][4 * g + j] += xv[a] * m[j];
     }
   }
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
-    int row = r0 + r + a;
+    const int row = r0 + r + a;
     if (row >= V) continue;
 #pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      int c = c0 + j;
-      float q = acc[a][j] + (bias ? bias[c] : 0.f);
-      if (Q) Q[(long long)row * N + c] = q;
-      float y = relu ? fmaxf(q, 0.f) : q;
-      if (R1) y += R1[(long long)row * ldr1 + c];
-      if (R2) y += R2[(long long)row * ldr2 + c];
-      Y[(long long)row * N + c] = y;
+    for (int g = 0; g < PER / 4; ++g) {
+      const int c = 64 * g + c0;
+      float y[4], q[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        q[j] = acc[a][4 * g + j] + (bias ? bias[c + j] : 0.f);
+        y[j] = relu ? fmaxf(q[j], 0.f) : q[j];
+      }
+      if (Q) *reinterpret_cast<float4*>(Q + (long long)row * N + c) = make_float4(q[0], q[1], q[2], q[3]);
+      if (R1) { const float4 t = *reinterpret_cast<const float4*>(R1 + (long long)row * ldr1 + c); y[0] += t.x; y[1] += t.y; y[2] += t.z; y[3] += t.w; }
+      if (R2) { const float4 t = *reinterpret_cast<const float4*>(R2 + (long long)row * ldr2 + c); y[0] += t.x; y[1] += t.y; y[2] += t.z; y[3] += t.w; }
+      *reinterpret_cast<float4*>(Y + (long long)row * N + c) = make_float4(y[0], y[1], y[2], y[3]);
     }
   }
 }
 
 // Weight gradient partials: part[g] = [dQ^T X (64 x K, row-major) ; sum dQ (64)]
-// over CTA g's contiguous row range.
-__global__ void __launch_bounds__(TPB) k_wgrad(int V, const float* dQ, int ldq, const float* X1, int ld1, int K1, const float* X2, int ld2,
-                                               int K2, float* part) {
-  __shared__ float dqs[32 * H];
-  __shared__ float xs[32 * (2 * H + 1)];
-  const int K = K1 + K2, XS = K + 1;
+// over CTA g's contiguous row range, X = [X1 | X2] (K = K1 + K2 in {8, 64,
+// 128}). With `mask`, dQ reads as zero where the mask entry is not positive. 32
+// rows at a time in shared memory; a thread owns 4 rows of 4 or 8 outputs and
+// reads a row's factors with two or three 16-byte loads, where a scalar read
+// per product bound it (46 us a call at 8,192 rows).
+template <int K1, int K2>
+__global__ void __launch_bounds__(TPB) k_wgrad(int V, const float* dQ, const float* mask, const float* X1, const float* X2, float* part) {
+  constexpr int K = K1 + K2, ROWS = 32;
+  constexpr int KT = K == 128 ? 8 : 4, KG = K / KT;       // columns of a thread, column groups
+  constexpr int OT = 64 * KG >= 4 * TPB ? 4 : 1;          // output rows of a thread
+  __shared__ __align__(16) float dqs[ROWS * H];
+  __shared__ __align__(16) float xs[ROWS * K];
   const int rows_per = (V + gridDim.x - 1) / gridDim.x;
-  const int rb = blockIdx.x * rows_per, re = min(V, rb + rows_per);
-  const int o = threadIdx.x >> 2, kq = threadIdx.x & 3, kw = K / 4, kb = kq * kw;
-  float acc[32], bacc = 0.f;
-  for (int j = 0; j < 32; ++j) acc[j] = 0.f;
-  for (int c0 = rb; c0 < re; c0 += 32) {
+  const int rb = min(V, (int)blockIdx.x * rows_per), re = min(V, rb + rows_per);
+  const int kg = threadIdx.x % KG, o = (threadIdx.x / KG) * OT;
+  const bool active = o < H;                              // K = 8 needs half the threads
+  float acc[OT][KT], bacc[OT];
+#pragma unroll
+  for (int a = 0; a < OT; ++a) {
+    bacc[a] = 0.f;
+#pragma unroll
+    for (int j = 0; j < KT; ++j) acc[a][j] = 0.f;
+  }
+  for (int c0 = rb; c0 < re; c0 += ROWS) {
+    const int nr = min(ROWS, re - c0);
     __syncthreads();
-    for (int i = threadIdx.x; i < 32 * H; i += TPB) {
-      int r = i / H, c = i % H, row = c0 + r;
-      dqs[i] = row < re ? dQ[(long long)row * ldq + c] : 0.f;
+    for (int i = threadIdx.x; i < nr * H / 4; i += TPB) {
+      float4 v = reinterpret_cast<const float4*>(dQ + (long long)c0 * H)[i];
+      if (mask) {
+        const float4 q = reinterpret_cast<const float4*>(mask + (long long)c0 * H)[i];
+        v = make_float4(q.x > 0.f ? v.x : 0.f, q.y > 0.f ? v.y : 0.f, q.z > 0.f ? v.z : 0.f, q.w > 0.f ? v.w : 0.f);
+      }
+      reinterpret_cast<float4*>(dqs)[i] = v;
     }
-    for (int i = threadIdx.x; i < 32 * K; i += TPB) {
-      int r = i / K, k = i % K, row = c0 + r;
-      float v = 0.f;
-      if (row < re) v = k < K1 ? X1[(long long)row * ld1 + k] : X2[(long long)row * ld2 + (k - K1)];
-      xs[r * XS + k] = v;
+    for (int i = threadIdx.x; i < nr * K1 / 4; i += TPB) {
+      const int r = i / (K1 / 4), k = i % (K1 / 4);
+      reinterpret_cast<float4*>(xs + r * K)[k] = reinterpret_cast<const float4*>(X1 + (long long)(c0 + r) * K1)[k];
     }
+    if constexpr (K2 > 0)
+      for (int i = threadIdx.x; i < nr * K2 / 4; i += TPB) {
+        const int r = i / (K2 / 4), k = i % (K2 / 4);
+        reinterpret_cast<float4*>(xs + r * K + K1)[k] = reinterpret_cast<const float4*>(X2 + (long long)(c0 + r) * K2)[k];
+      }
     __syncthreads();
-    for (int r = 0; r < 32; ++r) {
-      float g = dqs[r * H + o];
-      if (kq == 0) bacc += g;
-      for (int j = 0; j < kw; ++j) acc[j] += g * xs[r * XS + kb + j];
+    if (!active) continue;
+#pragma unroll 4
+    for (int r = 0; r < nr; ++r) {
+      float g[OT];
+      if constexpr (OT == 4) {
+        const float4 g4 = *reinterpret_cast<const float4*>(dqs + r * H + o);
+        g[0] = g4.x; g[1] = g4.y; g[2] = g4.z; g[3] = g4.w;
+      } else g[0] = dqs[r * H + o];
+#pragma unroll
+      for (int a = 0; a < OT; ++a) bacc[a] += g[a];
+#pragma unroll
+      for (int q = 0; q < KT / 4; ++q) {
+        const float4 x4 = *reinterpret_cast<const float4*>(xs + r * K + 64 * q + 4 * kg);
+        const float xv[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+        for (int a = 0; a < OT; ++a)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[a][4 * q + j] += g[a] * xv[j];
+      }
     }
   }
-  float* p = part + (long long)blockIdx.x * PART;
-  for (int j = 0; j < kw; ++j) p[o * K + kb + j] = acc[j];
-  if (kq == 0) p[H * K + o] = bacc;
+  if (!active) return;
+  float* p = part + (long long)blockIdx.x * (H * K + H);
+#pragma unroll
+  for (int a = 0; a < OT; ++a) {
+#pragma unroll
+    for (int q = 0; q < KT / 4; ++q)
+      *reinterpret_cast<float4*>(p + (o + a) * K + 64 * q + 4 * kg) =
+          make_float4(acc[a][4 * q], acc[a][4 * q + 1], acc[a][4 * q + 2], acc[a][4 * q + 3]);
+    if (kg == 0) p[H * K + o + a] = bacc[a];
+  }
 }
 
-// out[i] (+)= sum over g of part[g * PART + off + i], g in order.
-__global__ void k_reduce_parts(const float* part, int G, int off, int n, float* out, int accumulate) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// Every weight gradient of a backward pass from its partials, in one launch:
+// out[i] = sum over g < G of base[g stride + i], i < n; eight threads take every
+// eighth partial each, and their sums are added in order.
+struct Reduction { const float* base; float* out; int n, stride, G, first; };   // first: its first block
+constexpr int MAX_REDUCTIONS = 2 + 3 * NL;
+struct Reductions { Reduction r[MAX_REDUCTIONS]; int count; };
+__global__ void __launch_bounds__(TPB) k_reduce_all(const Reductions R) {
+  __shared__ float part[8][32];
+  int k = 0;
+  while (k + 1 < R.count && (int)blockIdx.x >= R.r[k + 1].first) ++k;
+  const Reduction q = R.r[k];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = 32 * ((int)blockIdx.x - q.first) + lane;
   float s = 0.f;
-  for (int g = 0; g < G; ++g) s += part[(long long)g * PART + off + i];
-  out[i] = accumulate ? out[i] + s : s;
-}
-
-__global__ void k_relu_mask(long long n, const float* dh, const float* q, float* dq) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  dq[i] = q[i] > 0.f ? dh[i] : 0.f;
+  if (i < q.n)
+    for (int g = w; g < q.G; g += 8) s += q.base[(long long)g * q.stride + i];
+  part[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && i < q.n) {
+    float t = part[0][lane];
+    for (int g = 1; g < 8; ++g) t += part[g][lane];
+    q.out[i] = t;
+  }
 }
 
 // ------------------------------------------------------------ messages
@@ -323,7 +387,10 @@ __global__ void __launch_bounds__(MSG_ROWS_TPB) k_msg_rows(LsView s, const float
 
 // Backward of k_msg_fwd. Row j gathers over its slots (j, i) the messages it
 // sent to i (transpose slot (i, j) holds e_ij): du_j, and per-CTA partials of
-// dE (64 x FE) and dc (64).
+// dE (64 x FE) and dc (64). As in the forward, a row of at most MSG_SLOTS slots
+// loads its columns, transpose slots and degrees one per lane and then every
+// neighbour's dm at once, where one slot after another was a chain of four
+// dependent loads each.
 __global__ void __launch_bounds__(TPB) k_msg_bwd(LsView s, const float* u, const float* Ef, const float* Ew, const float* cb,
                                                  const float* dm, int lddm, float* du, float* part) {
   __shared__ float red[TPB / 32][H * (FE + 1)];
@@ -336,30 +403,55 @@ __global__ void __launch_bounds__(TPB) k_msg_bwd(LsView s, const float* u, const
   float gc0 = 0.f, gc1 = 0.f;
   for (int j = gw; j < s.V; j += nw) {
     float d0 = 0.f, d1 = 0.f;
-    const float uj0 = u[(long long)j * H + c0], uj1 = u[(long long)j * H + c1];
-    for (int k = s.rowptr[j]; k < s.rowptr[j + 1]; ++k) {
-      int i = s.cols[k];
-      if (i == j) continue;
-      int kT = s.slot_T[k];
-      int deg = s.rowptr[i + 1] - s.rowptr[i] - 1;
-      if (deg <= 0) continue;
-      const float* e = Ef + (long long)kT * FES;
-      float t0 = uj0 + b0, t1 = uj1 + b1;
-      for (int f = 0; f < FE; ++f) { float ef = e[f]; t0 += e0[f] * ef; t1 += e1[f] * ef; }
-      float inv = 1.f / float(deg);
-      float m0 = t0 > 0.f ? dm[(long long)i * lddm + c0] * inv : 0.f;
-      float m1 = t1 > 0.f ? dm[(long long)i * lddm + c1] * inv : 0.f;
+    const float2 uj = *reinterpret_cast<const float2*>(u + (long long)j * H + c0);
+    const int kb = s.rowptr[j], ns = s.rowptr[j + 1] - kb;
+    auto slot = [&](int deg, float2 dmi, float4 q0, float4 q1, float4 q2) {
+      const float ef[FE] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y};
+      float t0 = uj.x + b0, t1 = uj.y + b1;
+#pragma unroll
+      for (int f = 0; f < FE; ++f) { t0 += e0[f] * ef[f]; t1 += e1[f] * ef[f]; }
+      const float inv = 1.f / float(deg);
+      const float m0 = t0 > 0.f ? dmi.x * inv : 0.f;
+      const float m1 = t1 > 0.f ? dmi.y * inv : 0.f;
       d0 += m0; d1 += m1;
-      for (int f = 0; f < FE; ++f) { float ef = e[f]; g0[f] += m0 * ef; g1[f] += m1 * ef; }
+#pragma unroll
+      for (int f = 0; f < FE; ++f) { g0[f] += m0 * ef[f]; g1[f] += m1 * ef[f]; }
       gc0 += m0; gc1 += m1;
+    };
+    if (ns <= MSG_SLOTS) {
+      const int il = lane < ns ? s.cols[kb + lane] : -1;
+      const int kTl = lane < ns ? s.slot_T[kb + lane] : 0;
+      const int degl = il >= 0 ? s.rowptr[il + 1] - s.rowptr[il] - 1 : 0;
+      float2 dv[MSG_SLOTS];
+#pragma unroll
+      for (int sl = 0; sl < MSG_SLOTS; ++sl) {
+        const int i = __shfl_sync(0xffffffffu, il, sl);
+        dv[sl] = sl < ns && i != j ? *reinterpret_cast<const float2*>(dm + (long long)i * lddm + c0) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int sl = 0; sl < MSG_SLOTS; ++sl) {
+        const int i = __shfl_sync(0xffffffffu, il, sl), kT = __shfl_sync(0xffffffffu, kTl, sl), deg = __shfl_sync(0xffffffffu, degl, sl);
+        if (sl < ns && i != j && deg > 0) {  // uniform over the warp
+          const float4* e4 = reinterpret_cast<const float4*>(Ef + (long long)kT * FES);
+          slot(deg, dv[sl], e4[0], e4[1], e4[2]);
+        }
+      }
+    } else {
+      for (int k = kb; k < kb + ns; ++k) {
+        const int i = s.cols[k];
+        if (i == j) continue;
+        const int deg = s.rowptr[i + 1] - s.rowptr[i] - 1;
+        if (deg <= 0) continue;
+        const float4* e4 = reinterpret_cast<const float4*>(Ef + (long long)s.slot_T[k] * FES);
+        slot(deg, *reinterpret_cast<const float2*>(dm + (long long)i * lddm + c0), e4[0], e4[1], e4[2]);
+      }
     }
-    du[(long long)j * H + c0] = d0;
-    du[(long long)j * H + c1] = d1;
+    *reinterpret_cast<float2*>(du + (long long)j * H + c0) = make_float2(d0, d1);
   }
   for (int f = 0; f < FE; ++f) { red[warp][c0 * FE + f] = g0[f]; red[warp][c1 * FE + f] = g1[f]; }
   red[warp][H * FE + c0] = gc0; red[warp][H * FE + c1] = gc1;
   __syncthreads();
-  float* p = part + (long long)blockIdx.x * PART;
+  float* p = part + (long long)blockIdx.x * (H * (FE + 1));
   for (int i = threadIdx.x; i < H * (FE + 1); i += TPB) {
     float v = 0.f;
     for (int w = 0; w < TPB / 32; ++w) v += red[w][i];
@@ -434,6 +526,7 @@ __global__ void k_build_S(LsView s, const float* zv, const float* ab, float* S, 
 // y = M v row by row (warp per row), static pattern and optional extra segment.
 __global__ void k_spmv(int V, const int* rowptr, const int* cols, const float* val, const int* xbegin, const int* xend, const int* xcols,
                        const float* xval, const float* v, float* y) {
+  v += 3ll * V * blockIdx.y; y += 3ll * V * blockIdx.y;   // one probe vector per grid row
   const int lane = threadIdx.x & 31, comp = lane >> 3, bi = lane & 7;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   for (int row = gw; row < V; row += nw) {
@@ -484,49 +577,52 @@ __global__ void k_loss_terms(int V, int P, const float* r, const float* y, const
   }
 }
 __global__ void k_loss_final(const double* parts, int G, int P, const double* pnorm, double* loss) {
-  if (threadIdx.x || blockIdx.x) return;
   double L = 0.0;
   for (int p = 0; p < P; ++p) {
     double T = 0.0;
-    for (int g = 0; g < G; ++g) T += parts[(long long)g * P + p];
+    for (int g = threadIdx.x; g < G; g += 32) T += parts[(long long)g * P + p];
+    for (int o = 16; o; o >>= 1) T += __shfl_xor_sync(0xffffffffu, T, o);
     L += 1.0 + T / pnorm[p];
   }
-  *loss = L / P;
+  if (threadIdx.x == 0) *loss = L / P;
 }
 
 // Gradient of the loss w.r.t. delta_i (through the softplus: dzv) and the
 // edge coefficients (dab), with gy_p = 2 (w_p - r_p) / (n_p P).
+// One thread per slot (i, j): the edge's for j > i, the vertex's on the own slot.
 __global__ void k_coef_grad(LsView s, int P, const float* r, const float* w, const double* pnorm, const float* zv, const float* ab,
                             float* dzv, float* dab) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.V) return;
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= s.nnzb) return;
+  const int i = s.slot_row[k], j = s.cols[k];
+  if (j < i) return;
   const long long n3 = 3ll * s.V;
   auto gy = [&](int p, int v, int c) { return float(2.0 * (double(w[n3 * p + 3 * v + c]) - r[n3 * p + 3 * v + c]) / (pnorm[p] * P)); };
   float gbi = 0.f;
-  for (int p = 0; p < P; ++p)
-    for (int c = 0; c < 3; ++c) gbi += gy(p, i, c) * r[n3 * p + 3 * i + c];
-  dzv[i] = gbi * sigm(zv[i]);
-  for (int k = s.rowptr[i]; k < s.rowptr[i + 1]; ++k) {
-    int j = s.cols[k];
-    if (j <= i) continue;
-    const float* A = s.valh + 9ll * k;
-    float AtA[9];
-    for (int a = 0; a < 3; ++a)
-      for (int b = 0; b < 3; ++b) AtA[3 * a + b] = A[a] * A[b] + A[3 + a] * A[3 + b] + A[6 + a] * A[6 + b];
-    float dc = 0.f, gbb = 0.f;
-    for (int p = 0; p < P; ++p) {
-      float gi[3], gj[3], ri[3], rj[3];
-      for (int c = 0; c < 3; ++c) { gi[c] = gy(p, i, c); gj[c] = gy(p, j, c); ri[c] = r[n3 * p + 3 * i + c]; rj[c] = r[n3 * p + 3 * j + c]; }
-      for (int a = 0; a < 3; ++a)
-        for (int b = 0; b < 3; ++b) {
-          dc += gi[a] * A[3 * a + b] * rj[b] + gj[b] * A[3 * a + b] * ri[a];
-          gbb += gj[a] * AtA[3 * a + b] * rj[b];
-        }
-    }
-    float a = ab[2ll * k], b = ab[2ll * k + 1];
-    dab[2ll * k] = dc * b + 2.f * a * gbi;
-    dab[2ll * k + 1] = dc * a + 2.f * b * gbb;
+  if (j == i) {
+    for (int p = 0; p < P; ++p)
+      for (int c = 0; c < 3; ++c) gbi += gy(p, i, c) * r[n3 * p + 3 * i + c];
+    dzv[i] = gbi * sigm(zv[i]);
+    return;
   }
+  const float* A = s.valh + 9ll * k;
+  float AtA[9];
+  for (int a = 0; a < 3; ++a)
+    for (int b = 0; b < 3; ++b) AtA[3 * a + b] = A[a] * A[b] + A[3 + a] * A[3 + b] + A[6 + a] * A[6 + b];
+  float dc = 0.f, gbb = 0.f;
+  for (int p = 0; p < P; ++p) {
+    float gi[3], gj[3], ri[3], rj[3];
+    for (int c = 0; c < 3; ++c) { gi[c] = gy(p, i, c); gj[c] = gy(p, j, c); ri[c] = r[n3 * p + 3 * i + c]; rj[c] = r[n3 * p + 3 * j + c]; }
+    for (int c = 0; c < 3; ++c) gbi += gi[c] * ri[c];
+    for (int a = 0; a < 3; ++a)
+      for (int b = 0; b < 3; ++b) {
+        dc += gi[a] * A[3 * a + b] * rj[b] + gj[b] * A[3 * a + b] * ri[a];
+        gbb += gj[a] * AtA[3 * a + b] * rj[b];
+      }
+  }
+  float a = ab[2ll * k], b = ab[2ll * k + 1];
+  dab[2ll * k] = dc * b + 2.f * a * gbi;
+  dab[2ll * k + 1] = dc * a + 2.f * b * gbb;
 }
 
 // Backward of k_dec_fwd: dh_r, and per-CTA partials of ddv (64), ddv0 (1),
@@ -582,7 +678,7 @@ __global__ void __launch_bounds__(TPB) k_dec_bwd(LsView s, const float* h, const
   if (lane < FE) { q[A0 + 2 * H + lane] = gAe; q[B0 + 2 * H + lane] = gBe; }
   if (lane == 0) { q[NP - 2] = gde0; q[NP - 1] = gde1; }
   __syncthreads();
-  float* p = part + (long long)blockIdx.x * PART;
+  float* p = part + (long long)blockIdx.x * NP;
   for (int i = threadIdx.x; i < NP; i += TPB) {
     float v = 0.f;
     for (int w2 = 0; w2 < TPB / 32; ++w2) v += red[w2][i];
@@ -600,8 +696,8 @@ __global__ void k_adam(float* w, float* m1, float* m2, const float* g, int n, fl
   w[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
 }
 
-void gemm(int V, const float* X1, int ld1, int K1, const float* X2, int ld2, int K2, const float* M, int N, const float* bias,
-          const float* R1, int ldr1, const float* R2, int ldr2, float* Q, float* Y, int relu, cudaStream_t s) {
+void gemm(int V, const float* X, int ldx, const float* mask, int K, const float* M, int N, const float* bias, const float* R1, int ldr1,
+          const float* R2, int ldr2, float* Q, float* Y, int relu, cudaStream_t s) {
   static std::atomic<unsigned> attr{0};  // one bit per device (steps of several contexts may run on host threads)
   int dev = 0;
   cudaGetDevice(&dev);
@@ -610,21 +706,20 @@ void gemm(int V, const float* X1, int ld1, int K1, const float* X2, int ld2, int
     cudaFuncSetAttribute(k_gemm<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
     attr.fetch_or(1u << dev);
   }
-  int K = K1 + K2;
-  size_t smem = sizeof(float) * (size_t(K) * N + 64 * (K + 1));
-  if (N == 64) k_gemm<64><<<nblk(V, 64), TPB, smem, s>>>(V, X1, ld1, K1, X2, ld2, K2, M, bias, R1, ldr1, R2, ldr2, Q, Y, relu);
-  else k_gemm<128><<<nblk(V, 64), TPB, smem, s>>>(V, X1, ld1, K1, X2, ld2, K2, M, bias, R1, ldr1, R2, ldr2, Q, Y, relu);
+  size_t smem = sizeof(float) * (size_t(K) * N + size_t(K) * 68);
+  if (N == 64) k_gemm<64><<<nblk(V, 64), TPB, smem, s>>>(V, X, ldx, mask, K, M, bias, R1, ldr1, R2, ldr2, Q, Y, relu);
+  else k_gemm<128><<<nblk(V, 64), TPB, smem, s>>>(V, X, ldx, mask, K, M, bias, R1, ldr1, R2, ldr2, Q, Y, relu);
 }
-void reduce(const float* part, int off, int n, float* out, cudaStream_t s) {
-  k_reduce_parts<<<nblk(n), TPB, 0, s>>>(part, GRID, off, n, out, 0);
-}
+// CTAs of k_wgrad: one to an SM until each has a few hundred rows (every CTA
+// writes a whole partial), then two.
+int wgrad_grid(int V) { return V < 65536 ? GRID / 2 : GRID; }
 
 }  // namespace
 
 size_t learned_work_floats(int V, int nnzb, bool training) {
   size_t VH = size_t(V) * H;
   size_t n = size_t(V) * FN + size_t(nnzb) * FES + VH * (NL + 1) + 3 * VH * NL + VH + V + 2ull * nnzb;
-  if (training) n += 7 * VH + V + 2ull * nnzb + size_t(GRID) * PART;
+  if (training) n += 5 * VH + V + 2ull * nnzb + size_t(GRID) * PART + 4 * MAX_REDUCTIONS;
   return n + 4 * 64;  // every buffer starts on a 16-byte boundary (vector loads and stores)
 }
 
@@ -638,19 +733,20 @@ void learned_work_carve(LearnedWork& w, float* base, int V, int nnzb, bool train
   for (int l = 0; l < NL; ++l) { w.u[l] = take(VH); w.m[l] = take(VH); w.q[l] = take(VH); }
   w.q0 = take(VH); w.zv = take(V); w.ab = take(2ull * nnzb);
   if (training) {
-    w.dh = take(VH); w.dh2 = take(VH); w.du = take(VH); w.dhm = take(2 * VH); w.dq = take(VH);
-    w.dzv = take(V); w.dab = take(2ull * nnzb); w.part = take(size_t(GRID) * PART);
+    w.dh = take(VH); w.dh2 = take(VH); w.du = take(VH); w.dhm = take(2 * VH);
+    w.dzv = take(V); w.dab = take(2ull * nnzb); w.part = take(size_t(GRID) * PART + 4 * MAX_REDUCTIONS);
   } else {
-    w.dh = w.dh2 = w.du = w.dhm = w.dq = w.dzv = w.dab = w.part = nullptr;
+    w.dh = w.dh2 = w.du = w.dhm = w.dzv = w.dab = w.part = nullptr;
   }
 }
 
 // B images of the hidden layers: per layer U (64 x 64) then W (64 x 128)
 constexpr int BIMG_U = 0, BIMG_W = H * H, BIMG_LSIZE = BIMG_W + H * 2 * H;
-constexpr size_t BIMG_OFF = (size_t(NPARAM) + WT_SIZE + 3) / 4 * 4;  // floats; 16-byte aligned
+constexpr size_t WT_OFF = (size_t(NPARAM) + 3) / 4 * 4;      // floats; both 16-byte aligned (vector loads)
+constexpr size_t BIMG_OFF = (WT_OFF + WT_SIZE + 3) / 4 * 4;
 size_t net_dev_floats() { return BIMG_OFF + size_t(NL) * BIMG_LSIZE / 2; }
 void net_dev_carve(NetDev& n, float* base) {
-  n.wq = base; n.wt = base + NPARAM;
+  n.wq = base; n.wt = base + WT_OFF;
   n.bimg = reinterpret_cast<unsigned short*>(base + BIMG_OFF);
 }
 
@@ -671,7 +767,7 @@ void learned_forward(const LsView& s, const NetDev& n, LearnedWork& w, float* S,
   k_edge_feats<<<nblk(s.nnzb), TPB, 0, st>>>(s.nnzb, s.valh, w.Ef);
   k_node_feats<<<nblk(V), TPB, 0, st>>>(s, w.Ef, w.X);
   // pre-activations (Q) are kept for the training backward only
-  gemm(V, w.X, FN, FN, nullptr, 0, 0, n.wt + WT_IN, H, wq + B_IN, nullptr, 0, nullptr, 0, w.training ? w.q0 : nullptr, w.h[0], 1, st);
+  gemm(V, w.X, FN, nullptr, FN, n.wt + WT_IN, H, wq + B_IN, nullptr, 0, nullptr, 0, w.training ? w.q0 : nullptr, w.h[0], 1, st);
   const int wgrid = nblk(32ll * V);
   for (int l = 0; l < NL; ++l) {
     const float* L = wq + LAYER0 + l * L_SIZE;
@@ -706,38 +802,45 @@ void learned_loss(const LsView& s, const NetDev& n, LearnedWork& w, float* S, co
                   float* Y, float* Wv, double* loss_parts, double* loss_out, float* grad, cudaStream_t st) {
   const int V = s.V;
   learned_forward(s, n, w, S, SPcg{}, st);
-  const int wgrid = nblk(32ll * V);
-  for (int p = 0; p < P; ++p) {
-    k_spmv<<<wgrid, TPB, 0, st>>>(V, s.rowptr, s.cols, S, nullptr, nullptr, nullptr, nullptr, probes + 3ll * V * p, Y + 3ll * V * p);
-    k_spmv<<<wgrid, TPB, 0, st>>>(V, s.rowptr, s.cols, s.valh, s.xbegin, s.xend, s.xcols, s.xvalh, Y + 3ll * V * p, Wv + 3ll * V * p);
-  }
+  const dim3 pgrid(nblk(32ll * V), P);
+  k_spmv<<<pgrid, TPB, 0, st>>>(V, s.rowptr, s.cols, S, nullptr, nullptr, nullptr, nullptr, probes, Y);
+  k_spmv<<<pgrid, TPB, 0, st>>>(V, s.rowptr, s.cols, s.valh, s.xbegin, s.xend, s.xcols, s.xvalh, Y, Wv);
   k_loss_terms<<<GRID, TPB, 0, st>>>(V, P, probes, Y, Wv, loss_parts);
   k_loss_final<<<1, 32, 0, st>>>(loss_parts, GRID, P, pnorm, loss_out);
   if (!grad || !w.training) return;
   const float* wq = n.wq;
-  k_coef_grad<<<nblk(V), TPB, 0, st>>>(s, P, probes, Wv, pnorm, w.zv, w.ab, w.dzv, w.dab);
-  k_dec_bwd<<<GRID, TPB, 0, st>>>(s, w.h[NL], w.Ef, wq, w.dzv, w.dab, w.dh, w.part);
-  reduce(w.part, 0, H + 1 + 2 * DE_IN + 2, grad + DV, st);
+  // the partials of every weight gradient in turn, summed by one launch at the end
+  Reductions R;
+  R.count = 0;
+  int blocks = 0;
+  float* next = w.part;
+  auto partials = [&](int n, int stride, int G, float* out) {
+    float* p = next;
+    next += (size_t(stride) * G + 3) / 4 * 4;
+    R.r[R.count++] = Reduction{p, out, n, stride, G, blocks};
+    blocks += nblk(n, 32);
+    return p;
+  };
+  const int wg = wgrad_grid(V);
+  constexpr int ND = H + 1 + 2 * DE_IN + 2, NW = H * 2 * H + H, NE = H * FE + H, NI = H * FN + H;
+  k_coef_grad<<<nblk(s.nnzb, 128), 128, 0, st>>>(s, P, probes, Wv, pnorm, w.zv, w.ab, w.dzv, w.dab);
+  k_dec_bwd<<<GRID, TPB, 0, st>>>(s, w.h[NL], w.Ef, wq, w.dzv, w.dab, w.dh, partials(ND, ND, GRID, grad + DV));
   float* dh = w.dh;
   float* dh_prev = w.dh2;
-  const long long VH = (long long)V * H;
   for (int l = NL - 1; l >= 0; --l) {
     const float* L = wq + LAYER0 + l * L_SIZE;
     float* G = grad + LAYER0 + l * L_SIZE;
-    k_relu_mask<<<nblk(VH), TPB, 0, st>>>(VH, dh, w.q[l], w.dq);
-    k_wgrad<<<GRID, TPB, 0, st>>>(V, w.dq, H, w.h[l], H, H, w.m[l], H, H, w.part);
-    reduce(w.part, 0, H * 2 * H + H, G + L_W, st);       // W then its bias (L_B follows L_W)
-    gemm(V, w.dq, H, H, nullptr, 0, 0, L + L_W, 2 * H, nullptr, nullptr, 0, nullptr, 0, nullptr, w.dhm, 0, st);
-    k_msg_bwd<<<GRID, TPB, 0, st>>>(s, w.u[l], w.Ef, L + L_E, L + L_C, w.dhm + H, 2 * H, w.du, w.part);
-    reduce(w.part, 0, H * FE + H, G + L_E, st);          // E then c (L_C follows L_E)
-    k_wgrad<<<GRID, TPB, 0, st>>>(V, w.du, H, w.h[l], H, H, nullptr, 0, 0, w.part);
-    reduce(w.part, 0, H * H, G + L_U, st);
-    gemm(V, w.du, H, H, nullptr, 0, 0, L + L_U, H, nullptr, dh, H, w.dhm, 2 * H, nullptr, dh_prev, 0, st);
+    // dq = dh where the pre-activation is positive: masked where it is read.
+    // W then its bias (L_B follows L_W), E then c (L_C follows L_E), U alone
+    k_wgrad<H, H><<<wg, TPB, 0, st>>>(V, dh, w.q[l], w.h[l], w.m[l], partials(NW, NW, wg, G + L_W));
+    gemm(V, dh, H, w.q[l], H, L + L_W, 2 * H, nullptr, nullptr, 0, nullptr, 0, nullptr, w.dhm, 0, st);
+    k_msg_bwd<<<GRID, TPB, 0, st>>>(s, w.u[l], w.Ef, L + L_E, L + L_C, w.dhm + H, 2 * H, w.du, partials(NE, NE, GRID, G + L_E));
+    k_wgrad<H, 0><<<wg, TPB, 0, st>>>(V, w.du, nullptr, w.h[l], nullptr, partials(H * H, H * H + H, wg, G + L_U));
+    gemm(V, w.du, H, nullptr, H, L + L_U, H, nullptr, dh, H, w.dhm, 2 * H, nullptr, dh_prev, 0, st);
     float* t = dh; dh = dh_prev; dh_prev = t;
   }
-  k_relu_mask<<<nblk(VH), TPB, 0, st>>>(VH, dh, w.q0, w.dq);
-  k_wgrad<<<GRID, TPB, 0, st>>>(V, w.dq, H, w.X, FN, FN, nullptr, 0, 0, w.part);
-  reduce(w.part, 0, H * FN + H, grad + W_IN, st);        // W_in then b_in
+  k_wgrad<FN, 0><<<wg, TPB, 0, st>>>(V, dh, w.q0, w.X, nullptr, partials(NI, NI, wg, grad + W_IN));   // W_in then b_in
+  k_reduce_all<<<blocks, TPB, 0, st>>>(R);
 }
 
 void launch_adam(float* master, float* m1, float* m2, const float* grad, int n, float lr, float b1, float b2, float eps, int t,

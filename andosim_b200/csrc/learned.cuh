@@ -65,7 +65,7 @@ struct LearnedWork {
   float *h[net::NL + 1], *u[net::NL], *m[net::NL], *q[net::NL], *q0;
   float *zv, *ab;                       // V, 2 nnzb
   // backward
-  float *dh, *dh2, *du, *dhm, *dq, *dzv, *dab;
+  float *dh, *dh2, *du, *dhm, *dzv, *dab;
   float* part;                          // per-CTA weight-gradient partials
 };
 
