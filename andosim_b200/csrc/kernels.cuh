@@ -118,9 +118,9 @@ struct PcgArgs {
   const int* xbegin; const int* xend; const int* xcols; const float* xval;  // extra contact segment
   const float* P;     // block-Jacobi inverse, 9V
   const float* b;
-  // z, p0 and p1: float4 rows (4V floats, 16-byte aligned) up to the largest
-  // system whose rows' state fits the registers, packed rows (3V) above it,
-  // where r and Ap (3V each) are used as well (pcg_packed_rows)
+  // z, p0 and p1: float4 rows (4V floats, 16-byte aligned) while the rows' state
+  // is in registers, packed rows (3V) above, where r and Ap (3V each) are used as
+  // well (pcg_packed_rows)
   float *x, *r, *z, *p0, *p1, *Ap;
   XrSlot* slots;      // XR_SLOTS
   Ctrl* ctrl;         // its arrival counter zeroed before the launch

@@ -27,18 +27,25 @@ namespace {
 
 // ---------------------------------------------------------- unscaled PCG
 // What bounds it: a small system by the two dependent reductions of an
-// iteration, a large one by reading the matrix from L2. So
-//  - each warp owns whole 32-row slices, one thread per row, and the row's
-//    r, z, p, A p and x stay in registers for the whole solve; only z and p
-//    are published, for the neighbours' products;
+// iteration, a large one by reading the matrix and its neighbours' vectors from
+// L2. So
+//  - each warp owns whole 32-row slices, one thread per row. A warp with one
+//    slice (ONE) keeps its rows' r, z, p, A p, P and x in registers for the
+//    whole solve; only z and p are published, for the neighbours' products. With
+//    more slices to a warp the rows' state stays in the caller's vectors (two
+//    or three rows' state per thread spilled: 26 us an iteration at 262,144
+//    rows against 20);
 //  - a warp copies a slice's blocks and columns, contiguous in the CSR arrays,
-//    into its own shared-memory buffer with 16-byte asynchronous copies. A
-//    warp with one slice (RPT = 1) copies it once per solve; a warp with two
-//    or three walks them up and down in turn, so that one of them is always
-//    still there. The row stride of 9 x 7 floats reads without bank conflicts;
+//    into its own shared-memory buffer with 16-byte asynchronous copies: once
+//    per solve if it has one slice; otherwise it walks its slices up and down in
+//    turn, so that one of them is always still there. The row stride of 9 x 7
+//    floats reads without bank conflicts;
 //  - the barrier of each dot product carries the sum (xr_reduce).
-// RPT = 0 keeps the rows' state in the caller's vectors, for any size.
 constexpr int PCG_WARPS = 24;                 // 24 x 9.4 KB of shared memory: a slice of 32 rows of 7 blocks each
+// With several slices to a warp the buffers leave room in the L1 for the
+// gathers, and the slices divide evenly: 262,144 rows on 19 warps with 9.1 KB
+// each 20.5 us an iteration, on 24 warps 28.4, on 12 26.9.
+constexpr int PCG_WARPS_MANY = 20, PCG_BUF_MANY = 9344;
 constexpr int PCG_TPB = 32 * PCG_WARPS;
 constexpr int PCG_CLUSTER_TPB = 512;
 constexpr int PCG_SMEM = 224 * 1024;          // all warps' buffers
@@ -111,14 +118,14 @@ __device__ inline int warp_copy_async(void* dst, const void* src, int n) {
   return off;
 }
 
-template <int RPT>
+template <bool ONE>
 __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
   Ctrl* ctrl = a.ctrl;
   if (ctrl->converged) return;
   extern __shared__ __align__(16) unsigned char pcg_dyn[];
   __shared__ XrSmem sh;
   __shared__ PcgScalars st;
-  constexpr int N = RPT > 0 ? RPT : 1, S = RPT > 0 ? 4 : 3, U = 4;
+  constexpr int S = ONE ? 4 : 3, U = 4;
   const int V = a.V, ns = (V + 31) >> 5, spc = (ns + (int)gridDim.x - 1) / (int)gridDim.x;
   const int w = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   const int s0 = blockIdx.x * spc, sn = max(0, min(spc, ns - s0));   // slices [s0, s0 + sn)
@@ -126,8 +133,8 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
   unsigned char* buf = pcg_dyn + (size_t)w * wbuf;
   float* bval = reinterpret_cast<float*>(buf);
   int* bcol = reinterpret_cast<int*>(buf + ((36 * cap + 16 + 15) & ~15));
-  float r[N][3], z[N][3], p[N][3], q[N][3], x[N][3], Pm[9];
-  int kb[N], cnt[N];
+  float r[3], z[3], p[3], q[3], x[3], Pm[9];   // ONE: the row's state
+  int kb = 0, cnt = 0;
   int held = -1, vo = 0, co = 0, hk0 = 0;   // slice in the buffer, element offsets of its first block and column, that block
   auto row_of = [&](int j) { return 32 * (s0 + j) + lane; };
   auto load_P = [&](int row, float (&m)[9]) {
@@ -138,24 +145,21 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
     o[1] = m[3] * v[0] + m[4] * v[1] + m[5] * v[2];
     o[2] = m[6] * v[0] + m[7] * v[1] + m[8] * v[2];
   };
-  // slice j's partials of the next reduction
-  auto hand_over = [&](int j, double v, float m0, float m1, float m2) {
+  // slice j's partials of the next reduction: the warp's, of all its slices in turn
+  auto hand_over = [&](double v, float m0, float m1, float m2) {
     v = xr_warp_sum(v);
     const unsigned m = __reduce_max_sync(0xffffffffu, max(xr_mag(m0), max(xr_mag(m1), xr_mag(m2))));
-    if (RPT > 0) { if (lane == 0) { sh.part[j] = v; sh.pmax[j] = m; } }
-    else if (lane == 0) { sh.part[w] += v; sh.pmax[w] = max(sh.pmax[w], m); }   // any number of slices: one partial per warp
+    if (lane == 0) { sh.part[w] += v; sh.pmax[w] = max(sh.pmax[w], m); }
   };
-  auto begin = [&]() { if (RPT == 0 && lane == 0) { sh.part[w] = 0.0; sh.pmax[w] = 0u; } __syncwarp(); };
-  const int nparts = RPT > 0 ? sn : nw;
-  auto reduce = [&](unsigned epoch, auto tail) { xr_reduce(sh, nparts, epoch, a.slots, &ctrl->bar_arrivals, &ctrl->bar_err, tail); };
+  auto begin = [&]() { if (lane == 0) { sh.part[w] = 0.0; sh.pmax[w] = 0u; } __syncwarp(); };
+  auto reduce = [&](unsigned epoch, auto tail) { xr_reduce(sh, nw, epoch, a.slots, &ctrl->bar_arrivals, &ctrl->bar_err, tail); };
 
   // init: x = 0, r = b, z = P r
   begin();
-  auto init = [&](int k, int j) {
+  for (int j = w; j < sn; j += nw) {
     const int row = row_of(j);
     double rz_loc = 0.0;
     float b[3] = {0.f, 0.f, 0.f}, zz[3];
-    kb[k] = 0; cnt[k] = 0;
     if (row < V) {
       for (int e = 0; e < 3; ++e) b[e] = a.b[3 * row + e];
       float m[9];
@@ -163,21 +167,15 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
       apply_P(m, b, zz);
       st4<S>(a.z, row, zz[0], zz[1], zz[2]);
       rz_loc = double(b[0]) * zz[0] + double(b[1]) * zz[1] + double(b[2]) * zz[2];
-      if (RPT == 1) for (int e = 0; e < 9; ++e) Pm[e] = m[e];
-      if (RPT > 0) {
-        kb[k] = a.rowptr[row]; cnt[k] = a.rowptr[row + 1] - kb[k];
-        for (int e = 0; e < 3; ++e) { r[k][e] = b[e]; z[k][e] = zz[e]; x[k][e] = 0.f; p[k][e] = 0.f; }
+      if (ONE) {
+        kb = a.rowptr[row]; cnt = a.rowptr[row + 1] - kb;
+        for (int e = 0; e < 9; ++e) Pm[e] = m[e];
+        for (int e = 0; e < 3; ++e) { r[e] = b[e]; z[e] = zz[e]; x[e] = 0.f; p[e] = 0.f; }
       } else {
         for (int e = 0; e < 3; ++e) { a.x[3 * row + e] = 0.f; a.r[3 * row + e] = b[e]; }
       }
     }
-    hand_over(j, rz_loc, b[0], b[1], b[2]);
-  };
-  if constexpr (RPT > 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) if (w + nw * k < sn) init(k, w + nw * k);
-  } else {
-    for (int j = w; j < sn; j += nw) init(0, j);
+    hand_over(rz_loc, b[0], b[1], b[2]);
   }
   reduce(1, [&](bool ok, double rz, unsigned mx) { st.start(ok, rz, mx, a.tol, false); });
   float beta = 0.f;
@@ -187,11 +185,14 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
   for (int it = 0; st.status == PCG_MAXIT && it < a.max_iters; ++it) {
     // ---- phase A: p_new = z + beta p_old, Ap = A p_new, p^T Ap
     begin();
-    auto product = [&](int k, int j) {
-      const int row = row_of(j);
-      int k0 = 0, n = 0;
-      if (RPT > 0) { k0 = kb[k]; n = cnt[k]; }
-      else if (row < V) { k0 = a.rowptr[row]; n = a.rowptr[row + 1] - k0; }
+    const int slices = w < sn ? (sn - 1 - w) / nw + 1 : 0;
+    for (int t = 0; t < slices; ++t) {
+      const int j = w + nw * ((it & 1) == 0 ? t : slices - 1 - t), row = row_of(j);   // up and down in turn
+      int k0 = kb, n = cnt;
+      if (!ONE) {
+        k0 = 0; n = 0;
+        if (row < V) { k0 = a.rowptr[row]; n = a.rowptr[row + 1] - k0; }
+      }
       if (held != j) {
         const int first_block = __shfl_sync(0xffffffffu, k0, 0);
         const int nb = __reduce_max_sync(0xffffffffu, n > 0 ? k0 + n - first_block : 0);
@@ -235,9 +236,8 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
       double pap_loc = 0.0;
       if (row < V) {
         float pv[3];
-        if (RPT > 0) {
-          for (int e = 0; e < 3; ++e) pv[e] = p[k][e] = first ? z[k][e] : z[k][e] + beta * p[k][e];
-          for (int e = 0; e < 3; ++e) q[k][e] = y[e];
+        if (ONE) {
+          for (int e = 0; e < 3; ++e) { pv[e] = p[e] = first ? z[e] : z[e] + beta * p[e]; q[e] = y[e]; }
         } else {
           const float4 zz = ld4<S>(a.z, row), pp = first ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4<S>(pold, row);
           pv[0] = first ? zz.x : zz.x + beta * pp.x; pv[1] = first ? zz.y : zz.y + beta * pp.y; pv[2] = first ? zz.z : zz.z + beta * pp.z;
@@ -246,55 +246,37 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
         st4<S>(pnew, row, pv[0], pv[1], pv[2]);
         pap_loc = double(pv[0]) * y[0] + double(pv[1]) * y[1] + double(pv[2]) * y[2];
       }
-      hand_over(j, pap_loc, 0.f, 0.f, 0.f);
-    };
-    const bool up = (it & 1) == 0;
-    if constexpr (RPT > 0) {
-      if (RPT == 1 || up) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) if (w + nw * k < sn) product(k, w + nw * k);
-      } else {
-#pragma unroll
-        for (int k = N - 1; k >= 0; --k) if (w + nw * k < sn) product(k, w + nw * k);
-      }
-    } else {
-      const int m = w < sn ? (sn - 1 - w) / nw + 1 : 0;
-      for (int t = 0; t < m; ++t) product(0, w + nw * (up ? t : m - 1 - t));
+      hand_over(pap_loc, 0.f, 0.f, 0.f);
     }
     reduce(2 + 2 * it, [&](bool ok, double pap, unsigned) { st.after_product(ok, pap); });
     if (st.status != PCG_MAXIT) break;
     const float alpha = st.coef;
     // ---- phase B: x, r, z, r^T z, |r|_inf
     begin();
-    auto update = [&](int k, int j) {
+    for (int j = w; j < sn; j += nw) {
       const int row = row_of(j);
       double rz_loc = 0.0;
-      float rv[3] = {0.f, 0.f, 0.f}, zv[3], m[9];
+      float rv[3] = {0.f, 0.f, 0.f}, zv[3];
       if (row < V) {
-        if (RPT != 1) load_P(row, m);
-        if (RPT > 0) {
-          for (int e = 0; e < 3; ++e) { x[k][e] += alpha * p[k][e]; r[k][e] -= alpha * q[k][e]; rv[e] = r[k][e]; }
+        if (ONE) {
+          for (int e = 0; e < 3; ++e) { x[e] += alpha * p[e]; rv[e] = r[e] -= alpha * q[e]; }
+          apply_P(Pm, rv, zv);
+          for (int e = 0; e < 3; ++e) z[e] = zv[e];
         } else {
+          float m[9];
+          load_P(row, m);
           const float4 pp = ld4<S>(pnew, row);
           const float pv[3] = {pp.x, pp.y, pp.z};
           for (int e = 0; e < 3; ++e) {
             a.x[3 * row + e] += alpha * pv[e];
-            rv[e] = a.r[3 * row + e] - alpha * a.Ap[3 * row + e];
-            a.r[3 * row + e] = rv[e];
+            rv[e] = a.r[3 * row + e] -= alpha * a.Ap[3 * row + e];
           }
+          apply_P(m, rv, zv);
         }
-        if (RPT == 1) apply_P(Pm, rv, zv); else apply_P(m, rv, zv);
-        if (RPT > 0) for (int e = 0; e < 3; ++e) z[k][e] = zv[e];
         st4<S>(a.z, row, zv[0], zv[1], zv[2]);
         rz_loc = double(rv[0]) * zv[0] + double(rv[1]) * zv[1] + double(rv[2]) * zv[2];
       }
-      hand_over(j, rz_loc, rv[0], rv[1], rv[2]);
-    };
-    if constexpr (RPT > 0) {
-#pragma unroll
-      for (int k = 0; k < N; ++k) if (w + nw * k < sn) update(k, w + nw * k);
-    } else {
-      for (int j = w; j < sn; j += nw) update(0, j);
+      hand_over(rz_loc, rv[0], rv[1], rv[2]);
     }
     reduce(3 + 2 * it, [&](bool ok, double rz, unsigned mx) { st.after_update(ok, rz, mx, a.tol, 0); });
     if (st.status != PCG_MAXIT) break;
@@ -302,12 +284,9 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
     first = false;
     float* t = pold; pold = pnew; pnew = t;
   }
-  if constexpr (RPT > 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-      const int row = row_of(w + nw * k);
-      if (w + nw * k < sn && row < V) for (int e = 0; e < 3; ++e) a.x[3 * row + e] = x[k][e];
-    }
+  if (ONE) {
+    const int row = row_of(w);
+    if (w < sn && row < V) for (int e = 0; e < 3; ++e) a.x[3 * row + e] = x[e];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) st.report(ctrl);
 }
@@ -1092,7 +1071,7 @@ size_t pcg_scaled_partials(int V) { return 3ull * (size_t)((V + 31) / 32 + 1); }
 
 namespace {
 using PcgKernel = void (*)(PcgArgs);
-PcgKernel pcg_kernel(int rpt) { return rpt == 1 ? k_pcg<1> : rpt == 2 ? k_pcg<2> : rpt == 3 ? k_pcg<3> : k_pcg<0>; }
+PcgKernel pcg_kernel(bool one) { return one ? k_pcg<true> : k_pcg<false>; }
 
 // Resident kernel of a shape: threads per CTA rounded up to a compiled bound,
 // and with it the registers, which decide how many neighbours' p are kept
@@ -1292,9 +1271,12 @@ cudaError_t launch_pcg_scaled(const PcgScaledArgs& args, bool learned, const Pcg
 
 bool pcg_packed_rows(int V) {
   const int ns = (V + 31) / 32, ctas = std::min(pcg_device().sms, XR_MAX_CTAS);
-  return (ns + ctas - 1) / ctas > 3 * PCG_WARPS;
+  return (ns + ctas - 1) / ctas > PCG_WARPS;
 }
 
+// Form of a solve, by its rows alone: one cluster up to 8,192 (3.8 us an
+// iteration there, 6.5 over every SM at 8,281), then one CTA on each SM with a
+// slice to each of its warps, from 113,665 rows on with several.
 cudaError_t launch_pcg(const PcgArgs& args, cudaStream_t s) {
   const PcgDevice D = pcg_device();
   PcgArgs a = args;
@@ -1309,10 +1291,11 @@ cudaError_t launch_pcg(const PcgArgs& args, cudaStream_t s) {
   }
   const int ctas = std::min(D.sms, XR_MAX_CTAS);
   const int spc = (ns + ctas - 1) / ctas, grid = (ns + spc - 1) / spc;
-  const int nw = std::min(spc, PCG_WARPS), rpt = (spc + nw - 1) / nw;
-  a.smem = nw * std::min(PCG_SMEM / nw, 24 * 1024);
+  const bool one = spc <= PCG_WARPS;   // as pcg_packed_rows
+  const int each = one ? 1 : (spc + PCG_WARPS_MANY - 1) / PCG_WARPS_MANY, nw = (spc + each - 1) / each;
+  a.smem = nw * std::min(PCG_SMEM / nw, one ? 24 * 1024 : PCG_BUF_MANY);
   void* p[] = {(void*)&a};
-  return launch_ctas((const void*)pcg_kernel(rpt <= 3 ? rpt : 0), false, grid, 32 * nw, a.smem, PCG_SMEM, p, s);
+  return launch_ctas((const void*)pcg_kernel(one), false, grid, 32 * nw, a.smem, PCG_SMEM, p, s);
 }
 
 }  // namespace ando

@@ -1,7 +1,7 @@
 """The PCG kernels at the sizes where their form changes.
 
 The unscaled PCG (``ando_pcg_solve_noalloc``) is one cluster up to 8,192 rows, then one CTA per SM
-with one to three 32-row slices to a warp, then a form that keeps its rows' state in memory. The
+with a 32-row slice to each warp, from 113,665 rows on with several. The
 scaled PCG of the CORRECTED step is one cluster (8,192 rows, 1,024 with contact blocks or wide
 rows), CTAs of 512 threads, of up to 1,024 on every SM, and a looping form above 151,552 rows.
 
@@ -63,7 +63,7 @@ def grid_csr(nx, ny, seed, hub=0):
 @pytest.mark.parametrize("nx,ny,hub,shift", [
     (1, 1, 0, 0), (33, 1, 0, 1), (31, 33, 0, 0), (40, 30, 900, 3), (128, 64, 0, 0),      # cluster
     (8193, 1, 0, 2), (300, 250, 3000, 0),                                                 # one slice to a warp
-    (400, 300, 0, 1), (500, 460, 0, 0), (600, 575, 0, 0),                                 # two, three, any number
+    (400, 300, 0, 1), (500, 460, 0, 0), (600, 575, 0, 0),                                 # several
 ])
 def test_unscaled_pcg(abi, nx, ny, hub, shift):
     """`shift`: the arrays start that many elements past a 16-byte boundary."""
