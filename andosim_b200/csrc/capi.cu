@@ -68,6 +68,7 @@ struct ando_ctx_s {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev_count = nullptr;  // a count has reached the host
   int V = 0, T = 0, nnzb = 0;
   double mu = 0, thickness = 0, density = 0;
   int el_semantics = -1;
@@ -130,18 +131,19 @@ struct ando_ctx_s {
   DevBuf<unsigned char> contact_out;   // contacts as public records, for ando_compute_contacts*
   int ncontacts = 0, n_pe = 0;
   int* ctrl_host_count = nullptr;  // pinned int for small device -> host counts
-  DevBuf<int> ekeys, ekeys_sorted, ebegin, eend, xflags, xkeys, xcols, xbegin, xend, nsel;
+  DevBuf<int> ekeys, ekeys_sorted, ebegin, eend, xcount, xoff, xcols, xbegin, xend, nsel;
   // merged extra blocks: 64-bit row:col keys, entry indices, run heads, block rows
   DevBuf<unsigned long long> xk0, xk1;
   DevBuf<int> xi0, xi1, xheads, xrow;
   int nx_raw = 0;
-  DevBuf<ContactEntry> ents, ents_sorted, xent;
+  DevBuf<ContactRec> crec;
+  DevBuf<int> ents, ents_sorted;
   DevBuf<float> xval;
   // SELL-32 copy of the scaled contact blocks (resident PCG)
   DevBuf<int> xs_width, xs_off, xs_col;
   DevBuf<float> xs_val;
   bool xs_ready = false;
-  int nx = 0, nent = 0;
+  int nx = 0;
   DevBuf<unsigned char> cub_tmp;
 
   // constraints
@@ -226,6 +228,7 @@ struct ando_ctx_s {
     if (counts_host) cudaFreeHost(counts_host);
     if (stage_host) cudaFreeHost(stage_host);
     if (ev0) cudaEventDestroy(ev0);
+    if (ev_count) cudaEventDestroy(ev_count);
     if (ev1) cudaEventDestroy(ev1);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -443,6 +446,37 @@ int detect(ando_ctx c, int nb, int phase = ANDO_PHASE_SETUP, double thresh = 0.0
   return ANDO_OK;
 }
 
+// Whether the sorted keys start a new run at k.
+template <class K>
+struct RunHead {
+  const K* key;
+  __device__ bool operator()(int k) const { return k == 0 || key[k] != key[k - 1]; }
+};
+
+// The off-diagonal entries of the contacts, sorted by (row, col), the first entry
+// of each block (xheads), and the blocks' rows and columns; *nu = blocks.
+template <class K>
+int extra_blocks(ando_ctx c, int nc, int nraw, int kb, int* nu) {
+  cudaStream_t s = c->stream;
+  K* k0 = reinterpret_cast<K*>(c->xk0.p);
+  K* k1 = reinterpret_cast<K*>(c->xk1.p);
+  launch_extra_entries(c->crec.p, c->xoff.p, nc, kb, k0, c->xi0.p, s);
+  size_t bytes = 0, sel_bytes = 0;
+  thrust::counting_iterator<int> iota(0);
+  const RunHead<K> head{k1};
+  CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, k0, k1, c->xi0.p, c->xi1.p, nraw, 0, 2 * kb, s));
+  CK(cub::DeviceSelect::If(nullptr, sel_bytes, iota, c->xheads.p, c->nsel.p, nraw, head, s));
+  CK(c->cub_reserve(std::max(bytes, sel_bytes)));
+  CK(cub::DeviceRadixSort::SortPairs(c->cub_tmp.p, bytes, k0, k1, c->xi0.p, c->xi1.p, nraw, 0, 2 * kb, s));
+  CK(cub::DeviceSelect::If(c->cub_tmp.p, sel_bytes, iota, c->xheads.p, c->nsel.p, nraw, head, s));
+  CK(cudaMemcpyAsync(c->ctrl_host_count, c->nsel.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  *nu = *c->ctrl_host_count;
+  CK(c->xrow.reserve(*nu)); CK(c->xcols.reserve(*nu));
+  launch_extra_rows(k1, c->xheads.p, *nu, kb, c->xrow.p, c->xcols.p, s);
+  return ANDO_OK;
+}
+
 // Per-step contact constants: k_bar and barrier derivatives at the frozen
 // gap, the per-vertex constant gradient/diagonal, and the extra off-diagonal
 // block segment sorted by row.
@@ -451,70 +485,53 @@ int prepare_contacts(ando_ctx c, const StepParams& sp, const double* g_base, con
   MeshDev m = c->mesh_dev();
   int nc = c->ncontacts, V = c->V;
   c->xs_ready = false;
-  if (nc) { launch_contact_prep(m, c->contacts.p, nc, sp, c->stream); ph.launched(); }
-  int ne = 16 * nc;
-  c->nent = ne;
-  CK(c->ekeys.reserve(ne + 1)); CK(c->ekeys_sorted.reserve(ne + 1));
-  CK(c->ents.reserve(ne + 1)); CK(c->ents_sorted.reserve(ne + 1));
   CK(c->ebegin.reserve(V)); CK(c->eend.reserve(V));
-  CK(c->xflags.reserve(ne + 1)); CK(c->xkeys.reserve(ne + 1)); CK(c->xent.reserve(ne + 1));
   CK(c->xbegin.reserve(V)); CK(c->xend.reserve(V)); CK(c->xrow.reserve(1)); CK(c->xcols.reserve(1)); CK(c->xval.reserve(9));
   CK(c->nsel.reserve(1));
-  if (ne == 0) {
+  if (nc == 0) {
     CK(cudaMemsetAsync(c->ebegin.p, 0, sizeof(int) * V, c->stream));
     CK(cudaMemsetAsync(c->eend.p, 0, sizeof(int) * V, c->stream));
     c->nx = 0; c->nx_raw = 0;
-    launch_contact_vertex(m, c->contacts.p, c->ents_sorted.p, c->ebegin.p, c->eend.p, sp, g_base, c->g_const.p, c->diag_const.p, c->stream);
+    launch_contact_vertex(V, c->crec.p, c->ents_sorted.p, c->ebegin.p, c->eend.p, sp, g_base, c->g_const.p, c->diag_const.p, c->stream);
     ph.launched();
     CK(cudaGetLastError());
     return ANDO_OK;
   }
-  launch_contact_entries(c->contacts.p, nc, V, sp.semantics == 0 && sp.enable_friction && sp.friction_mu > 0.0, c->ekeys.p, c->ents.p, c->stream);
-  ph.launched();
+  const int ne = 4 * nc;
+  CK(c->ekeys.reserve(ne)); CK(c->ekeys_sorted.reserve(ne)); CK(c->ents.reserve(ne)); CK(c->ents_sorted.reserve(ne));
+  CK(c->crec.reserve(nc)); CK(c->xcount.reserve(nc + 1ull)); CK(c->xoff.reserve(nc + 1ull));
+  launch_contact_prep(m, c->contacts.p, nc, sp, sp.semantics == 0 && sp.enable_friction && sp.friction_mu > 0.0, c->crec.p, c->ekeys.p, c->ents.p,
+                      c->xcount.p, c->stream);
+  // entries by vertex (V: nothing to add), in contact order
   int bits = 1;
   while ((1ll << bits) <= (long long)V) ++bits;
-  size_t bytes = 0;
+  size_t bytes = 0, scan_bytes = 0;
   CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, c->ekeys.p, c->ekeys_sorted.p, c->ents.p, c->ents_sorted.p, ne, 0, bits, c->stream));
-  CK(c->cub_reserve(bytes));
+  CK(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, c->xcount.p, c->xoff.p, nc + 1, c->stream));
+  CK(c->cub_reserve(std::max(bytes, scan_bytes)));
+  CK(cub::DeviceScan::ExclusiveSum(c->cub_tmp.p, scan_bytes, c->xcount.p, c->xoff.p, nc + 1, c->stream));
+  CK(cudaMemcpyAsync(c->ctrl_host_count, c->xoff.p + nc, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaEventRecord(c->ev_count, c->stream));
   CK(cub::DeviceRadixSort::SortPairs(c->cub_tmp.p, bytes, c->ekeys.p, c->ekeys_sorted.p, c->ents.p, c->ents_sorted.p, ne, 0, bits, c->stream));
   launch_vertex_ranges(c->ekeys_sorted.p, ne, V, c->ebegin.p, c->eend.p, c->stream);
-  launch_contact_vertex(m, c->contacts.p, c->ents_sorted.p, c->ebegin.p, c->eend.p, sp, g_base, c->g_const.p, c->diag_const.p, c->stream);
-  // extra segment: off-diagonal barrier blocks, kept in row order
-  launch_extra_flags(c->ents_sorted.p, c->ekeys_sorted.p, ne, c->xflags.p, c->stream);
+  launch_contact_vertex(V, c->crec.p, c->ents_sorted.p, c->ebegin.p, c->eend.p, sp, g_base, c->g_const.p, c->diag_const.p, c->stream);
   ph.launched(3);
-  bytes = 0;
-  CK(cub::DeviceSelect::Flagged(nullptr, bytes, c->ents_sorted.p, c->xflags.p, c->xent.p, c->nsel.p, ne, c->stream));
-  CK(c->cub_reserve(bytes));
-  CK(cub::DeviceSelect::Flagged(c->cub_tmp.p, bytes, c->ents_sorted.p, c->xflags.p, c->xent.p, c->nsel.p, ne, c->stream));
-  CK(cub::DeviceSelect::Flagged(c->cub_tmp.p, bytes, c->ekeys_sorted.p, c->xflags.p, c->xkeys.p, c->nsel.p, ne, c->stream));
-  CK(cudaMemcpyAsync(c->ctrl_host_count, c->nsel.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  int nraw = *c->ctrl_host_count, nu = 0;
+  // off-diagonal barrier blocks, merged by (row, col) and kept in row order; the
+  // device sorts the vertex entries while the host waits for their number
+  CK(cudaEventSynchronize(c->ev_count));
+  const int nraw = *c->ctrl_host_count;
+  int nu = 0;
   c->nx_raw = nraw;
   if (nraw) {
-    // merge the entries of each (row, col) into one block: sort by row:col
-    // (stable, so entries stay in contact order inside a block), then one
-    // thread per run of equal keys
     CK(c->xk0.reserve(nraw)); CK(c->xk1.reserve(nraw)); CK(c->xi0.reserve(nraw)); CK(c->xi1.reserve(nraw)); CK(c->xheads.reserve(nraw));
-    launch_extra_key64(c->xent.p, c->xkeys.p, nraw, c->xk0.p, c->xi0.p, c->stream);
-    bytes = 0;
-    CK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, c->xk0.p, c->xk1.p, c->xi0.p, c->xi1.p, nraw, 0, 32 + bits, c->stream));
-    CK(c->cub_reserve(bytes));
-    CK(cub::DeviceRadixSort::SortPairs(c->cub_tmp.p, bytes, c->xk0.p, c->xk1.p, c->xi0.p, c->xi1.p, nraw, 0, 32 + bits, c->stream));
-    launch_run_heads(c->xk1.p, nraw, c->xflags.p, c->stream);
-    bytes = 0;
-    thrust::counting_iterator<int> iota(0);
-    CK(cub::DeviceSelect::Flagged(nullptr, bytes, iota, c->xflags.p, c->xheads.p, c->nsel.p, nraw, c->stream));
-    CK(c->cub_reserve(bytes));
-    CK(cub::DeviceSelect::Flagged(c->cub_tmp.p, bytes, iota, c->xflags.p, c->xheads.p, c->nsel.p, nraw, c->stream));
-    CK(cudaMemcpyAsync(c->ctrl_host_count, c->nsel.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    nu = *c->ctrl_host_count;
-    CK(c->xrow.reserve(nu)); CK(c->xcols.reserve(nu)); CK(c->xval.reserve(9ull * nu));
-    if (sp.semantics == ANDO_SEMANTICS_CORRECTED) CK(c->xvalh.reserve(9ull * nu));
-    launch_extra_merge(c->contacts.p, c->xent.p, c->xk1.p, c->xi1.p, c->xheads.p, nu, nraw, fixed, sp, nullptr, c->xrow.p, c->xcols.p,
-                       c->xval.p, nullptr, c->stream);
-    ph.launched(4);
+    int kb = 1;
+    while ((1ll << kb) < (long long)V) ++kb;
+    int rc = 2 * kb <= 32 ? extra_blocks<unsigned>(c, nc, nraw, kb, &nu) : extra_blocks<unsigned long long>(c, nc, nraw, kb, &nu);
+    if (rc) return rc;
+    CK(c->xval.reserve(9ull * nu));
+    if (sp.semantics == ANDO_SEMANTICS_CORRECTED) CK(c->xvalh.reserve(9ull * nu));   // both values come with the scaled assembly
+    else launch_extra_merge(c->crec.p, c->xi1.p, c->xheads.p, c->xrow.p, c->xcols.p, nu, nraw, fixed, sp, nullptr, c->xval.p, nullptr, c->stream);
+    ph.launched(3);
   }
   c->nx = nu;
   launch_vertex_ranges(c->xrow.p, nu, V, c->xbegin.p, c->xend.p, c->stream);
@@ -855,8 +872,7 @@ int enqueue_scaled_assembly(ando_ctx c, const StepParams& sp, cudaStream_t s) {
     CK(cudaMemsetAsync(c->xs_col.p, 0xff, sizeof(int) * size_t(places), s));
     xs.off = c->xs_off.p; xs.begin = c->xbegin.p; xs.col = c->xs_col.p; xs.val = c->xs_val.p;
   }
-  launch_extra_merge(c->contacts.p, c->xent.p, c->xk1.p, c->xi1.p, c->xheads.p, c->nx, c->nx_raw, c->fixed.p, sp, c->Linv.p,
-                     nullptr, nullptr, nullptr, c->xvalh.p, s, xs);
+  launch_extra_merge(c->crec.p, c->xi1.p, c->xheads.p, c->xrow.p, c->xcols.p, c->nx, c->nx_raw, c->fixed.p, sp, c->Linv.p, c->xval.p, c->xvalh.p, s, xs);
   return ANDO_OK;
 }
 
@@ -1022,7 +1038,12 @@ int inner_newton_corrected(ando_ctx c, const ando_params& p, const StepParams& s
     c->solve_first = false;
     st.strain_active = c->ctrl_host->strain_active;
     st.contacts = std::max(st.contacts, c->ncontacts);
-    if (c->ctrl_host->converged) { ret = 1.0; return ANDO_OK; }
+    if (c->ctrl_host->converged) {   // no assembly follows: the blocks' unscaled values alone (ando_last_contact_blocks)
+      launch_extra_merge(c->crec.p, c->xi1.p, c->xheads.p, c->xrow.p, c->xcols.p, c->nx, c->nx_raw, c->fixed.p, sp, nullptr, c->xval.p, nullptr, s);
+      CK(cudaGetLastError());
+      ret = 1.0;
+      return ANDO_OK;
+    }
     {
       Phase ph(c, ANDO_PHASE_ASSEMBLE);
       c->write_val = c->keep_system;                       // unscaled copy only for ando_last_system
@@ -1167,7 +1188,7 @@ int capture_frame(ando_ctx c, const ando_params& p, const StepParams& sp, bool l
   launch_predict(c->V, c->x.p, c->v.p, p.dt, c->x_old.p, c->x_hat.p, s);
   CAP(cudaMemsetAsync(c->ebegin.p, 0, sizeof(int) * c->V, s), "memset");
   CAP(cudaMemsetAsync(c->eend.p, 0, sizeof(int) * c->V, s), "memset");
-  launch_contact_vertex(m, c->contacts.p, c->ents_sorted.p, c->ebegin.p, c->eend.p, sp, c->g_el.p, c->g_const.p, c->diag_const.p, s);
+  launch_contact_vertex(c->V, c->crec.p, c->ents_sorted.p, c->ebegin.p, c->eend.p, sp, c->g_el.p, c->g_const.p, c->diag_const.p, s);
   cudaStreamCaptureStatus cs;
   cudaGraph_t g = nullptr;
   const cudaGraphNode_t* deps = nullptr;
@@ -1389,6 +1410,7 @@ int32_t ando_ctx_create(int32_t device, ando_ctx* out) {
   c->device = device;
   cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_count, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
   if (e == cudaSuccess) e = cudaMallocHost(&c->ctrl_host, sizeof(Ctrl));
   if (e == cudaSuccess) e = cudaMallocHost(&c->sctl_host, sizeof(StepCtl));

@@ -79,8 +79,22 @@ struct ContactDev {
 // The fields up to the weights, as the public ando_contact holds them.
 constexpr int CONTACT_OUT_BYTES = 168;
 
-// Contact contribution entry (contact c, local i, local j), sorted by row vertex.
-struct ContactEntry { int contact, li, lj, col; };
+// What the block sums read of a contact: 96 bytes (three sectors; the merged
+// off-diagonal blocks read the first two) in place of ContactDev's 224, so a
+// contact met from its four vertices and twelve blocks costs a third.
+struct alignas(32) ContactRec {
+  double nn[3], w[4], d2V;
+  int idx[4];
+  double dV;
+  unsigned mask;   // bit i: vertex i carries a weight; REC_HESS, REC_GRAD: a Hessian / gradient to add
+  unsigned pad;
+};
+static_assert(sizeof(ContactRec) == 96 && offsetof(ContactRec, idx) % 16 == 0, "records are read in 16-byte pieces");
+constexpr unsigned REC_HESS = 16u, REC_GRAD = 32u;
+
+// Contact entries, sorted by vertex and in contact order within one: 4 * contact
+// + local vertex, with ENTRY_FRICTION where the vertex takes the contact's friction.
+constexpr int ENTRY_FRICTION = 1 << 30;
 
 // --------------------------------------------------------- mesh on device
 struct MeshDev {

@@ -321,9 +321,12 @@ __device__ inline double contact_kbar(const MeshDev& m, const ContactDev& C, dou
 
 // Per-contact constants of a step: k_bar, the normalised frozen normal and the
 // barrier derivatives at the frozen gap (barrier.cpp:67-149 reads contact.gap
-// and contact.normal from detection time).
-__global__ void k_contact_prep(MeshDev m, ContactDev* cs, int nc, StepParams p) {
+// and contact.normal from detection time). Also the contact's record for the
+// block sums, its four vertex entries (key = vertex, or V where the contact adds
+// nothing there) and the number of its off-diagonal blocks.
+__global__ void k_contact_prep(MeshDev m, ContactDev* cs, int nc, StepParams p, int friction, ContactRec* recs, int* keys, int* ents, int* xcount) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c == nc) xcount[c] = 0;   // closes the scan
   if (c >= nc) return;
   ContactDev& C = cs[c];
   // CORRECTED: the inertial part of the stiffness is sum(m w^2) / g^2 at the
@@ -337,31 +340,28 @@ __global__ void k_contact_prep(MeshDev m, ContactDev* cs, int nc, StepParams p) 
   C.in_dom = barrier_type && in_domain(C.gap, p.contact_gap_max);
   C.dV = C.in_dom ? bar_grad(C.gap, p.contact_gap_max, C.kbar) : 0.0;
   C.d2V = C.in_dom ? bar_hess(C.gap, p.contact_gap_max, C.kbar) : 0.0;
-}
-
-// Entry slots: 16 per contact, (c, i, j) at c*16 + i*4 + j. Valid barrier
-// entries and (c,0,0) friction entries get key = row vertex, others key = V.
-// Entry kinds (ContactEntry.col < 0 encodes "friction only").
-__global__ void k_contact_entries(const ContactDev* cs, int nc, int V, int friction, int* keys, ContactEntry* ents) {
-  long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (long long)nc * 16) return;
-  int c = int(e / 16), i = int((e % 16) / 4), j = int(e % 4);
-  const ContactDev& C = cs[c];
-  int cnt = C.count > 1 ? C.count : 1;
-  bool barrier = C.in_dom && C.d2V != 0.0 && i < cnt && j < cnt && C.w[i] != 0.0 && C.w[j] != 0.0 &&
-                 C.idx[i] >= 0 && C.idx[j] >= 0 && C.idx[i] < V && C.idx[j] < V;
-  // a barrier gradient entry is represented by the (i,i) entry even when d2V == 0 but dV != 0
-  bool grad_only = !barrier && i == j && C.in_dom && C.dV != 0.0 && i < cnt && C.w[i] != 0.0 && C.idx[i] >= 0 && C.idx[i] < V;
-  bool fric = friction && C.type >= 0 && i == 0 && j == 0 && C.idx[0] >= 0 && C.idx[0] < V;
-  ContactEntry E; E.contact = c; E.li = i; E.lj = j;
-  if (barrier || grad_only || fric) {
-    keys[e] = C.idx[i];
-    E.col = (barrier || grad_only) ? C.idx[j] : -1;
-    E.li = i | (fric ? 8 : 0) | (grad_only ? 16 : 0);
-  } else {
-    keys[e] = V; E.col = -1;
+  ContactRec R;
+  R.nn[0] = nn.x; R.nn[1] = nn.y; R.nn[2] = nn.z;
+  R.d2V = C.d2V; R.dV = C.dV; R.pad = 0;
+  R.mask = (C.in_dom && C.d2V != 0.0 ? REC_HESS : 0u) | (C.in_dom && C.dV != 0.0 ? REC_GRAD : 0u);
+  const int cnt = C.count > 1 ? C.count : 1;
+  for (int i = 0; i < 4; ++i) {
+    R.w[i] = C.w[i]; R.idx[i] = C.idx[i];
+    if (i < cnt && R.w[i] != 0.0 && R.idx[i] >= 0 && R.idx[i] < m.V) R.mask |= 1u << i;
   }
-  ents[e] = E;
+  recs[c] = R;
+  const bool fric = friction && C.type >= 0 && R.idx[0] >= 0 && R.idx[0] < m.V;
+  int4 key, ent;
+  int* kp = &key.x;
+  for (int i = 0; i < 4; ++i) kp[i] = ((R.mask >> i & 1u) && (R.mask & (REC_HESS | REC_GRAD))) || (i == 0 && fric) ? R.idx[i] : m.V;
+  ent.x = 4 * c | (fric ? ENTRY_FRICTION : 0); ent.y = 4 * c + 1; ent.z = 4 * c + 2; ent.w = 4 * c + 3;
+  reinterpret_cast<int4*>(keys)[c] = key;
+  reinterpret_cast<int4*>(ents)[c] = ent;
+  int n = 0;
+  if (R.mask & REC_HESS)
+    for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 4; ++j) n += (R.mask >> i & R.mask >> j & 1u) && R.idx[i] != R.idx[j];
+  xcount[c] = n;
 }
 
 __global__ void k_vertex_ranges(const int* keys, int n, int V, int* begin, int* end) {
@@ -376,39 +376,54 @@ __global__ void k_vertex_ranges(const int* keys, int n, int V, int* begin, int* 
 
 // Per-vertex constants of a step: elastic gradient (REFERENCE: on the rest
 // mesh, so constant) + contact barrier gradient, and the contact Hessian
-// blocks that land on the diagonal. Contact terms are summed in contact order.
-__global__ void k_contact_vertex(MeshDev m, const ContactDev* cs, const ContactEntry* ents, const int* begin, const int* end,
-                                 StepParams p, const double* g_base, double* g_const, double* diag_const) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= m.V) return;
-  d3 g = ld3(g_base, v);
-  double H[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int k = begin[v]; k < end[v]; ++k) {
-    ContactEntry E = ents[k];
-    if (E.col < 0) continue;  // friction only
-    const ContactDev& C = cs[E.contact];
-    int i = E.li & 3, j = E.lj;
-    d3 n = mk(C.nn[0], C.nn[1], C.nn[2]);
-    if (i == j && C.dV != 0.0 && C.w[i] != 0.0) g = g + n * (C.dV * C.w[i]);
-    if (E.col == v && !(E.li & 16)) {
-      d3 gi = n * C.w[i], gj = n * C.w[j];
-      for (int r = 0; r < 3; ++r)
-        for (int q = 0; q < 3; ++q) {
-          double val = C.d2V * (comp(gi, r) * comp(gj, q));
-          if (fabs(val) < p.barrier_tol) continue;
-          H[r * 3 + q] += val;
-        }
+// blocks that land on the diagonal. Contact terms are summed in contact order:
+// 16 lanes take a vertex, one component each (12 of them), and walk its entries
+// four at a time, so that the records' latency, which bounds a walk of one entry
+// after the other, is met once for four.
+constexpr int CV_LANES = 16, CV_AHEAD = 4;
+__global__ void __launch_bounds__(256) k_contact_vertex(int V, const ContactRec* __restrict__ recs, const int* __restrict__ ents,
+                                                        const int* __restrict__ begin, const int* __restrict__ end, StepParams p,
+                                                        const double* g_base, double* g_const, double* diag_const) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, v = t / CV_LANES, q = t % CV_LANES;
+  if (v >= V || q >= 12) return;
+  const bool grad = q >= 9;
+  const int r = grad ? q - 9 : q / 3, s = grad ? 0 : q % 3;
+  double sum = grad ? g_base[3ll * v + r] : 0.0;
+  const int e = end[v];
+  for (int k = begin[v]; k < e; k += CV_AHEAD) {
+    unsigned id[CV_AHEAD], mask[CV_AHEAD];
+    double n_r[CV_AHEAD], n_s[CV_AHEAD], w[CV_AHEAD], d[CV_AHEAD];
+    int4 idx[CV_AHEAD];
+#pragma unroll
+    for (int u = 0; u < CV_AHEAD; ++u) id[u] = ents[min(k + u, e - 1)] & ~ENTRY_FRICTION;
+#pragma unroll
+    for (int u = 0; u < CV_AHEAD; ++u) {
+      const ContactRec& R = recs[id[u] >> 2];
+      n_r[u] = R.nn[r]; n_s[u] = R.nn[s]; w[u] = R.w[id[u] & 3]; d[u] = grad ? R.dV : R.d2V;
+      mask[u] = k + u < e ? R.mask : 0u;
+      idx[u] = *reinterpret_cast<const int4*>(R.idx);
+    }
+#pragma unroll
+    for (int u = 0; u < CV_AHEAD; ++u) {
+      const int i = id[u] & 3;
+      if (!(mask[u] >> i & 1u)) continue;   // friction only
+      if (grad) {
+        if (mask[u] & REC_GRAD) sum = sum + n_r[u] * (d[u] * w[u]);
+        continue;
+      }
+      if (!(mask[u] & REC_HESS)) continue;
+      const double gi = n_r[u] * w[u];
+      for (int j = 0; j < 4; ++j) {
+        if (!(mask[u] >> j & 1u) || (j == 0 ? idx[u].x : j == 1 ? idx[u].y : j == 2 ? idx[u].z : idx[u].w) != v) continue;
+        const double gj = n_s[u] * (j == i ? w[u] : recs[id[u] >> 2].w[j]);
+        const double val = d[u] * (gi * gj);
+        if (fabs(val) < p.barrier_tol) continue;
+        sum += val;
+      }
     }
   }
-  st3(g_const, v, g);
-  for (int k = 0; k < 9; ++k) diag_const[9 * v + k] = H[k];
-}
-
-__global__ void k_extra_flags(const ContactEntry* ents, const int* keys, int n, int* flags) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  ContactEntry E = ents[k];
-  flags[k] = (E.col >= 0 && E.col != keys[k] && !(E.li & 16)) ? 1 : 0;
+  if (grad) g_const[3ll * v + r] = sum;
+  else diag_const[9ll * v + q] = sum;
 }
 
 // ---------------------------------------------------------- Newton iteration
@@ -595,7 +610,7 @@ __global__ void k_strain_face(MeshDev m, const double* x, StepParams p, unsigned
 __global__ void __launch_bounds__(256, 3) k_gradient(MeshDev m, const double* x, const double* x_hat, const double* x_prev, const double* g_const,
                            const double* diag_const, const unsigned char* sflags, const StrainSV* sv,
                            const int* pin_vertex, const int* pin_head, const double* pin_target, int num_pins, const WallDev* walls,
-                           const ContactDev* contacts, const ContactEntry* ents, const int* ebegin, const int* eend,
+                           const ContactDev* contacts, const int* ents, const int* ebegin, const int* eend,
                            StepParams p, const unsigned char* fixed, double* g, float* b, double* diag_extra, Ctrl* ctrl) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double local = 0.0;
@@ -689,9 +704,9 @@ __global__ void __launch_bounds__(256, 3) k_gradient(MeshDev m, const double* x,
     if (p.enable_friction && p.friction_mu > 0.0) {
       d3 disp = xi - ld3(x_prev, i);
       for (int k = ebegin[i]; k < eend[i]; ++k) {
-        ContactEntry E = ents[k];
-        if (!(E.li & 8)) continue;
-        const ContactDev& C = contacts[E.contact];
+        const int entry = ents[k];
+        if (!(entry & ENTRY_FRICTION)) continue;
+        const ContactDev& C = contacts[(entry & ~ENTRY_FRICTION) >> 2];
         d3 cn = mk(C.n[0], C.n[1], C.n[2]);
         d3 tg = disp - cn * dot(disp, cn);
         double tn = nrm(tg);
@@ -1008,21 +1023,33 @@ __global__ void __launch_bounds__(ASM_SLICE_TPB) k_assemble_scaled_slice(MeshDev
   for (int q = threadIdx.x; q < nsell; q += ASM_SLICE_TPB) vs[q] = ss[q];
 }
 
-// Contact blocks outside the static pattern. Entries of the same (row, col)
-// arrive adjacent (sorted by the 64-bit key row:col, stably, so in contact
-// order) and merge into one block: the FP64 sum of k_extra_values' per-entry
-// blocks, each with its |v| < barrier_tol drop rule. With Linv the merged
-// block is scaled (L_row^-1 H L_col^-T) before the rounding to FP32.
-__global__ void k_extra_key64(const ContactEntry* xent, const int* xkeys, int n, unsigned long long* key, int* idx) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  key[k] = ((unsigned long long)(unsigned)xkeys[k] << 32) | (unsigned long long)(unsigned)xent[k].col;
-  idx[k] = k;
+// Contact blocks outside the static pattern. Each contact's ordered pairs of
+// vertices leave at the contact's offset, in (i, j) order, with the key row:col
+// (`bits` bits each) and 16 * contact + 4 i + j; a stable sort by the key then
+// puts the entries of a block side by side in contact order. Keys are 32 bits
+// wide up to 65,536 vertices and 64 above: the sort moves 8 bytes an entry in
+// place of 12 and passes over 2 * bits bits.
+template <class K>
+__global__ void k_extra_entries(const ContactRec* __restrict__ recs, const int* __restrict__ off, int nc, int bits, K* key, int* id) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = int(t / 16), e = int(t % 16), i = e / 4, j = e % 4;
+  unsigned mask = 0;
+  int row = 0, col = 0;
+  if (c < nc) { mask = recs[c].mask; row = recs[c].idx[i]; col = recs[c].idx[j]; }
+  const bool on = (mask & REC_HESS) && (mask >> i & mask >> j & 1u) && row != col;
+  const unsigned all = __ballot_sync(0xffffffffu, on) >> (threadIdx.x & 16) & 0xffffu;
+  if (!on) return;
+  const int at = off[c] + __popc(all & ((1u << e) - 1u));
+  key[at] = K(row) << bits | K(col);
+  id[at] = 16 * c + e;
 }
-__global__ void k_run_heads(const unsigned long long* key, int n, int* flags) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  flags[k] = (k == 0 || key[k] != key[k - 1]) ? 1 : 0;
+template <class K>
+__global__ void k_extra_rows(const K* __restrict__ key, const int* __restrict__ heads, int nu, int bits, int* xrow, int* xcols) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= nu) return;
+  const K k = key[heads[u]];
+  xrow[u] = int(k >> bits);
+  xcols[u] = int(k & ((K(1) << bits) - 1));
 }
 // SELL-32 layout of the merged blocks for the resident PCG: a slice of 32 rows
 // is as wide as its row with the most blocks. The scan of the slice widths is
@@ -1053,26 +1080,30 @@ __global__ void __launch_bounds__(1024) k_x_scan(int ns, const int* width, long 
   }
   if (threadIdx.x == 0) { off[ns] = int(min(carry, limit)); ctrl->xs_blocks = carry <= limit ? int(carry) : -1; }
 }
-__global__ void k_extra_merge(const ContactDev* cs, const ContactEntry* xent, const unsigned long long* key, const int* idx, const int* heads,
-                              int nu, int n, const unsigned char* fixed, StepParams p, const double* Linv, int* xrow, int* xcols,
-                              float* xval, float* xvalh, XsLayout xs) {
+// The entries of a block merge into one: the FP64 sum of the per-contact blocks
+// in contact order, each value below barrier_tol dropped on its own. With Linv
+// the merged block is scaled (L_row^-1 H L_col^-T) before the rounding to FP32.
+__global__ void __launch_bounds__(128) k_extra_merge(const ContactRec* __restrict__ recs, const int* __restrict__ id, const int* __restrict__ heads,
+                                                     const int* __restrict__ xrow, const int* __restrict__ xcols, int nu, int n,
+                                                     const unsigned char* fixed, StepParams p, const double* __restrict__ Linv, float* xval,
+                                                     float* xvalh, XsLayout xs) {
   int u = blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= nu) return;
   int k0 = heads[u], k1 = u + 1 < nu ? heads[u + 1] : n;
-  int row = int(key[k0] >> 32), col = int(key[k0] & 0xffffffffull);
-  if (xrow) { xrow[u] = row; xcols[u] = col; }
+  const int row = xrow[u], col = xcols[u];
   double H[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   bool zero = fixed && (fixed[row] || fixed[col]);
   if (!zero) {
     for (int k = k0; k < k1; ++k) {
-      ContactEntry E = xent[idx[k]];
-      const ContactDev& C = cs[E.contact];
-      int i = E.li & 3, j = E.lj;
-      d3 nn = mk(C.nn[0], C.nn[1], C.nn[2]);
-      d3 gi = nn * C.w[i], gj = nn * C.w[j];
+      const int e = id[k], i = e >> 2 & 3, j = e & 3;
+      const double2* R = reinterpret_cast<const double2*>(recs + (unsigned(e) >> 4));
+      const double2 a = R[0], b = R[1], c = R[2], d = R[3];   // nn, w, d2V
+      const double wi = i == 0 ? b.y : i == 1 ? c.x : i == 2 ? c.y : d.x, wj = j == 0 ? b.y : j == 1 ? c.x : j == 2 ? c.y : d.x;
+      d3 nn = mk(a.x, a.y, b.x);
+      d3 gi = nn * wi, gj = nn * wj;
       for (int r = 0; r < 3; ++r)
         for (int q = 0; q < 3; ++q) {
-          double v = C.d2V * (comp(gi, r) * comp(gj, q));
+          double v = d.y * (comp(gi, r) * comp(gj, q));
           if (!(fabs(v) < p.barrier_tol)) H[3 * r + q] += v;
         }
     }
@@ -1429,21 +1460,16 @@ void launch_detect_write(const MeshDev& m, const double* x, const RigidDev* bodi
   long long units = (long long)m.V * (1 + nb);
   if (units) k_detect_write<<<nblk(units), TPB, 0, s>>>(m, x, bodies, nb, literal_pt, thresh, offsets, out);
 }
-void launch_contact_prep(const MeshDev& m, ContactDev* c, int nc, const StepParams& p, cudaStream_t s) {
-  if (nc) k_contact_prep<<<nblk(nc), TPB, 0, s>>>(m, c, nc, p);
-}
-void launch_contact_entries(const ContactDev* c, int nc, int V, int friction, int* keys, ContactEntry* ents, cudaStream_t s) {
-  if (nc) k_contact_entries<<<nblk(16ll * nc), TPB, 0, s>>>(c, nc, V, friction, keys, ents);
+void launch_contact_prep(const MeshDev& m, ContactDev* c, int nc, const StepParams& p, int friction, ContactRec* recs, int* keys, int* ents,
+                         int* xcount, cudaStream_t s) {
+  if (nc) k_contact_prep<<<nblk(nc + 1ll), TPB, 0, s>>>(m, c, nc, p, friction, recs, keys, ents, xcount);
 }
 void launch_vertex_ranges(const int* keys, int n, int V, int* begin, int* end, cudaStream_t s) {
   if (V) k_vertex_ranges<<<nblk(V), TPB, 0, s>>>(keys, n, V, begin, end);
 }
-void launch_contact_vertex(const MeshDev& m, const ContactDev* c, const ContactEntry* ents, const int* begin, const int* end,
-                           const StepParams& p, const double* g_base, double* g_const, double* diag_const, cudaStream_t s) {
-  if (m.V) k_contact_vertex<<<nblk(m.V), TPB, 0, s>>>(m, c, ents, begin, end, p, g_base, g_const, diag_const);
-}
-void launch_extra_flags(const ContactEntry* ents, const int* keys, int n, int* flags, cudaStream_t s) {
-  if (n) k_extra_flags<<<nblk(n), TPB, 0, s>>>(ents, keys, n, flags);
+void launch_contact_vertex(int V, const ContactRec* recs, const int* ents, const int* begin, const int* end, const StepParams& p,
+                           const double* g_base, double* g_const, double* diag_const, cudaStream_t s) {
+  if (V) k_contact_vertex<<<nblk(CV_LANES * (long long)V), TPB, 0, s>>>(V, recs, ents, begin, end, p, g_base, g_const, diag_const);
 }
 void launch_ctrl_reset(Ctrl* ctrl, cudaStream_t s) { k_ctrl_reset<<<1, 1, 0, s>>>(ctrl); }
 void launch_strain_face(const MeshDev& m, const double* x, const StepParams& p, unsigned char* flags, StrainSV* sv, Ctrl* ctrl, cudaStream_t s) {
@@ -1455,7 +1481,7 @@ void launch_pin_heads(const int* pin_vertex, int num_pins, int* pin_head, cudaSt
 void launch_gradient(const MeshDev& m, const double* x, const double* x_hat, const double* x_prev, const double* g_const,
                      const double* diag_const, const unsigned char* sflags, const StrainSV* sv,
                      const int* pin_vertex, const int* pin_head, const double* pin_target, int num_pins, const WallDev* walls,
-                     const ContactDev* contacts, const ContactEntry* ents, const int* ebegin, const int* eend,
+                     const ContactDev* contacts, const int* ents, const int* ebegin, const int* eend,
                      const StepParams& p, const unsigned char* fixed, double* g, float* b, double* diag_extra, Ctrl* ctrl, cudaStream_t s) {
   if (m.V) k_gradient<<<nblk(m.V), TPB, 0, s>>>(m, x, x_hat, x_prev, g_const, diag_const, sflags, sv, pin_vertex, pin_head, pin_target, num_pins, walls,
                                                 contacts, ents, ebegin, eend, p, fixed, g, b, diag_extra, ctrl);
@@ -1494,20 +1520,25 @@ void launch_assemble_scaled(const MeshDev& m, const unsigned char* sflags, const
   k_assemble_scaled<<<nblk(m.nnzb, tpb), tpb, 0, s>>>(m, sflags, sv, diag_extra, enable_strain, fixed, Linv, chol_ok, val, valh, sell_base,
                                                       valh_sell, ctrl);
 }
-void launch_extra_key64(const ContactEntry* xent, const int* xkeys, int n, unsigned long long* key, int* idx, cudaStream_t s) {
-  if (n) k_extra_key64<<<nblk(n), TPB, 0, s>>>(xent, xkeys, n, key, idx);
+template <class K>
+void launch_extra_entries(const ContactRec* recs, const int* off, int nc, int bits, K* key, int* id, cudaStream_t s) {
+  if (nc) k_extra_entries<K><<<nblk(16ll * nc), TPB, 0, s>>>(recs, off, nc, bits, key, id);
 }
-void launch_run_heads(const unsigned long long* key, int n, int* flags, cudaStream_t s) {
-  if (n) k_run_heads<<<nblk(n), TPB, 0, s>>>(key, n, flags);
+template <class K>
+void launch_extra_rows(const K* key, const int* heads, int nu, int bits, int* xrow, int* xcols, cudaStream_t s) {
+  if (nu) k_extra_rows<K><<<nblk(nu), TPB, 0, s>>>(key, heads, nu, bits, xrow, xcols);
 }
+template void launch_extra_entries(const ContactRec*, const int*, int, int, unsigned*, int*, cudaStream_t);
+template void launch_extra_entries(const ContactRec*, const int*, int, int, unsigned long long*, int*, cudaStream_t);
+template void launch_extra_rows(const unsigned*, const int*, int, int, int*, int*, cudaStream_t);
+template void launch_extra_rows(const unsigned long long*, const int*, int, int, int*, int*, cudaStream_t);
 void launch_x_layout(int V, const int* begin, const int* end, long long limit, int* width, int* off, Ctrl* ctrl, cudaStream_t s) {
   k_x_widths<<<nblk(V), TPB, 0, s>>>(V, begin, end, width);
   k_x_scan<<<1, 1024, 0, s>>>((V + 31) / 32, width, limit, off, ctrl);
 }
-void launch_extra_merge(const ContactDev* c, const ContactEntry* xent, const unsigned long long* key, const int* idx, const int* heads, int nu,
-                        int n, const unsigned char* fixed, const StepParams& p, const double* Linv, int* xrow, int* xcols, float* xval,
-                        float* xvalh, cudaStream_t s, XsLayout xs) {
-  if (nu) k_extra_merge<<<nblk(nu), TPB, 0, s>>>(c, xent, key, idx, heads, nu, n, fixed, p, Linv, xrow, xcols, xval, xvalh, xs);
+void launch_extra_merge(const ContactRec* recs, const int* id, const int* heads, const int* xrow, const int* xcols, int nu, int n,
+                        const unsigned char* fixed, const StepParams& p, const double* Linv, float* xval, float* xvalh, cudaStream_t s, XsLayout xs) {
+  if (nu) k_extra_merge<<<nblk(nu, 128), 128, 0, s>>>(recs, id, heads, xrow, xcols, nu, n, fixed, p, Linv, xval, xvalh, xs);
 }
 void launch_ls_wall(int V, const double* x, const float* d, WallDev w, Ctrl* ctrl, cudaStream_t s) {
   if (V) k_ls_wall<<<nblk(V), TPB, 0, s>>>(V, x, d, w, ctrl);

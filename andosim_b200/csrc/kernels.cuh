@@ -27,12 +27,11 @@ void launch_rigid_world(RigidDev* bodies_dev, const RigidDev* bodies_host, int n
 // contact detection: count per (PT vertex) + (rigid body, vertex); literal PT only when T == 1.
 void launch_detect_count(const MeshDev& m, const double* x, const RigidDev* bodies, int nb, int literal_pt, double thresh, int* counts, cudaStream_t s);
 void launch_detect_write(const MeshDev& m, const double* x, const RigidDev* bodies, int nb, int literal_pt, double thresh, const int* offsets, ContactDev* out, cudaStream_t s);
-void launch_contact_prep(const MeshDev& m, ContactDev* c, int nc, const StepParams& p, cudaStream_t s);
-void launch_contact_entries(const ContactDev* c, int nc, int V, int friction, int* keys, ContactEntry* ents, cudaStream_t s);
+void launch_contact_prep(const MeshDev& m, ContactDev* c, int nc, const StepParams& p, int friction, ContactRec* recs, int* keys, int* ents,
+                         int* xcount, cudaStream_t s);  // xcount[nc] = 0
 void launch_vertex_ranges(const int* sorted_keys, int n, int V, int* begin, int* end, cudaStream_t s);
-void launch_contact_vertex(const MeshDev& m, const ContactDev* c, const ContactEntry* ents, const int* begin, const int* end,
-                           const StepParams& p, const double* g_base, double* g_const, double* diag_const, cudaStream_t s);
-void launch_extra_flags(const ContactEntry* ents, const int* keys, int n, int* flags, cudaStream_t s);
+void launch_contact_vertex(int V, const ContactRec* recs, const int* ents, const int* begin, const int* end, const StepParams& p,
+                           const double* g_base, double* g_const, double* diag_const, cudaStream_t s);
 
 // Newton iteration
 void launch_ctrl_reset(Ctrl* ctrl, cudaStream_t s);
@@ -40,7 +39,7 @@ void launch_strain_face(const MeshDev& m, const double* x, const StepParams& p, 
 void launch_gradient(const MeshDev& m, const double* x, const double* x_hat, const double* x_prev, const double* g_const,
                      const double* diag_const, const unsigned char* sflags, const StrainSV* sv,
                      const int* pin_vertex, const int* pin_head, const double* pin_target, int num_pins, const WallDev* walls,
-                     const ContactDev* contacts, const ContactEntry* ents, const int* ebegin, const int* eend,
+                     const ContactDev* contacts, const int* ents, const int* ebegin, const int* eend,
                      const StepParams& p, const unsigned char* fixed, double* g, float* b, double* diag_extra, Ctrl* ctrl, cudaStream_t s);
 void launch_check(Ctrl* ctrl, double tol, cudaStream_t s);
 void launch_pin_heads(const int* pin_vertex, int num_pins, int* pin_head, cudaStream_t s);
@@ -64,17 +63,19 @@ void launch_assemble_scaled(const MeshDev& m, const unsigned char* sflags, const
                             const unsigned char* fixed, const double* Linv, const unsigned char* chol_ok, float* val, float* valh,
                             const int* sell_base, float* valh_sell, const Ctrl* ctrl, cudaStream_t s, int tpb = 256,
                             const int* chunk_off = nullptr, int wmax = 0);
-void launch_extra_key64(const ContactEntry* xent, const int* xkeys, int n, unsigned long long* key, int* idx, cudaStream_t s);
-void launch_run_heads(const unsigned long long* key, int n, int* flags, cudaStream_t s);
+template <class K>
+void launch_extra_entries(const ContactRec* recs, const int* off, int nc, int bits, K* key, int* id, cudaStream_t s);
+template <class K>
+void launch_extra_rows(const K* key, const int* heads, int nu, int bits, int* xrow, int* xcols, cudaStream_t s);
 // SELL-32 copy of the merged scaled blocks for the resident PCG: slice offsets
 // (32 x width), columns (-1: padding, set by the caller) and 9 planes of 32
 // lanes per slot; begin = first block of each row
 struct XsLayout { const int* off = nullptr; const int* begin = nullptr; int* col = nullptr; float* val = nullptr; };
 // its slice widths and offsets; ctrl->xs_blocks = places in all, -1 when over `limit`
 void launch_x_layout(int V, const int* begin, const int* end, long long limit, int* width, int* off, Ctrl* ctrl, cudaStream_t s);
-void launch_extra_merge(const ContactDev* c, const ContactEntry* xent, const unsigned long long* key, const int* idx, const int* heads, int nu,
-                        int n, const unsigned char* fixed, const StepParams& p, const double* Linv, int* xrow, int* xcols, float* xval,
-                        float* xvalh, cudaStream_t s, XsLayout xs = XsLayout{});
+void launch_extra_merge(const ContactRec* recs, const int* id, const int* heads, const int* xrow, const int* xcols, int nu, int n,
+                        const unsigned char* fixed, const StepParams& p, const double* Linv, float* xval, float* xvalh, cudaStream_t s,
+                        XsLayout xs = XsLayout{});
 void launch_ls_wall(int V, const double* x, const float* d, WallDev w, Ctrl* ctrl, cudaStream_t s);
 void launch_ls_contacts(const ContactDev* c, int nc, const double* x, const float* d, Ctrl* ctrl, cudaStream_t s);
 void launch_update(int V, double* x, const float* d, Ctrl* ctrl, cudaStream_t s);
