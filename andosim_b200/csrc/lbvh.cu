@@ -32,7 +32,7 @@ namespace ando {
 namespace {
 
 constexpr int TPB = 256;
-inline int nblk(long long n) { return int((n + TPB - 1) / TPB); }
+inline int nblk(long long n, int tpb = TPB) { return int((n + tpb - 1) / tpb); }
 
 using Box = LbvhBox;
 
@@ -454,30 +454,60 @@ __device__ inline void emit(bool hit, int q, int prim, int2* out, int* count, in
   }
 }
 
-// One thread per query. kind 0: query = vertex (point box +-1e-4 inflated by
+// One lane per query. kind 0: query = vertex (point box +-1e-4 inflated by
 // pad), prims = triangles, skip incident triangles. kind 1: query = edge,
 // prims = edges, keep e1 < e2 without shared vertex. kind 2: query = edge,
 // prims = triangles, skip triangles that hold either end of the edge.
 //
-// A query is a chain of dependent node loads, and there are only about 30
-// warps of them to an SM, so what a step waits for is the time. Overlapping
-// leaves therefore go into a shared-memory queue of the warp (ballots, no
-// memory round trip); only when it fills does the warp turn to them, 32 at
-// once: load the leaf, drop incident primitives, close the gaps, and append
-// what is left with one atomic. Testing each leaf where it is met and appending
-// each step's hits with an atomic of its own put two trips through L2 into
-// every step that met a leaf, all of them on the one counter.
-constexpr int QUEUE = 256;   // entries per warp; a step adds at most 128
-__global__ void __launch_bounds__(TPB) k_query(const double* x, const double* x1, const int* qprims, const int* qorder, int kind, int nq, float pad, int n,
+// A descent is a chain of dependent node loads, and with one to a query there
+// were about a hundred of them to a warp, half the lanes idle in each. The queries
+// of a warp are neighbours (Morton order at rest), so the warp descends once for
+// all of them: per step it takes up to eight nodes from its stack, a lane to each
+// child box, and keeps the children that meet one of the warp's group boxes; the
+// leaves found are then tested against every lane's own box, 32 tests a
+// broadcast. A group is the largest aligned run of lanes whose common box is no
+// larger than GROUP_SPREAD (runs of up to four: FOUR_SPREAD) times the patch that
+// as many boxes of their size, or of a primitive's where that is larger (the
+// root's box over sqrt(n)), fill. A run that spans a seam of the order, or sheets
+// that have moved apart, so falls into smaller groups, down to single lanes, in
+// place of descending through all that lies between. The tests that decide are
+// each query's own: the pairs are those of one descent per query.
+//
+// Hits that are not incident (the leaves' vertices are loaded beside the tests)
+// gather in a shared-memory queue of the warp and leave it with one atomic for up
+// to QUEUE of them.
+//
+// Two curtains of 256^2 (swept boxes; 50 to 57 thousand cycles of a warp go to 20
+// steps, half of them, and the rest to 130 leaves and 70 hits): the edge-edge
+// query 156 -> 135 us, vertex-triangle 140 -> 87; four sheets of 96^2, a frame's
+// eight queries 1296 -> 850; one hanging cloth of 97^2, both 117 -> 44. The spread:
+// at 2.0 the sheets' edges take 180 us in place of 166 (long tails of leaves), at
+// 1.0 the curtains' vertices 98 in place of 87 (22 groups a step); runs of up to
+// four lanes may spread twice as far, which halves the groups there and adds no
+// leaves. 64 registers instead of 76 spill and cost a third.
+constexpr int QUEUE = 256;                        // hits per warp
+constexpr int QSTACK = 256, QSTACK_WIDE = 128;    // nodes per warp; above QSTACK_WIDE one node is taken at a time
+constexpr int QLEAVES = 64;                       // leaves per warp; a step adds at most 32
+constexpr int Q_TPB = 128;
+constexpr float GROUP_SPREAD = 1.5f, FOUR_SPREAD = 3.f;
+struct QueryWarp {
+  float4 box[32][2];        // group boxes: lo, hi and the smallest leaf position that concerns the group
+  float4 leaf[QLEAVES][2];  // leaf boxes: lo, hi, position
+  int4 prim[32];            // of the leaves under test: primitive and vertices
+  int2 hits[QUEUE];
+  int stack[QSTACK];
+};
+__global__ void __launch_bounds__(Q_TPB) k_query(const double* x, const double* x1, const int* qprims, const int* qorder, int kind, int nq, float pad, int n,
                         const int4* leafv, const int* rank, const LbvhWide* wide, const Box* nodes, int2* out, int* count, int cap) {
-  __shared__ int2 queue[TPB / 32][QUEUE];
-  int2* const qu = queue[threadIdx.x >> 5];
+  __shared__ __align__(16) QueryWarp warps[Q_TPB / 32];
+  QueryWarp& W = warps[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  int held = 0;   // entries in the queue (uniform over the warp)
+  int held = 0;   // entries in the queue (this and the other counts are uniform over the warp)
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   bool active = t < nq;
   const int q = active && qorder ? qorder[t] : t;
   Box qb;
+  qb.lo[0] = qb.lo[1] = qb.lo[2] = FLT_MAX; qb.hi[0] = qb.hi[1] = qb.hi[2] = -FLT_MAX;
   int qa = -1, qc = -1;
   if (active) {
     if (kind == 0) {
@@ -500,85 +530,146 @@ __global__ void __launch_bounds__(TPB) k_query(const double* x, const double* x1
       if (pad > 0.f) for (int k = 0; k < 3; ++k) { qb.lo[k] -= pad; qb.hi[k] += pad; }
     }
   }
-  // Depth-first traversal of the four-wide hierarchy: each step loads one
-  // 128-byte node and tests its (up to) four child boxes; an overlapping leaf
-  // child is queued, the first overlapping internal child is entered
-  // and the others go on the stack. The binary hierarchy is at most 64 levels
-  // deep with unique 64-bit keys, the four-wide one half that, so three
-  // pushes per level fit 96 slots; an overflow would be reported through
-  // count[1] instead of dropping candidates silently.
-  //
   // The edge-edge query is a self query: each pair is found from the edge
   // that comes first in the tree's sorted leaf order (children whose leaves
   // all come before the query's own position are skipped) and reported with
   // the lower edge index first, which is the set the q < prim rule of a full
   // query gives.
-  constexpr int STACK = 96;
-  int stack[STACK];
-  int sp = 0;
-  const int qpos = active && kind == 1 ? rank[q] : -1;
-  const bool single = active && n == 1;  // one primitive: the root (node 0) is its leaf
-  int node = active && n > 1 ? 0 : -1;
-  auto push = [&](bool hit, int pos) {
-    const unsigned mask = __ballot_sync(0xffffffffu, hit);
-    if (hit) qu[held + __popc(mask & ((1u << lane) - 1u))] = make_int2(q, pos);
-    held += __popc(mask);
-  };
-  auto flush = [&]() {
-    int kept = 0;
-    __syncwarp();
-    for (int k0 = 0; k0 < held; k0 += 32) {
-      bool hit = false;
-      int2 pr = make_int2(0, 0);
-      if (k0 + lane < held) {
-        pr = qu[k0 + lane];
-        const int4 lv = leafv[pr.y];
-        if (kind == 0) hit = lv.y != pr.x && lv.z != pr.x && lv.w != pr.x;
-        else {
-          const int a = qprims[2 * pr.x], b = qprims[2 * pr.x + 1];
-          hit = lv.y != a && lv.y != b && lv.z != a && lv.z != b && (kind == 1 || (lv.w != a && lv.w != b));
-        }
-        // (lower, higher) edge index for the self query
-        pr = kind == 1 ? make_int2(min(pr.x, lv.x), max(pr.x, lv.x)) : make_int2(pr.x, lv.x);
+  const int qpos = !active ? INT_MAX : kind == 1 ? rank[q] : -1;
+  // group boxes: level by level the box of the lane's aligned run of 2^l lanes
+  int groups = 0;
+  {
+    Box u = qb, best = qb;
+    int first = qpos, best_first = qpos, level = 0;
+    const Box root = nodes[0];
+    const float prim = ((root.hi[0] - root.lo[0]) + (root.hi[1] - root.lo[1]) + (root.hi[2] - root.lo[2])) * rsqrtf(float(n));
+    float sum = active ? fmaxf((qb.hi[0] - qb.lo[0]) + (qb.hi[1] - qb.lo[1]) + (qb.hi[2] - qb.lo[2]), prim) : 0.f;
+    int members = active;
+#pragma unroll
+    for (int l = 1; l <= 5; ++l) {
+      const int o = 1 << (l - 1);
+      for (int e = 0; e < 3; ++e) {
+        u.lo[e] = fminf(u.lo[e], __shfl_xor_sync(0xffffffffu, u.lo[e], o));
+        u.hi[e] = fmaxf(u.hi[e], __shfl_xor_sync(0xffffffffu, u.hi[e], o));
       }
-      const unsigned mask = __ballot_sync(0xffffffffu, hit);
-      if (hit) qu[kept + __popc(mask & ((1u << lane) - 1u))] = pr;   // kept <= k0: only entries already read
-      kept += __popc(mask);
-      __syncwarp();
+      first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      members += __shfl_xor_sync(0xffffffffu, members, o);
+      if ((u.hi[0] - u.lo[0]) + (u.hi[1] - u.lo[1]) + (u.hi[2] - u.lo[2]) <= (l <= 2 ? FOUR_SPREAD : GROUP_SPREAD) * sum * rsqrtf(float(max(members, 1)))) {
+        level = l; best = u; best_first = first;
+      }
     }
+    const bool lead = active && (lane & ((1 << level) - 1)) == 0;   // lane 0 of a run is active where any is
+    const unsigned mask = __ballot_sync(0xffffffffu, lead);
+    if (lead) {
+      const int g = __popc(mask & ((1u << lane) - 1u));
+      W.box[g][0] = make_float4(best.lo[0], best.lo[1], best.lo[2], best.hi[0]);
+      W.box[g][1] = make_float4(best.hi[1], best.hi[2], __int_as_float(best_first), 0.f);
+    }
+    groups = __popc(mask);
+  }
+  auto flush = [&]() {
     int base = 0;
-    if (lane == 0 && kept) base = atomicAdd(count, kept);
+    __syncwarp();
+    if (lane == 0) base = atomicAdd(count, held);
     base = __shfl_sync(0xffffffffu, base, 0);
-    for (int k = lane; k < kept; k += 32)
-      if (base + k < cap) out[base + k] = qu[k];
+    for (int k = lane; k < held; k += 32)
+      if (base + k < cap) out[base + k] = W.hits[k];
     held = 0;
     __syncwarp();
   };
-  push(single && overlap(qb, nodes[0]), 0);
-  while (__any_sync(0xffffffffu, node >= 0)) {
-    int h[4] = {-1, -1, -1, -1};
-    if (node >= 0) {
-      const float4* r = reinterpret_cast<const float4*>(wide + node);
-      const float4 f0 = __ldg(r), f1 = __ldg(r + 1), f2 = __ldg(r + 2), f3 = __ldg(r + 3), f4 = __ldg(r + 4), f5 = __ldg(r + 5);
-      const int4 ch = __ldg(reinterpret_cast<const int4*>(r) + 6), cm = __ldg(reinterpret_cast<const int4*>(r) + 7);
-      int next = -1;
-      auto slot = [&](float lox, float loy, float loz, float hix, float hiy, float hiz, int c, int m, int& hk) {
-        if (!(m > qpos && qb.lo[0] <= hix && qb.hi[0] >= lox && qb.lo[1] <= hiy && qb.hi[1] >= loy && qb.lo[2] <= hiz && qb.hi[2] >= loz))
-          return;
-        if (c < 0) hk = -c - 1;
-        else if (next < 0) next = c;
-        else if (sp < STACK) stack[sp++] = c;
-        else atomicAdd(count + 1, 1);
-      };
-      slot(f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, ch.x, cm.x, h[0]);
-      slot(f1.z, f1.w, f2.x, f2.y, f2.z, f2.w, ch.y, cm.y, h[1]);
-      slot(f3.x, f3.y, f3.z, f3.w, f4.x, f4.y, ch.z, cm.z, h[2]);
-      slot(f4.z, f4.w, f5.x, f5.y, f5.z, f5.w, ch.w, cm.w, h[3]);
-      node = next >= 0 ? next : (sp > 0 ? stack[--sp] : -1);
+  // The binary hierarchy is at most 64 levels deep with unique 64-bit keys, the
+  // four-wide one half that. Eight nodes at a time are taken from a stack of up to
+  // QSTACK_WIDE nodes and add at most 24; one at a time then adds three a level:
+  // 128 + 24 + 96 nodes. An overflow would be reported through count[1] instead
+  // of dropping candidates silently.
+  int sp = 0, nl = 0;
+  if (groups > 0) {
+    if (n > 1) {
+      sp = 1;
+      if (lane == 0) W.stack[0] = 0;
+    } else {       // one primitive: the root (node 0) is its leaf
+      nl = 1;
+      if (lane == 0) {
+        const Box b = nodes[0];
+        W.leaf[0][0] = make_float4(b.lo[0], b.lo[1], b.lo[2], b.hi[0]);
+        W.leaf[0][1] = make_float4(b.hi[1], b.hi[2], __int_as_float(0), 0.f);
+      }
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) push(h[k] >= 0 && h[k] > qpos, h[k]);
-    if (held > QUEUE - 128) flush();
+  }
+  __syncwarp();
+  while (sp > 0 || nl > 0) {
+    if (sp > 0) {
+      const int take = sp <= QSTACK_WIDE ? min(8, sp) : 1;
+      const int node = (lane >> 2) < take ? W.stack[sp - 1 - (lane >> 2)] : -1, k = lane & 3;
+      sp -= take;
+      float2 a = make_float2(FLT_MAX, FLT_MAX), b = make_float2(FLT_MAX, -FLT_MAX), c = make_float2(-FLT_MAX, -FLT_MAX);
+      int child = 0, last = INT_MIN;
+      if (node >= 0) {
+        const float2* r = reinterpret_cast<const float2*>(wide + node) + 3 * k;
+        a = __ldg(r); b = __ldg(r + 1); c = __ldg(r + 2);
+        child = __ldg(reinterpret_cast<const int*>(wide + node) + 24 + k);
+        last = __ldg(reinterpret_cast<const int*>(wide + node) + 28 + k);
+      }
+      bool hit = false;
+      for (int g = 0; g < groups; ++g) {
+        const float4 u = W.box[g][0], w = W.box[g][1];
+        hit |= (last > __float_as_int(w.z)) & (u.x <= b.y) & (u.w >= a.x) & (u.y <= c.x) & (w.x >= a.y) & (u.z <= c.y) & (w.y >= b.x);
+      }
+      const unsigned inner = __ballot_sync(0xffffffffu, hit && child >= 0), leaves = __ballot_sync(0xffffffffu, hit && child < 0);
+      if (hit && child >= 0) {
+        const int at = sp + __popc(inner & ((1u << lane) - 1u));
+        if (at < QSTACK) W.stack[at] = child;
+        else atomicAdd(count + 1, 1);
+      }
+      if (hit && child < 0) {
+        const int at = nl + __popc(leaves & ((1u << lane) - 1u));
+        W.leaf[at][0] = make_float4(a.x, a.y, b.x, b.y);
+        W.leaf[at][1] = make_float4(c.x, c.y, __int_as_float(-child - 1), 0.f);
+      }
+      sp = min(sp + __popc(inner), QSTACK);
+      nl += __popc(leaves);
+      __syncwarp();
+    }
+    while (nl >= 32 || (sp == 0 && nl > 0)) {
+      const int m = min(nl, 32);
+      nl -= m;
+      int4 mine = make_int4(0, 0, 0, 0);
+      if (lane < m) mine = leafv[__float_as_int(W.leaf[nl + lane][1].z)];
+      unsigned met = 0;   // bit e: the lane's box meets leaf nl + e
+#pragma unroll 8
+      for (int e = 0; e < m; ++e) {
+        const float4 u = W.leaf[nl + e][0], w = W.leaf[nl + e][1];
+        const bool h = (__float_as_int(w.z) > qpos) & (qb.lo[0] <= u.w) & (qb.hi[0] >= u.x) & (qb.lo[1] <= w.x) & (qb.hi[1] >= u.y) &
+                       (qb.lo[2] <= w.y) & (qb.hi[2] >= u.z);
+        met |= unsigned(h) << e;
+      }
+      W.prim[lane] = mine;
+      __syncwarp();
+      for (unsigned left = met; left; left &= left - 1) {
+        const int e = __ffs(left) - 1;
+        const int4 lv = W.prim[e];
+        const bool incident = kind == 0 ? (lv.y == q) | (lv.z == q) | (lv.w == q)
+                                        : (lv.y == qa) | (lv.y == qc) | (lv.z == qa) | (lv.z == qc) | (kind == 2 && (lv.w == qa || lv.w == qc));
+        met ^= unsigned(incident) << e;
+      }
+      while (__any_sync(0xffffffffu, met != 0)) {
+        // as many of each lane's hits as the queue takes from all lanes
+        const int room = QUEUE - held;
+        int mineto = __popc(met), upto = mineto;
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += v; }
+        const int total = __shfl_sync(0xffffffffu, upto, 31);
+        int at = upto - mineto;
+        for (; met && at < room; met &= met - 1, ++at) {
+          const int prim = W.prim[__ffs(met) - 1].x;
+          // (lower, higher) edge index for the self query
+          W.hits[held + at] = kind == 1 ? make_int2(min(q, prim), max(q, prim)) : make_int2(q, prim);
+        }
+        held += min(total, room);
+        if (held == QUEUE) flush();
+      }
+      __syncwarp();
+    }
   }
   if (held) flush();
 }
@@ -857,7 +948,7 @@ cudaError_t run_query(Lbvh& B, const double* x, const double* x1, int kind, cons
   for (int attempt = 0; attempt < 2; ++attempt) {
     int cap = int(scratch.n);
     if ((e = cudaMemsetAsync(counter.p, 0, 3 * sizeof(int), s))) return e;
-    k_query<<<nblk(nq), TPB, 0, s>>>(x, x1, qprims, B.qorder, kind, nq, pad, B.n, B.leafv.p, B.rank.p, B.wide.p, B.nodes.p,
+    k_query<<<nblk(nq, Q_TPB), Q_TPB, 0, s>>>(x, x1, qprims, B.qorder, kind, nq, pad, B.n, B.leafv.p, B.rank.p, B.wide.p, B.nodes.p,
                                      scratch.p, counter.p, cap);
     B.launches += 1;
     int cnt2[2] = {0, 0};
@@ -893,7 +984,7 @@ cudaError_t Lbvh::contacts_launch(const double* x, int kind, const int* qprims, 
   if (scratch.n < 1024) if ((e = scratch.reserve(1024))) return e;
   if ((e = surv.reserve(scratch.n))) return e;
   const int cap = int(scratch.n);
-  k_query<<<nblk(nq), TPB, 0, s>>>(x, nullptr, qprims, qorder, kind, nq, pad, n, leafv.p, rank.p, wide.p, nodes.p, scratch.p, counter.p, cap);
+  k_query<<<nblk(nq, Q_TPB), Q_TPB, 0, s>>>(x, nullptr, qprims, qorder, kind, nq, pad, n, leafv.p, rank.p, wide.p, nodes.p, scratch.p, counter.p, cap);
   k_pairs_gap<<<NARROW_GRID, TPB, 0, s>>>(scratch.p, counter.p, cap, kind, prims, qprims, x, gap, surv.p, counter.p + 2);
   launches += 2;
   return cudaGetLastError();
@@ -922,7 +1013,7 @@ cudaError_t Lbvh::query_toi(const double* x, const double* x1, const double* ext
   if (scratch.n < 1024) if ((e = scratch.reserve(1024))) return e;
   const int cap = int(scratch.n);
   if ((e = cudaMemsetAsync(counter.p, 0, 3 * sizeof(int), s))) return e;
-  k_query<<<nblk(nq), TPB, 0, s>>>(x, x1, qprims, qorder, kind, nq, pad, n, leafv.p, rank.p, wide.p, nodes.p, scratch.p, counter.p, cap);
+  k_query<<<nblk(nq, Q_TPB), Q_TPB, 0, s>>>(x, x1, qprims, qorder, kind, nq, pad, n, leafv.p, rank.p, wide.p, nodes.p, scratch.p, counter.p, cap);
   k_pairs_toi<<<NARROW_GRID, TPB, 0, s>>>(scratch.p, counter.p, cap, kind, prims, qprims, x, x1, ext, pad, eta_min, near, toi, overflow);
   launches += 2;
   return cudaGetLastError();
@@ -956,7 +1047,7 @@ cudaError_t Lbvh::count_crossings(const double* x, const int* edges, int ne, flo
     const int cap = int(scratch.n);
     if ((e = cudaMemsetAsync(counter.p, 0, 3 * sizeof(int), s))) return e;
     if ((e = cudaMemsetAsync(total.p, 0, sizeof(unsigned long long), s))) return e;
-    k_query<<<nblk(ne), TPB, 0, s>>>(x, nullptr, edges, qorder, 2, ne, pad, n, leafv.p, rank.p, wide.p, nodes.p, scratch.p, counter.p, cap);
+    k_query<<<nblk(ne, Q_TPB), Q_TPB, 0, s>>>(x, nullptr, edges, qorder, 2, ne, pad, n, leafv.p, rank.p, wide.p, nodes.p, scratch.p, counter.p, cap);
     k_pairs_cross<<<NARROW_GRID, TPB, 0, s>>>(scratch.p, counter.p, cap, prims, edges, x, total.p);
     launches += 2;
     int cnt2[2] = {0, 0};
