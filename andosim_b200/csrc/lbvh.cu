@@ -199,16 +199,23 @@ __device__ inline Box unite(const Box& a, const Box& b) {
 // parent has more ("cut subtree"). Above it: the top nodes (more than RF_CUT
 // leaves), numbered compactly.
 //
-// k_refit_cut: one CTA per cut subtree (grid-stride over the cut list). With
-// Karras numbering a node covering leaves [lo, hi] has its index in [lo, hi],
-// so every node of a subtree over [c0, c1] has a shared-memory slot (index -
-// c0): the subtree's topology is staged once, each node is finished in shared
-// memory by the second of its children to arrive (block-scope arrival
-// counters), and the subtree's node boxes and child records are written in
-// one pass afterwards; thread 0 puts the subtree's root box into its parent's
-// record. The leaf boxes are computed from the positions here.
+// k_refit_cut: one CTA per cut subtree (grid-stride over the cut list). A
+// node covers a run of leaves, so its box is a minimum over that run: the CTA
+// builds the boxes of 2, 4, 8, ... leaves from each position (ten rounds of one
+// unite a leaf, one barrier each), and after the round that fits its length each
+// node unites the two runs that cover its own. Nothing waits for a child and all
+// lanes work in every round; climbing from the leaves with arrival counters
+// took a chain of some fifteen shared-memory atomics and fences at 14 active
+// lanes of 32, and its staged topology left room for three CTAs of 512 on an SM.
+// Boxes go to the four-wide records only; of the binary nodes' boxes just the
+// subtree's root is read again. The leaf boxes are computed from the positions
+// here. Shared-memory bandwidth bounds it now (some 18 accesses a leaf and round).
+// A frame's refits: two curtains of 151^2 499 -> 280 us, of 256^2 818 -> 627, four
+// sheets of 96^2 276 -> 169; one cloth of 97^2 31 -> 19. Two leaves to a thread,
+// three CTAs of 512: 564 for the largest but 327 and 187 for the others.
 //
-// k_refit_top: one CTA finishes the top nodes the same way in shared memory,
+// k_refit_top: one CTA finishes the top nodes in shared memory, each by the second
+// of its children to arrive (block-scope arrival counters),
 // reading the cut subtrees' boxes from nodes[], and writes them in one pass.
 //
 // When the top has more nodes than one CTA holds (or than the caller's
@@ -217,8 +224,7 @@ __device__ inline Box unite(const Box& a, const Box& b) {
 // second arrival zeroes the counter for the next refit) and k_refit_top does
 // nothing. Min/max are exact, so every box has the same bits in any arrival
 // order.
-constexpr int RF_TPB = 512, RF_CUT = 1024;
-struct RefitSmem { Box leaf[RF_CUT]; Box node[RF_CUT]; int4 topo[RF_CUT]; int arr[RF_CUT]; };
+constexpr int RF_CUT = 1024;   // leaves of a subtree, and threads of its CTA
 constexpr int TOP_TPB = 1024, TOP_MAX = 4096;
 // top node: {node index, parent's top number (-1 at the root), left, right};
 // a child is its top number (>= 0) or -(1 + its nodes[] index) below the cut
@@ -262,96 +268,81 @@ __device__ inline void store_slot(LbvhWide* wide, int ws, const Box& b) {
   d[2] = make_float2(b.hi[1], b.hi[2]);
 }
 
-// The climbs below touch shared memory only (their block-scope fences then
-// have no global store to wait for); each kernel writes its boxes to global
-// memory in one pass after the climb.
-__global__ void __launch_bounds__(RF_TPB) k_refit_cut(const double* x, const double* x1, const int* prims, int arity, float pad,
-                                                      const int* order, int n, const int* parent, const int4* topo, const int2* cuts,
-                                                      const int* meta, int top_cap, Box* nodes, int* arrive, const int* wslot, LbvhWide* wide) {
-  extern __shared__ __align__(16) unsigned char rf_raw[];
-  RefitSmem& S = *reinterpret_cast<RefitSmem*>(rf_raw);
-  const int ncut = meta[1];
+__global__ void __launch_bounds__(RF_CUT, 2) k_refit_cut(const double* x, const double* x1, const int* prims, int arity, float pad,
+                                                         const int* order, int n, const int* parent, const int4* topo, const int2* cuts,
+                                                         const int* meta, int top_cap, Box* nodes, int* arrive, const int* wslot, LbvhWide* wide) {
+  __shared__ float run[2][6][RF_CUT];   // boxes of runs of 2^k leaves from each position, even and odd k
+  const int ncut = meta[1], t = threadIdx.x;
   const bool top_global = meta[0] > top_cap;
+  auto load = [&](int k, int i) {
+    Box b;
+    for (int e = 0; e < 3; ++e) { b.lo[e] = run[k & 1][e][i]; b.hi[e] = run[k & 1][3 + e][i]; }
+    return b;
+  };
+  auto store = [&](int k, const Box& b) {
+    for (int e = 0; e < 3; ++e) { run[k & 1][e][t] = b.lo[e]; run[k & 1][3 + e][t] = b.hi[e]; }
+  };
   for (int cb = blockIdx.x; cb < ncut; cb += gridDim.x) {
     const int2 cut = cuts[cb];
     if (cut.x < 0) continue;  // uniform over the CTA
-    const int c0 = cut.x, c1 = cut.y;
-    __syncthreads();  // the previous subtree's shared memory is no longer read
-    for (int t = threadIdx.x; t <= c1 - c0; t += RF_TPB) {
-      S.arr[t] = 0;
-      const int q = c0 + t;
-      if (q < n - 1) S.topo[t] = topo[q];
-      S.leaf[t] = prim_box(x, x1, prims, arity, order[q], pad);
+    const int c0 = cut.x, m = cut.y - c0 + 1, q = c0 + t;
+    const bool leaf = t < m, inner = leaf && q < n - 1;
+    const int prim = leaf ? order[q] : -1, wl = leaf ? wslot[n - 1 + q] : -1, wn = inner ? wslot[q] : -1;
+    int first = 0, length = 0;
+    if (inner) {
+      const int4 tp = topo[q];
+      // a node that is not wholly in this subtree is another's, or a top node
+      if (tp.x >= c0 && tp.z < c0 + m) { first = tp.x - c0; length = tp.z - tp.x + 1; }
+    }
+    __syncthreads();  // the previous subtree's boxes are no longer read
+    Box box;
+    if (leaf) {
+      box = prim_box(x, x1, prims, arity, prim, pad);
+      store(0, box);
+      if (wl >= 0) store_slot(wide, wl, box);
+      if (m == 1) nodes[n - 1 + c0] = box;
     }
     __syncthreads();
-    const int4 outside = make_int4(-1, 0, 0, -1);  // fails the inside test
-    for (int t = threadIdx.x; t <= c1 - c0; t += RF_TPB) {
-      const int i = c0 + t;
-      Box box = S.leaf[t];
-      int chi = i;  // last leaf under the current node
-      int p = n > 1 ? parent[n - 1 + i] : -1;
-      int4 tp = p >= c0 && p <= c1 ? S.topo[p - c0] : outside;
-      while (p >= 0 && tp.x >= c0 && tp.z <= c1) {  // p's leaves all in this subtree
-        const int plo = tp.x, pl = tp.y, phi = tp.z, pp = tp.w;
-        const bool from_left = chi == pl;
-        // the sibling covers [sl, sh]: a leaf when sl == sh, else internal node sidx
-        const int sl = from_left ? pl + 1 : plo, sh = from_left ? phi : pl, sidx = from_left ? pl + 1 : pl;
-        __threadfence_block();
-        if (atomicAdd(&S.arr[p - c0], 1) == 0) break;
-        __threadfence_block();
-        box = unite(box, sl == sh ? ld_box_volatile(&S.leaf[sl - c0]) : ld_box_volatile(&S.node[sidx - c0]));
-        S.node[p - c0] = box;
-        chi = phi;
-        p = pp;
-        tp = p >= c0 && p <= c1 ? S.topo[p - c0] : outside;
+    for (int k = 1; (1 << k) <= m; ++k) {
+      if (t + (1 << k) <= m) {   // there is such a run
+        box = unite(box, load(k - 1, t + (1 << (k - 1))));
+        store(k, box);
       }
-    }
-    __syncthreads();
-    // write-out: the boxes of the subtree's leaves and internal nodes, each
-    // also into its four-wide slot
-    for (int t = threadIdx.x; t <= c1 - c0; t += RF_TPB) {
-      const int q = c0 + t;
-      nodes[n - 1 + q] = S.leaf[t];
-      const int wl = wslot[n - 1 + q];
-      if (wl >= 0) store_slot(wide, wl, S.leaf[t]);
-      if (q < n - 1) {
-        const int4 tq = S.topo[t];
-        if (tq.x >= c0 && tq.z <= c1) {
-          nodes[q] = S.node[t];
-          const int wn = wslot[q];
-          if (wn >= 0) store_slot(wide, wn, S.node[t]);
-        }
+      __syncthreads();
+      if (length >> k == 1) {
+        const Box b = unite(load(k, first), load(k, first + length - (1 << k)));
+        if (wn >= 0) store_slot(wide, wn, b);
+        if (length == m) nodes[q] = b;
       }
     }
     // with more top nodes than k_refit_top holds, thread 0 carries on from
-    // the subtree's root (index c0 or c1, or the leaf) through the top nodes;
-    // that needs every thread's nodes[] published first
+    // the subtree's root (index c0 or c1, or the leaf) through the top nodes,
+    // once the root's box is published
     if (top_global) {
       __threadfence();
       __syncthreads();
     }
     if (top_global && threadIdx.x == 0) {
+      const int c1 = cut.y;
       int root = -1;  // internal root index, -1: a single leaf
-      if (c1 > c0) root = (S.topo[0].x == c0 && S.topo[0].z == c1) ? c0 : c1;
-      Box box = root < 0 ? S.leaf[0] : S.node[root - c0];
-      int p = root < 0 ? (n > 1 ? parent[n - 1 + c0] : -1) : S.topo[root - c0].w;
+      if (m > 1) root = c0 < n - 1 && topo[c0].x == c0 && topo[c0].z == c1 ? c0 : c1;
+      Box up = ld_box_cg(nodes + (root < 0 ? n - 1 + c0 : root));
+      int p = root < 0 ? (n > 1 ? parent[n - 1 + c0] : -1) : topo[root].w;
       int chi = c1;
-      if (p >= 0) {
-        while (p >= 0) {
-          const int4 tp = __ldg(topo + p);
-          const bool from_left = chi == tp.y;
-          int prior;
-          asm volatile("atom.add.acq_rel.gpu.s32 %0, [%1], 1;" : "=r"(prior) : "l"(arrive + p) : "memory");
-          if (prior == 0) break;
-          arrive[p] = 0;
-          const int sl = from_left ? tp.y + 1 : tp.x, sh = from_left ? tp.z : tp.y, sidx = from_left ? tp.y + 1 : tp.y;
-          box = unite(box, ld_box_cg(nodes + (sl == sh ? n - 1 + sl : sidx)));
-          nodes[p] = box;
-          const int wp = wslot[p];
-          if (wp >= 0) store_slot(wide, wp, box);
-          chi = tp.z;
-          p = tp.w;
-        }
+      while (p >= 0) {
+        const int4 tp = __ldg(topo + p);
+        const bool from_left = chi == tp.y;
+        int prior;
+        asm volatile("atom.add.acq_rel.gpu.s32 %0, [%1], 1;" : "=r"(prior) : "l"(arrive + p) : "memory");
+        if (prior == 0) break;
+        arrive[p] = 0;
+        const int sl = from_left ? tp.y + 1 : tp.x, sh = from_left ? tp.z : tp.y, sidx = from_left ? tp.y + 1 : tp.y;
+        up = unite(up, ld_box_cg(nodes + (sl == sh ? n - 1 + sl : sidx)));
+        nodes[p] = up;
+        const int wp = wslot[p];
+        if (wp >= 0) store_slot(wide, wp, up);
+        chi = tp.z;
+        p = tp.w;
       }
     }
   }
@@ -894,16 +885,15 @@ cudaError_t Lbvh::refit(const double* x, const double* x1, float pad, cudaStream
 // The global arrival counters are zero between refits: the build zeroes them
 // and every refit leaves them zero (each node's second arrival resets it).
 cudaError_t Lbvh::launch_refit(const double* x, const double* x1, float pad, cudaStream_t s) {
-  static_assert(sizeof(RefitSmem) <= 227 * 1024 && sizeof(TopSmem) <= 227 * 1024, "refit tile exceeds shared memory");
-  // Once per device: the call is 0.3 us from one thread and 200 us when sixteen
+  static_assert(sizeof(TopSmem) <= 227 * 1024, "refit tile exceeds shared memory");
+  // Set once per device: the call is 0.3 us from one thread and 200 us when sixteen
   // contexts step at once, for it waits there for the others' launches.
   static std::atomic<unsigned> attr{0};
   cudaError_t e = cudaSuccess;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 32 || !(attr.load() & (1u << dev))) {
-    e = cudaFuncSetAttribute(k_refit_cut, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(RefitSmem)));
-    if (!e) e = cudaFuncSetAttribute(k_refit_top, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TopSmem)));
+    e = cudaFuncSetAttribute(k_refit_top, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TopSmem)));
     if (e) return e;
     if (dev < 32) attr.fetch_or(1u << dev);
   }
@@ -919,10 +909,10 @@ cudaError_t Lbvh::launch_refit(const double* x, const double* x1, float pad, cud
     return n;
   }();
   // grid-stride over the cut list (its length stays on the device): about
-  // three subtrees per SM resident at once
-  const int grid = std::max(1, std::min(3 * sms, 2 * ((n + 255) / 256)));
+  // two subtrees per SM resident at once
+  const int grid = std::max(1, std::min(2 * sms, 2 * ((n + 255) / 256)));
   const int cap = top_cap < 0 || top_cap > TOP_MAX ? TOP_MAX : top_cap;
-  k_refit_cut<<<grid, RF_TPB, sizeof(RefitSmem), s>>>(x, x1, prims, arity, pad, order.p, n, parent.p, topo.p, cuts.p, meta.p, cap,
+  k_refit_cut<<<grid, RF_CUT, 0, s>>>(x, x1, prims, arity, pad, order.p, n, parent.p, topo.p, cuts.p, meta.p, cap,
                                                       nodes.p, arrive.p, wslot.p, wide.p);
   if (n > RF_CUT) k_refit_top<<<1, TOP_TPB, sizeof(TopSmem), s>>>(meta.p, cap, toprec.p, nodes.p, wslot.p, wide.p);
   return cudaGetLastError();
