@@ -154,9 +154,10 @@ struct ando_ctx_s {
   WallDev first_wall_host{};
 
   // whole-frame CUDA graph (REFERENCE semantics without contact detection)
-  bool one_stream = false;         // the broad phase's halves one after the other (batch steps)
-  cudaStream_t cap2 = nullptr, cap3 = nullptr;
-  // the edge-edge broad phase runs on `side` beside the vertex-triangle one
+  cudaStream_t cap2 = nullptr;     // capture of the frame graph's loop body
+  // the edge-edge broad phase runs on `side` beside the vertex-triangle one,
+  // or after it on the main stream (one_stream: batch steps)
+  bool one_stream = false;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   DevBuf<unsigned char> cub_tmp_side;
@@ -217,7 +218,6 @@ struct ando_ctx_s {
     if (frame_exec) cudaGraphExecDestroy(frame_exec);
     if (sctl_host) cudaFreeHost(sctl_host);
     if (cap2) cudaStreamDestroy(cap2);
-    if (cap3) cudaStreamDestroy(cap3);
     if (side) cudaStreamDestroy(side);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
@@ -622,12 +622,11 @@ int inner_newton(ando_ctx c, const ando_params& p, const StepParams& sp, ando_st
       launch_gradient(m, c->x.p, c->x_hat.p, c->x_prev.p, c->g_const.p, c->diag_const.p, c->sflags.p, c->sv.p,
                       c->pin_vertex.p, c->pin_head.p, c->pin_target.p, c->num_pins, c->walls.p, c->contacts.p, c->ents_sorted.p,
                       c->ebegin.p, c->eend.p, sp, nullptr, c->g.p, c->b.p, c->diag_extra.p, c->ctrl.p, c->stream);
-      launch_check(c->ctrl.p, p.pcg_tol, c->stream);
-      ph.launched(2);
+      ph.launched();
     }
     {
       Phase ph(c, ANDO_PHASE_ASSEMBLE);
-      launch_assemble(m, c->sflags.p, c->sv.p, c->diag_extra.p, sp.enable_strain, nullptr, c->val.p, c->precond.p, c->ctrl.p, c->stream);
+      launch_assemble(m, c->sflags.p, c->sv.p, c->diag_extra.p, sp.enable_strain, nullptr, c->val.p, c->precond.p, c->ctrl.p, p.pcg_tol, c->stream);
       ph.launched();
     }
     {
@@ -1160,34 +1159,15 @@ int grow_toi_candidates(ando_ctx c, int need) {
   return ANDO_OK;
 }
 
-// One Newton iteration of the REFERENCE step as a fixed launch sequence
-// (also the body of the graph's inner loop).
-void enqueue_reference_iteration(ando_ctx c, const ando_params& p, const StepParams& sp, const PcgArgs& pa, bool ls_wall,
-                                 const WallDev& wall, cudaStream_t s, cudaError_t& err) {
-  MeshDev m = c->mesh_dev();
-  launch_ctrl_reset(c->ctrl.p, s);
-  if (sp.enable_strain) launch_strain_face(m, c->x.p, sp, c->sflags.p, c->sv.p, c->ctrl.p, s);
-  launch_gradient(m, c->x.p, c->x_hat.p, c->x_prev.p, c->g_const.p, c->diag_const.p, c->sflags.p, c->sv.p,
-                  c->pin_vertex.p, c->pin_head.p, c->pin_target.p, c->num_pins, c->walls.p, c->contacts.p, c->ents_sorted.p,
-                  c->ebegin.p, c->eend.p, sp, nullptr, c->g.p, c->b.p, c->diag_extra.p, c->ctrl.p, s);
-  launch_check(c->ctrl.p, p.pcg_tol, s);
-  launch_assemble(m, c->sflags.p, c->sv.p, c->diag_extra.p, sp.enable_strain, nullptr, c->val.p, c->precond.p, c->ctrl.p, s);
-  cudaError_t e = launch_pcg(pa, s);
-  if (e != cudaSuccess && err == cudaSuccess) err = e;
-  if (ls_wall) launch_ls_wall(c->V, c->x.p, c->d.p, wall, c->ctrl.p, s);
-  launch_update(c->V, c->x.p, c->d.p, c->ctrl.p, s);
-}
-
-int kernels_per_iteration(const StepParams& sp, bool ls_wall) { return 7 + (sp.enable_strain ? 1 : 0) + (ls_wall ? 1 : 0); }
+int kernels_per_iteration(const StepParams& sp, bool ls_wall) { return 4 + (sp.enable_strain ? 1 : 0) + (ls_wall ? 1 : 0); }
 
 // Capture the whole REFERENCE frame (no contacts) as one graph:
 //   predict, per-step constants, control init,
-//   WHILE(inner steps) { inner begin, WHILE(Newton) { iteration, Newton control }, beta control },
+//   WHILE { Newton iteration; its last kernel decides on the next one and on the beta loop },
 //   velocity update, control block -> host.
 int capture_frame(ando_ctx c, const ando_params& p, const StepParams& sp, bool ls_wall, const WallDev& wall) {
-  CK(need_stream(c->cap2)); CK(need_stream(c->cap3));
-  cudaStream_t s = c->stream, s2 = c->cap2, s3 = c->cap3;
-  cudaError_t err = cudaSuccess;
+  CK(need_stream(c->cap2));
+  cudaStream_t s = c->stream, s2 = c->cap2;
   int max_it = p.max_newton_steps;
   if (p.enable_friction) max_it = std::max(max_it, p.friction_min_newton_steps);
   PcgArgs pa;
@@ -1200,7 +1180,6 @@ int capture_frame(ando_ctx c, const ando_params& p, const StepParams& sp, bool l
   int depth = 0;   // open captures, closed on failure
   auto abort_capture = [&](const char* what, cudaError_t e) {
     cudaGraph_t g;
-    if (depth >= 3) cudaStreamEndCapture(s3, &g);
     if (depth >= 2) cudaStreamEndCapture(s2, &g);
     if (depth >= 1) { cudaStreamEndCapture(s, &g); if (g) cudaGraphDestroy(g); }
     cudaGetLastError();
@@ -1210,55 +1189,41 @@ int capture_frame(ando_ctx c, const ando_params& p, const StepParams& sp, bool l
   CAP(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "begin");
   depth = 1;
   launch_predict(c->V, c->x.p, c->v.p, p.dt, c->x_old.p, c->x_hat.p, s);
-  CAP(cudaMemsetAsync(c->ebegin.p, 0, sizeof(int) * c->V, s), "memset");
-  CAP(cudaMemsetAsync(c->eend.p, 0, sizeof(int) * c->V, s), "memset");
-  launch_contact_vertex(c->V, c->crec.p, c->ents_sorted.p, c->ebegin.p, c->eend.p, sp, c->g_el.p, c->g_const.p, c->diag_const.p, s);
+  if (sp.enable_friction) {   // the gradient walks the (empty) contact lists
+    CAP(cudaMemsetAsync(c->ebegin.p, 0, sizeof(int) * c->V, s), "memset");
+    CAP(cudaMemsetAsync(c->eend.p, 0, sizeof(int) * c->V, s), "memset");
+  }
+  launch_contact_vertex(c->V, c->crec.p, c->ents_sorted.p, nullptr, nullptr, sp, c->g_el.p, c->g_const.p, c->diag_const.p, s);
   cudaStreamCaptureStatus cs;
   cudaGraph_t g = nullptr;
   const cudaGraphNode_t* deps = nullptr;
   size_t nd = 0;
   CAP(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd), "capture info");
-  cudaGraphConditionalHandle h_outer;
-  CAP(cudaGraphConditionalHandleCreate(&h_outer, g, 0, 0), "outer handle");
-  launch_ctl_init(c->sctl.p, p.beta_max, max_it, h_outer, s);
+  cudaGraphConditionalHandle h_loop;
+  CAP(cudaGraphConditionalHandleCreate(&h_loop, g, 0, 0), "loop handle");
+  launch_ctl_init(c->sctl.p, p.beta_max, max_it, c->ctrl.p, h_loop, s);
   CAP(cudaGetLastError(), "ctl init");
   CAP(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd), "capture info");
   cudaGraphNodeParams cp = {};
   cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = h_outer;
+  cp.conditional.handle = h_loop;
   cp.conditional.type = cudaGraphCondTypeWhile;
   cp.conditional.size = 1;
-  cudaGraphNode_t n_outer;
-  CAP(cudaGraphAddNode(&n_outer, g, deps, nd, &cp), "outer node");
-  CAP(cudaStreamUpdateCaptureDependencies(s, &n_outer, 1, cudaStreamSetCaptureDependencies), "deps");
-  cudaGraph_t body_outer = cp.conditional.phGraph_out[0];
-  CAP(cudaStreamBeginCaptureToGraph(s2, body_outer, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "begin outer body");
+  cudaGraphNode_t n_loop;
+  CAP(cudaGraphAddNode(&n_loop, g, deps, nd, &cp), "loop node");
+  CAP(cudaStreamUpdateCaptureDependencies(s, &n_loop, 1, cudaStreamSetCaptureDependencies), "deps");
+  CAP(cudaStreamBeginCaptureToGraph(s2, cp.conditional.phGraph_out[0], nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "begin body");
   depth = 2;
-  cudaGraphConditionalHandle h_newton;
-  CAP(cudaGraphConditionalHandleCreate(&h_newton, body_outer, 0, 0), "newton handle");
-  launch_inner_begin(c->sctl.p, h_newton, s2);
-  cudaGraph_t g2 = nullptr;
-  CAP(cudaStreamGetCaptureInfo(s2, &cs, nullptr, &g2, &deps, &nd), "capture info 2");
-  cudaGraphNodeParams cp2 = {};
-  cp2.type = cudaGraphNodeTypeConditional;
-  cp2.conditional.handle = h_newton;
-  cp2.conditional.type = cudaGraphCondTypeWhile;
-  cp2.conditional.size = 1;
-  cudaGraphNode_t n_newton;
-  CAP(cudaGraphAddNode(&n_newton, g2, deps, nd, &cp2), "newton node");
-  CAP(cudaStreamUpdateCaptureDependencies(s2, &n_newton, 1, cudaStreamSetCaptureDependencies), "deps 2");
-  cudaGraph_t body_newton = cp2.conditional.phGraph_out[0];
-  CAP(cudaStreamBeginCaptureToGraph(s3, body_newton, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal), "begin newton body");
-  depth = 3;
-  enqueue_reference_iteration(c, p, sp, pa, ls_wall, wall, s3, err);
-  CAP(err, "iteration");
-  launch_newton_ctl(c->sctl.p, c->ctrl.p, h_newton, s3);
-  CAP(cudaGetLastError(), "newton body");
-  CAP(cudaStreamEndCapture(s3, &tmp), "end newton body");
-  depth = 2;
-  launch_outer_ctl(c->sctl.p, p.beta_max, h_outer, s2);
-  CAP(cudaGetLastError(), "outer body");
-  CAP(cudaStreamEndCapture(s2, &tmp), "end outer body");
+  if (sp.enable_strain) launch_strain_face(m, c->x.p, sp, c->sflags.p, c->sv.p, c->ctrl.p, s2);
+  launch_gradient(m, c->x.p, c->x_hat.p, c->x_prev.p, c->g_const.p, c->diag_const.p, c->sflags.p, c->sv.p,
+                  c->pin_vertex.p, c->pin_head.p, c->pin_target.p, c->num_pins, c->walls.p, c->contacts.p, c->ents_sorted.p,
+                  c->ebegin.p, c->eend.p, sp, nullptr, c->g.p, c->b.p, c->diag_extra.p, c->ctrl.p, s2);
+  launch_assemble(m, c->sflags.p, c->sv.p, c->diag_extra.p, sp.enable_strain, nullptr, c->val.p, c->precond.p, c->ctrl.p, p.pcg_tol, s2);
+  CAP(launch_pcg(pa, s2), "solve");
+  if (ls_wall) launch_ls_wall(c->V, c->x.p, c->d.p, wall, c->ctrl.p, s2);
+  launch_update_ctl(c->V, c->x.p, c->d.p, c->ctrl.p, c->sctl.p, p.beta_max, h_loop, s2);
+  CAP(cudaGetLastError(), "body");
+  CAP(cudaStreamEndCapture(s2, &tmp), "end body");
   depth = 1;
   double damp = p.velocity_damping > 0.0 ? 1.0 - std::min(std::max(p.velocity_damping, 0.0), 1.0) : 1.0;
   launch_velocity_ctl(c->V, c->x.p, c->x_old.p, p.dt, damp, c->v.p, c->sctl.p, s);
@@ -1754,11 +1719,6 @@ int32_t ando_step(ando_ctx c, const ando_params* params, const ando_pin* pins, i
     rc = restore_start(c);
     if (rc) return rc;
   }
-  {
-    Phase ph(c, ANDO_PHASE_SETUP);
-    launch_predict(c->V, c->x.p, c->v.p, p.dt, c->x_old.p, c->x_hat.p, s);
-    ph.launched();
-  }
   const bool graph_ok = c->use_graphs && !c->prof && p.semantics == ANDO_SEMANTICS_REFERENCE && num_rigids == 0 && c->T != 1 &&
                         p.contact_restitution <= 0.0;
   if (graph_ok) {
@@ -1785,7 +1745,7 @@ int32_t ando_step(ando_ctx c, const ando_params* params, const ando_pin* pins, i
       st.newton_iters = h.newton_iters; st.pcg_iters = h.pcg_iters; st.pcg_max_per_newton = h.pcg_max;
       st.pcg_not_converged = h.pcg_not_converged; st.line_search_fail = h.line_search_fail; st.strain_active = h.strain_active;
       st.beta = h.beta; st.last_alpha = h.last_alpha; st.contacts = 0; st.graph_launched = 1;
-      long long launches = 5 + 2ll * h.inner_steps + (long long)h.iterations_run * kernels_per_iteration(sp, ls_wall);
+      long long launches = 4 + (long long)h.iterations_run * kernels_per_iteration(sp, ls_wall);
       c->profile.launches += launches;
       c->profile.pcg_iterations += h.pcg_iters;
       c->profile.newton_iterations += h.newton_iters;
@@ -1796,6 +1756,11 @@ int32_t ando_step(ando_ctx c, const ando_params* params, const ando_pin* pins, i
       if (stats) *stats = st;
       return ANDO_OK;
     }
+  }
+  {
+    Phase ph(c, ANDO_PHASE_SETUP);
+    launch_predict(c->V, c->x.p, c->v.p, p.dt, c->x_old.p, c->x_hat.p, s);
+    ph.launched();
   }
   if (p.semantics == ANDO_SEMANTICS_CORRECTED) {
     int k = 1;
@@ -1905,7 +1870,7 @@ int32_t ando_eval_system(ando_ctx c, const ando_params* params, const ando_pin* 
   launch_gradient(m, c->x.p, c->x_hat.p, c->x_prev.p, c->g_const.p, c->diag_const.p, c->sflags.p, c->sv.p,
                   c->pin_vertex.p, c->pin_head.p, c->pin_target.p, c->num_pins, c->walls.p, c->contacts.p, c->ents_sorted.p,
                   c->ebegin.p, c->eend.p, sp, sp.semantics ? c->fixed.p : nullptr, c->g.p, c->b.p, c->diag_extra.p, c->ctrl.p, s);
-  launch_assemble(m, c->sflags.p, c->sv.p, c->diag_extra.p, sp.enable_strain, sp.semantics ? c->fixed.p : nullptr, c->val.p, c->precond.p, c->ctrl.p, s);
+  launch_assemble(m, c->sflags.p, c->sv.p, c->diag_extra.p, sp.enable_strain, sp.semantics ? c->fixed.p : nullptr, c->val.p, c->precond.p, c->ctrl.p, -1.0, s);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(s));
   return ANDO_OK;

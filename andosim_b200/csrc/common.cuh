@@ -163,7 +163,8 @@ struct StepCtl {
   double beta, ret, last_alpha;
   int bi, phase, newton_it, max_it;   // phase 0: beta loop, 1: error-reduction pass, 2: done
   int newton_iters, pcg_iters, pcg_max, pcg_not_converged, line_search_fail, strain_active, error;
-  int iterations_run, inner_steps;    // Newton bodies and inner steps executed (launch accounting)
+  int iterations_run;                 // Newton bodies executed (launch accounting)
+  int arrived;                        // blocks of the iteration's last kernel
 };
 
 // Bounded grid barrier with acquire/release atomics: every CTA adds one

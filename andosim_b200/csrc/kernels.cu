@@ -389,8 +389,8 @@ __global__ void __launch_bounds__(256) k_contact_vertex(int V, const ContactRec*
   const bool grad = q >= 9;
   const int r = grad ? q - 9 : q / 3, s = grad ? 0 : q % 3;
   double sum = grad ? g_base[3ll * v + r] : 0.0;
-  const int e = end[v];
-  for (int k = begin[v]; k < e; k += CV_AHEAD) {
+  const int e = end ? end[v] : 0;
+  for (int k = begin ? begin[v] : 0; k < e; k += CV_AHEAD) {
     unsigned id[CV_AHEAD], mask[CV_AHEAD];
     double n_r[CV_AHEAD], n_s[CV_AHEAD], w[CV_AHEAD], d[CV_AHEAD];
     int4 idx[CV_AHEAD];
@@ -427,12 +427,13 @@ __global__ void __launch_bounds__(256) k_contact_vertex(int V, const ContactRec*
 }
 
 // ---------------------------------------------------------- Newton iteration
-__global__ void k_ctrl_reset(Ctrl* c) {
+__device__ inline void ctrl_reset(Ctrl* c) {
   c->gnorm_bits = 0ull; c->ls_mask = (1u << 20) - 1u; c->converged = 0;
   c->pcg_iters = 0; c->pcg_converged = 0; c->pcg_status = PCG_SKIPPED; c->pcg_rel = 0.0;
   c->alpha = 0.0; c->strain_active = 0; c->bar_err = 0; c->bar_arrivals = 0ull;
   c->learned_iters = 0; c->fallback_ran = 0;
 }
+__global__ void k_ctrl_reset(Ctrl* c) { ctrl_reset(c); }
 
 // Thin SVD of the 3x2 deformation gradient through the eigenpairs of F^T F
 // (restates the JacobiSVD call of strain_limiting.cpp:28-50: sigma sorted
@@ -803,10 +804,12 @@ __device__ inline void slot_block(const MeshDev& m, int s, int row, int col, con
 }
 
 __global__ void k_assemble(MeshDev m, const unsigned char* sflags, const StrainSV* sv, const double* diag_extra, int enable_strain,
-                           const unsigned char* fixed, float* val, float* precond, const Ctrl* ctrl) {
-  if (ctrl->converged) return;
+                           const unsigned char* fixed, float* val, float* precond, Ctrl* ctrl, double tol) {
+  // the norm test of the gradient before it; later kernels read the flag
+  const bool converged = __longlong_as_double((long long)ctrl->gnorm_bits) < tol;
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= m.nnzb) return;
+  if (s == 0) ctrl->converged = converged ? 1 : 0;
+  if (converged || s >= m.nnzb) return;
   int row = m.slot_row[s], col = m.cols[s];
   if (fixed && (fixed[row] || fixed[col])) {
     // kinematic pin: decoupled row and column, unit diagonal (diag_extra holds I)
@@ -1349,23 +1352,25 @@ __global__ void k_rigid_coupling(MeshDev m, const ContactDev* cs, StepParams p, 
 }
 
 // ------------------------------------------------------- graph step control
-__global__ void k_ctl_init(StepCtl* c, double beta_max, int max_it, cudaGraphConditionalHandle outer) {
+__global__ void k_ctl_init(StepCtl* c, double beta_max, int max_it, Ctrl* ctrl, cudaGraphConditionalHandle loop) {
   c->beta = 0.0; c->ret = 0.0; c->last_alpha = 0.0;
   c->bi = 0; c->newton_it = 0; c->max_it = max_it;
   c->newton_iters = c->pcg_iters = c->pcg_max = c->pcg_not_converged = c->line_search_fail = c->strain_active = c->error = 0;
-  c->iterations_run = c->inner_steps = 0;
+  c->iterations_run = 0;
+  c->arrived = 0;
   c->phase = (0.0 < beta_max) ? 0 : 2;
-  cudaGraphSetConditional(outer, c->phase != 2 ? 1u : 0u);
+  if (c->phase == 0 && max_it <= 0) {   // an inner step of no iteration: a failed line search
+    c->line_search_fail = 1;
+    c->phase = 2;
+  }
+  ctrl_reset(ctrl);
+  cudaGraphSetConditional(loop, c->phase != 2 ? 1u : 0u);
 }
 
-__global__ void k_inner_begin(StepCtl* c, cudaGraphConditionalHandle newton) {
-  c->newton_it = 0;
-  c->inner_steps++;
-  cudaGraphSetConditional(newton, c->max_it > 0 ? 1u : 0u);
-}
-
-// After one Newton iteration: the decisions of inner_newton_step (integrator.cpp:169-235).
-__global__ void k_newton_ctl(StepCtl* c, const Ctrl* ctrl, cudaGraphConditionalHandle newton) {
+// After one Newton iteration: the decisions of inner_newton_step
+// (integrator.cpp:169-235) and, where they end the inner step, of the beta loop.
+// Returns whether another iteration follows.
+__device__ inline bool next_iteration(StepCtl* c, const Ctrl* ctrl, double alpha, double beta_max) {
   bool stop = false;
   c->iterations_run++;
   c->strain_active = ctrl->strain_active;
@@ -1376,18 +1381,13 @@ __global__ void k_newton_ctl(StepCtl* c, const Ctrl* ctrl, cudaGraphConditionalH
     c->pcg_iters += ctrl->pcg_iters;
     c->pcg_max = max(c->pcg_max, ctrl->pcg_iters);
     if (!ctrl->pcg_converged) c->pcg_not_converged++;
-    c->last_alpha = ctrl->alpha;
-    if (ctrl->alpha < 1e-8) { c->ret = 0.0; stop = true; }
-    else if (ctrl->alpha > 0.99) { c->ret = 1.0; stop = true; }
+    c->last_alpha = alpha;
+    if (alpha < 1e-8) { c->ret = 0.0; stop = true; }
+    else if (alpha > 0.99) { c->ret = 1.0; stop = true; }
     else if (++c->newton_it >= c->max_it) { c->ret = 0.5; stop = true; }
   }
-  cudaGraphSetConditional(newton, stop ? 0u : 1u);
-}
-
-// After one inner Newton step: beta accumulation and the error-reduction pass
-// (integrator.cpp:98-121).
-__global__ void k_outer_ctl(StepCtl* c, double beta_max, cudaGraphConditionalHandle outer) {
-  if (c->error) { c->phase = 2; cudaGraphSetConditional(outer, 0u); return; }
+  if (!stop) return true;
+  if (c->error) { c->phase = 2; return false; }
   if (c->phase == 0) {
     double a = c->ret;
     c->beta = c->beta + (1.0 - c->beta) * a;
@@ -1399,7 +1399,34 @@ __global__ void k_outer_ctl(StepCtl* c, double beta_max, cudaGraphConditionalHan
   } else {
     c->phase = 2;
   }
-  cudaGraphSetConditional(outer, c->phase != 2 ? 1u : 0u);
+  c->newton_it = 0;
+  return c->phase != 2;
+}
+
+// k_update, then (the last block to finish) the step's decisions and the reset of
+// the iteration's control block: launches of one thread each took as long as the
+// kernels they stood between (a frame of a 32 x 32 cloth: 173 us for the step with
+// them, and with two nested graph loops, 140 without).
+__global__ void k_update_ctl(int V, double* x, const float* d, Ctrl* ctrl, StepCtl* c, double beta_max, cudaGraphConditionalHandle loop) {
+  const bool converged = ctrl->converged;
+  const unsigned mask = ctrl->ls_mask;
+  const double a = !converged && mask ? ldexp(1.0, -(__ffs(mask) - 1)) : 0.0;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (!converged && !(a < 1e-8) && i < V) {
+    double s = a * 1.25;
+    x[3 * i] += s * double(d[3 * i]);
+    x[3 * i + 1] += s * double(d[3 * i + 1]);
+    x[3 * i + 2] += s * double(d[3 * i + 2]);
+  }
+  __syncthreads();   // the block has read the control block
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(&c->arrived, 1) != (int)gridDim.x - 1) return;
+  __threadfence();
+  c->arrived = 0;
+  const bool more = next_iteration(c, ctrl, a, beta_max);
+  ctrl_reset(ctrl);
+  cudaGraphSetConditional(loop, more ? 1u : 0u);
 }
 
 __global__ void k_velocity_ctl(int V, const double* x, const double* x_old, double dt, double damp_scale, double* v, const StepCtl* c) {
@@ -1414,15 +1441,11 @@ __global__ void k_velocity_ctl(int V, const double* x, const double* x_old, doub
 
 }  // namespace
 
-void launch_ctl_init(StepCtl* c, double beta_max, int max_it, cudaGraphConditionalHandle outer, cudaStream_t s) {
-  k_ctl_init<<<1, 1, 0, s>>>(c, beta_max, max_it, outer);
+void launch_ctl_init(StepCtl* c, double beta_max, int max_it, Ctrl* ctrl, cudaGraphConditionalHandle loop, cudaStream_t s) {
+  k_ctl_init<<<1, 1, 0, s>>>(c, beta_max, max_it, ctrl, loop);
 }
-void launch_inner_begin(StepCtl* c, cudaGraphConditionalHandle newton, cudaStream_t s) { k_inner_begin<<<1, 1, 0, s>>>(c, newton); }
-void launch_newton_ctl(StepCtl* c, const Ctrl* ctrl, cudaGraphConditionalHandle newton, cudaStream_t s) {
-  k_newton_ctl<<<1, 1, 0, s>>>(c, ctrl, newton);
-}
-void launch_outer_ctl(StepCtl* c, double beta_max, cudaGraphConditionalHandle outer, cudaStream_t s) {
-  k_outer_ctl<<<1, 1, 0, s>>>(c, beta_max, outer);
+void launch_update_ctl(int V, double* x, const float* d, Ctrl* ctrl, StepCtl* c, double beta_max, cudaGraphConditionalHandle loop, cudaStream_t s) {
+  k_update_ctl<<<nblk(V > 0 ? V : 1), TPB, 0, s>>>(V, x, d, ctrl, c, beta_max, loop);
 }
 void launch_velocity_ctl(int V, const double* x, const double* x_old, double dt, double damp_scale, double* v, const StepCtl* c, cudaStream_t s) {
   if (V) k_velocity_ctl<<<nblk(3ll * V), TPB, 0, s>>>(V, x, x_old, dt, damp_scale, v, c);
@@ -1488,8 +1511,8 @@ void launch_gradient(const MeshDev& m, const double* x, const double* x_hat, con
 }
 void launch_check(Ctrl* ctrl, double tol, cudaStream_t s) { k_check<<<1, 1, 0, s>>>(ctrl, tol); }
 void launch_assemble(const MeshDev& m, const unsigned char* sflags, const StrainSV* sv, const double* diag_extra, int enable_strain,
-                     const unsigned char* fixed, float* val, float* precond, const Ctrl* ctrl, cudaStream_t s) {
-  if (m.nnzb) k_assemble<<<nblk(m.nnzb), TPB, 0, s>>>(m, sflags, sv, diag_extra, enable_strain, fixed, val, precond, ctrl);
+                     const unsigned char* fixed, float* val, float* precond, Ctrl* ctrl, double tol, cudaStream_t s) {
+  if (m.nnzb) k_assemble<<<nblk(m.nnzb), TPB, 0, s>>>(m, sflags, sv, diag_extra, enable_strain, fixed, val, precond, ctrl, tol);
 }
 void launch_diag_factor(const MeshDev& m, const unsigned char* sflags, const StrainSV* sv, const double* diag_extra, int enable_strain,
                         const unsigned char* fixed, const double* g, double* Linv, float* Lf, float* bhat, unsigned char* chol_ok,

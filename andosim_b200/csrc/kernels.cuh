@@ -44,7 +44,7 @@ void launch_gradient(const MeshDev& m, const double* x, const double* x_hat, con
 void launch_check(Ctrl* ctrl, double tol, cudaStream_t s);
 void launch_pin_heads(const int* pin_vertex, int num_pins, int* pin_head, cudaStream_t s);
 void launch_assemble(const MeshDev& m, const unsigned char* sflags, const StrainSV* sv, const double* diag_extra, int enable_strain,
-                     const unsigned char* fixed, float* val, float* precond, const Ctrl* ctrl, cudaStream_t s);
+                     const unsigned char* fixed, float* val, float* precond, Ctrl* ctrl, double tol, cudaStream_t s);  // converged: |g| < tol
 // scaled system (CORRECTED): L = chol(A_ii), A^ = L^-1 A L^-T (kernels.cu)
 // tpb: threads per block (a tuning knob; one thread per vertex / slot, so the
 // results do not depend on it)
@@ -89,10 +89,9 @@ void launch_rigid_coupling(const MeshDev& m, const ContactDev* c, int nc, const 
                            const int* offsets, long long units, double dt, cudaStream_t s);
 
 // whole-frame CUDA graph control (kernels.cu)
-void launch_ctl_init(StepCtl* c, double beta_max, int max_it, cudaGraphConditionalHandle outer, cudaStream_t s);
-void launch_inner_begin(StepCtl* c, cudaGraphConditionalHandle newton, cudaStream_t s);
-void launch_newton_ctl(StepCtl* c, const Ctrl* ctrl, cudaGraphConditionalHandle newton, cudaStream_t s);
-void launch_outer_ctl(StepCtl* c, double beta_max, cudaGraphConditionalHandle outer, cudaStream_t s);
+void launch_ctl_init(StepCtl* c, double beta_max, int max_it, Ctrl* ctrl, cudaGraphConditionalHandle loop, cudaStream_t s);
+// launch_update, and whether another Newton iteration of the frame follows (ctrl is reset for it)
+void launch_update_ctl(int V, double* x, const float* d, Ctrl* ctrl, StepCtl* c, double beta_max, cudaGraphConditionalHandle loop, cudaStream_t s);
 void launch_velocity_ctl(int V, const double* x, const double* x_old, double dt, double damp_scale, double* v, const StepCtl* c, cudaStream_t s);
 
 // CORRECTED semantics (corrected.cu)
