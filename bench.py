@@ -670,7 +670,7 @@ def run_ours(args, rank, world, local, pg):
     roof = None
     if pcg_ms > 0:
         achieved = pb / (pcg_ms * 1e-3) / 1e9
-        roof = {"bound": "hbm", "kernel": "k_pcg_scaled (learned and block-Jacobi launches)", "achieved": round(achieved, 1),
+        roof = {"bound": "hbm", "kernel": "k_pcg_res (learned and block-Jacobi launches)", "achieved": round(achieved, 1),
                 "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4), "traffic": PCG_TRAFFIC,
                 "peak_source": source, "bytes_per_launch": int(pb // launches),
                 "launches": int(launches), "avg_launch_us": round(pcg_ms * 1e3 / launches, 2),
