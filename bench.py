@@ -205,7 +205,8 @@ def assembly_bytes(V, nnzb, learned=True):
 
 # DRAM bytes (read + write) per launch of the kernel on this workload, from one ncu capture (the summaries
 # under profiles/ give the command): the PCG's matrix and vectors come from DRAM once per launch and from L2
-# for every later iteration; the assembly's figure is k_diag_factor plus k_assemble_scaled_slice (44.9 + 27.9 MB).
+# for every later iteration (captured on the looping form; the resident form reads the same once per launch and
+# has no capture of its own); the assembly's figure is k_diag_factor plus k_assemble_scaled_slice (44.9 + 27.9 MB).
 PCG_TRAFFIC = 53_985_536
 ASSEMBLY_TRAFFIC = 72_798_720
 
