@@ -151,9 +151,10 @@ struct Ctrl {
   unsigned long long bar_arrivals;  // xr_reduce (and grid_sync_ar): arrivals since the launcher zeroed it
 };
 
+// PCG_NOT_SPD: |p^T A p| < 1e-16, or p^T A p or a residual that is not finite.
 // PCG_PRECOND: the learned preconditioner lost positive definiteness
-// (r^T z <= 0); PCG_STALL: its residual stopped improving. Both hand the
-// solve back to block-Jacobi.
+// (r^T z <= 0); PCG_STALL: its residual stopped improving. All three hand a
+// learned solve back to block-Jacobi.
 enum PcgStatus { PCG_OK = 0, PCG_MAXIT = 1, PCG_NOT_SPD = 2, PCG_TIMEOUT = 3, PCG_SKIPPED = 4, PCG_PRECOND = 5, PCG_STALL = 6 };
 
 // Device-side control of one step (integrator.cpp:98-121 and 152-236) when the
@@ -247,9 +248,10 @@ __device__ inline double xr_warp_sum(double v) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// |v| as bits whose unsigned order is the order of the magnitudes; a NaN
-// counts as 0 (fmax drops it)
-__device__ inline unsigned xr_mag(float v) { return v == v ? __float_as_uint(fabsf(v)) : 0u; }
+// |v| as bits whose unsigned order is the order of the magnitudes, with a NaN
+// above infinity: the maximum of a vector that holds one is not a small residual
+__device__ inline unsigned xr_mag(float v) { return __float_as_uint(fabsf(v)); }
+constexpr unsigned XR_NOT_FINITE = 0x7f800000u;   // xr_mag of infinity; a NaN's is above
 
 // Sum of part[0, n) and max of pmax[0, n) over the calling warp's lanes; the
 // total is lane 0's. (Lanes past n hold zeros, so up to 32 entries need only

@@ -3,7 +3,7 @@
 //
 // Same iteration as the reference: x0 = 0, r = b, block-Jacobi z = P r,
 // stop when |r|_inf / |b|_inf < tol (or |r|_inf when |b|_inf < 1e-16), fail
-// when |p^T A p| < 1e-16. Vectors and the BSR matrix are FP32; every dot
+// when |p^T A p| < 1e-16 or a NaN or infinity appears. Vectors and the BSR matrix are FP32; every dot
 // product and norm is accumulated in FP64 and reduced in a fixed order, so
 // results are bitwise reproducible run to run.
 //
@@ -14,6 +14,7 @@
 // The barriers are bounded (common.cuh): on timeout the kernel reports
 // PCG_TIMEOUT instead of spinning forever.
 #include <algorithm>
+#include <cfloat>
 #include <mutex>
 #include <type_traits>
 #include <utility>
@@ -62,19 +63,21 @@ struct PcgScalars {
     rz = rz0; binf = double(__uint_as_float(mx)); rel = 0.0; iters = 0; since = 0; coef = 0.f; status = PCG_MAXIT;
     if (!ok) { status = PCG_TIMEOUT; return; }
     best = rel = binf < 1e-16 ? binf : 1.0;
-    if (rel < double(tol)) status = PCG_OK;
+    if (mx >= XR_NOT_FINITE) status = PCG_NOT_SPD;
+    else if (rel < double(tol)) status = PCG_OK;
     else if (learned && !(rz > 0.0)) status = PCG_PRECOND;
   }
   __device__ void after_product(bool ok, double pap) {
     if (!ok) { status = PCG_TIMEOUT; return; }
     ++iters;
-    if (fabs(pap) < 1e-16) status = PCG_NOT_SPD;
+    if (!(fabs(pap) >= 1e-16)) status = PCG_NOT_SPD;   // a NaN too
     else coef = float(rz / pap);
   }
   __device__ void after_update(bool ok, double rz_new, unsigned mx, float tol, int stall_window) {
     if (!ok) { status = PCG_TIMEOUT; return; }
     const double rinf = double(__uint_as_float(mx));
     rel = binf < 1e-16 ? rinf : rinf / binf;
+    if (mx >= XR_NOT_FINITE) { status = PCG_NOT_SPD; return; }
     if (rel < double(tol)) { status = PCG_OK; return; }
     if (stall_window > 0) {   // learned preconditioner
       if (!(rz_new > 0.0)) { status = PCG_PRECOND; return; }
@@ -470,8 +473,11 @@ __device__ inline double warp_sum(double v) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
+// the larger of two magnitudes, a NaN above all (fmax would drop it, and a
+// residual that is NaN throughout would count as 0)
+__device__ inline double mag_max(double a, double b) { return b > a || b != b ? b : a; }
 __device__ inline double warp_max(double v) {
-  for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  for (int o = 16; o; o >>= 1) v = mag_max(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
 constexpr int RED_T = 1024;
@@ -484,7 +490,7 @@ __device__ inline void fixed_reduce(const double* part, const double* pm, int n,
     double s = 0.0, m = 0.0;
     for (int k = t; k < n; k += RED_T) {
       s += __ldcg(part + k);  // written by other CTAs before the barrier: read from L2
-      if (MAX) m = fmax(m, __ldcg(pm + k));
+      if (MAX) m = mag_max(m, __ldcg(pm + k));
     }
     sh.s[t] = s;
     if (MAX) sh.m[t] = m;
@@ -634,7 +640,7 @@ __global__ void __launch_bounds__(SCALED_MAX_TPB) k_pcg_scaled(PcgScaledArgs a) 
     double rz_loc = 0.0, binf_loc = 0.0;
     if (i < V) {
       float b0 = a.bhat[3 * i], b1 = a.bhat[3 * i + 1], b2 = a.bhat[3 * i + 2];
-      binf_loc = fmax(fabs(double(b0)), fmax(fabs(double(b1)), fabs(double(b2))));
+      binf_loc = mag_max(fabs(double(b0)), mag_max(fabs(double(b1)), fabs(double(b2))));
       a.xh[3 * i] = 0.0; a.xh[3 * i + 1] = 0.0; a.xh[3 * i + 2] = 0.0;
       st4<S>(r, i, b0, b1, b2);
       if (LEARNED) {
@@ -661,7 +667,8 @@ __global__ void __launch_bounds__(SCALED_MAX_TPB) k_pcg_scaled(PcgScaledArgs a) 
   else fixed_reduce<true>(part_rz, part_rinf, ns, sh, rz, binf);
   if (ok) {
     rel = binf < 1e-16 ? binf : 1.0;
-    if (rel < double(a.tol)) status = PCG_OK;
+    if (!(binf <= FLT_MAX)) status = PCG_NOT_SPD;
+    else if (rel < double(a.tol)) status = PCG_OK;
     else if (LEARNED && !(rz > 0.0)) status = PCG_PRECOND;
   }
   float* pold = a.p0;
@@ -692,7 +699,7 @@ __global__ void __launch_bounds__(SCALED_MAX_TPB) k_pcg_scaled(PcgScaledArgs a) 
     double pap;
     fixed_reduce<false>(part_pap, nullptr, ns, sh, pap, dummy);
     iters = it + 1;
-    if (fabs(pap) < 1e-16) { status = PCG_NOT_SPD; break; }
+    if (!(fabs(pap) >= 1e-16)) { status = PCG_NOT_SPD; break; }   // a NaN too
     float alpha = float(rz / pap);
     // ---- phase B: x^ += alpha p, r -= alpha Ap, z = S r, r^T z, |L r|_inf
     if (!LEARNED) {
@@ -715,7 +722,7 @@ __global__ void __launch_bounds__(SCALED_MAX_TPB) k_pcg_scaled(PcgScaledArgs a) 
             sx[3 * i] = a.xh[3 * i]; sx[3 * i + 1] = a.xh[3 * i + 1]; sx[3 * i + 2] = a.xh[3 * i + 2];
           }
           rz_new_loc = double(r0) * r0 + double(r1) * r1 + double(r2) * r2;
-          rinf_loc = fmax(fabs(double(r0)), fmax(fabs(double(r1)), fabs(double(r2))));
+          rinf_loc = mag_max(fabs(double(r0)), mag_max(fabs(double(r1)), fabs(double(r2))));
         }
         rz_new_loc = warp_sum(rz_new_loc);
         rinf_loc = warp_max(rinf_loc);
@@ -736,7 +743,7 @@ __global__ void __launch_bounds__(SCALED_MAX_TPB) k_pcg_scaled(PcgScaledArgs a) 
           st4<S>(rn, row, r0, r1, r2);
           st4<S>(a.z, row, y0, y1, y2);
           rz_new_loc = double(r0) * y0 + double(r1) * y1 + double(r2) * y2;
-          rinf_loc = fmax(fabs(double(r0)), fmax(fabs(double(r1)), fabs(double(r2))));
+          rinf_loc = mag_max(fabs(double(r0)), mag_max(fabs(double(r1)), fabs(double(r2))));
         }
         rz_new_loc = warp_sum(rz_new_loc);
         rinf_loc = warp_max(rinf_loc);
@@ -749,6 +756,7 @@ __global__ void __launch_bounds__(SCALED_MAX_TPB) k_pcg_scaled(PcgScaledArgs a) 
     fixed_reduce<true>(part_rz, part_rinf, ns, sh, rz_new, rinf);
     rel = binf < 1e-16 ? rinf : rinf / binf;
     if (LEARNED) { float* t = r; r = rn; rn = t; }
+    if (!(rinf <= FLT_MAX)) { status = PCG_NOT_SPD; break; }
     if (rel < double(a.tol)) { status = PCG_OK; break; }
     if (LEARNED) {
       if (!(rz_new > 0.0)) { status = PCG_PRECOND; break; }

@@ -424,7 +424,8 @@ ANDO_API int32_t ando_last_gradient(ando_ctx ctx, double* gradient, int32_t num_
  * reported, and the next call clears the status words. A caller that needs the
  * PCG status passes at least one output; the call then synchronises `stream`
  * and reports iterations, the PCG status (0 converged, 1 max iterations, 2 not
- * SPD, 3 barrier timeout) and the final relative residual. */
+ * SPD or not finite: |p^T A p| < 1e-16, or a NaN or infinity in the system or
+ * the iteration, 3 barrier timeout) and the final relative residual. */
 ANDO_API int32_t ando_pcg_solve_noalloc(int32_t device, void* stream, int32_t num_rows, const int32_t* rowptr,
                                         const int32_t* cols, const float* vals, const float* rhs, float* x, float* work,
                                         int64_t work_floats, double tol, int32_t max_iters, int32_t* iterations,
