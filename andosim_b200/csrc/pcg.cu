@@ -3,9 +3,9 @@
 //
 // Same iteration as the reference: x0 = 0, r = b, block-Jacobi z = P r,
 // stop when |r|_inf / |b|_inf < tol (or |r|_inf when |b|_inf < 1e-16), fail
-// when |p^T A p| < 1e-16 or a NaN or infinity appears. Vectors and the BSR matrix are FP32; every dot
-// product and norm is accumulated in FP64 and reduced in a fixed order, so
-// results are bitwise reproducible run to run.
+// when |p^T A p| < 1e-16 or a NaN or infinity appears. Vectors and the BSR
+// matrix are FP32; every dot product and norm is accumulated in FP64 and reduced
+// in a fixed order, so results are bitwise reproducible run to run.
 //
 // Per iteration there are two barriers over the launch's CTAs:
 //   A: p_new = z + beta p_old (recomputed on the fly for gathered columns),
@@ -43,11 +43,13 @@ namespace {
 //    floats reads without bank conflicts;
 //  - the barrier of each dot product carries the sum (xr_reduce).
 constexpr int PCG_WARPS = 24;                 // 24 x 9.4 KB of shared memory: a slice of 32 rows of 7 blocks each
+// (a launch of up to 20 warps takes the kernel compiled for 20, with 96 registers
+// to a thread in place of 80: 90,000 rows 7.8 us an iteration in place of 8.6)
 // With several slices to a warp the buffers leave room in the L1 for the
 // gathers, and the slices divide evenly: 262,144 rows on 19 warps with 9.1 KB
-// each 20.5 us an iteration, on 24 warps 28.4, on 12 26.9.
+// each 20.5 us an iteration, on 24 warps 28.4, on 12 26.9 (with a row's sum in
+// one part; in eight, 21.8 on 19 warps).
 constexpr int PCG_WARPS_MANY = 20, PCG_BUF_MANY = 9344;
-constexpr int PCG_TPB = 32 * PCG_WARPS;
 constexpr int PCG_CLUSTER_TPB = 512;
 constexpr int PCG_SMEM = 224 * 1024;          // all warps' buffers
 
@@ -121,14 +123,92 @@ __device__ inline int warp_copy_async(void* dst, const void* src, int n) {
   return off;
 }
 
-template <bool ONE>
-__global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
+// The roundings of the unscaled PCG are written out, so that its forms agree:
+// y + a x, and a . b with the middle product rounded first.
+__device__ inline float axpy(float a, float x, float y) { return __fmaf_rn(a, x, y); }
+__device__ inline float dot3(float a0, float a1, float a2, float b0, float b1, float b2) {
+  return __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1)));
+}
+// t += block h times q
+__device__ inline void block_product(const float* h, const float (&q)[3], float (&t)[3]) {
+  for (int c = 0; c < 3; ++c) t[c] = __fadd_rn(t[c], dot3(h[3 * c], h[3 * c + 1], h[3 * c + 2], q[0], q[1], q[2]));
+}
+
+// A row's product is summed in eight parts, block e into part e mod 8, and the
+// parts by halves: ((0 + 4) + (2 + 6)) + ((1 + 5) + (3 + 7)), the sum of a
+// butterfly over eight lanes. One block after the other rounds 15 to 35 % worse
+// (root mean square, against 64 bits), and on systems whose blocks span eleven
+// orders of magnitude (a strain limit met by an irregular mesh) that decides
+// whether a solve takes 8 iterations or none of 1,000 suffices.
+// Blocks of half h in the order of its four parts: 0 4 2 6 and 1 5 3 7.
+__device__ inline int half_block(int h, int u) { return h + (u == 1 ? 4 : u == 2 ? 2 : u == 3 ? 6 : 0); }
+__device__ inline void add_half(const float (&t)[4][3], float (&y)[3]) {
+  for (int c = 0; c < 3; ++c) y[c] += __fadd_rn(__fadd_rn(t[0][c], t[1][c]), __fadd_rn(t[2][c], t[3][c]));
+}
+// One half's blocks among [0, n), B of them gathered at once (4 or 2), added to
+// its parts. col(e): the block's column or its handle.
+template <int B, class Col, class Vec>
+__device__ inline void add_parts(int h, int n, const Col& col, const float* val, const Vec& vec, float (&t)[4][3]) {
+  for (int e0 = h; e0 < n; e0 += 8) {
+#pragma unroll
+    for (int b = 0; b < 4; b += B) {
+      typename Vec::Raw raw[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (half_block(e0, b + u) < n) vec.load(col(half_block(e0, b + u)), raw[u]);
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (half_block(e0, b + u) < n) {
+          float q[3];
+          vec.value(raw[u], q);
+          block_product(val + 9 * half_block(e0, b + u), q, t[b + u]);
+        }
+    }
+  }
+}
+
+// The lane's row in general: its first `held` blocks (8 | held, or all) from the
+// buffer, the others and the extra segment's from memory. One copy of the code
+// for the three: a register spilled is a store that every barrier waits for.
+struct RowAt { int row, k0, n, held; const int* cols; const float* val; };   // cols, val: in the buffer
+template <int B, class Vec>
+__device__ inline void add_row(const PcgArgs& a, const RowAt r, const Vec& vec, float (&y)[3]) {
+  const int xb = a.xbegin && r.row < a.V ? a.xbegin[r.row] : 0, xn = a.xbegin && r.row < a.V ? a.xend[r.row] - xb : 0;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    float t[4][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+#pragma unroll 1
+    for (int s = 0; s < (a.xbegin ? 3 : 2); ++s) {
+      const int* cols = s == 0 ? r.cols : s == 1 ? a.cols + r.k0 + r.held : a.xcols + xb;
+      const float* val = s == 0 ? r.val : s == 1 ? a.val + 9ll * (r.k0 + r.held) : a.xval + 9ll * xb;
+      const int n = s == 0 ? r.held : s == 1 ? r.n - r.held : xn;
+      add_parts<B>(h, n, [&](int e) { return s == 0 ? vec.held(cols[e]) : vec.handle(cols[e]); }, val, vec, t);
+    }
+    add_half(t, y);
+  }
+}
+
+// p_new = z + beta p_old of a column: from the published rows
+template <int S> struct NewP {
+  const float* z; const float* pold; float beta; bool first;
+  struct Raw { float4 z, p; };
+  __device__ int handle(int col) const { return col; }
+  __device__ int held(int c) const { return c; }   // of a column entry in the buffer
+  __device__ void load(int c, Raw& r) const { r.z = ld4<S>(z, c); r.p = first ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4<S>(pold, c); }
+  __device__ void value(const Raw& r, float (&v)[3]) const {
+    v[0] = first ? r.z.x : axpy(beta, r.p.x, r.z.x); v[1] = first ? r.z.y : axpy(beta, r.p.y, r.z.y); v[2] = first ? r.z.z : axpy(beta, r.p.z, r.z.z);
+  }
+};
+
+// ALL: the CTA's rows have all their blocks in the buffers, and none elsewhere.
+template <bool ONE, bool ALL>
+__device__ __forceinline__ void pcg_solve(const PcgArgs& a, XrSmem& sh, PcgScalars& st) {
   Ctrl* ctrl = a.ctrl;
-  if (ctrl->converged) return;
   extern __shared__ __align__(16) unsigned char pcg_dyn[];
-  __shared__ XrSmem sh;
-  __shared__ PcgScalars st;
-  constexpr int S = ONE ? 4 : 3, U = 4;
+  constexpr int S = ONE ? 4 : 3;
+  // P and x of the row too, whose registers the other copy needs: a register
+  // spilled is a store that each barrier waits for (1 to 2 us an iteration)
+  constexpr bool KEEP = ONE && ALL;
   const int V = a.V, ns = (V + 31) >> 5, spc = (ns + (int)gridDim.x - 1) / (int)gridDim.x;
   const int w = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   const int s0 = blockIdx.x * spc, sn = max(0, min(spc, ns - s0));   // slices [s0, s0 + sn)
@@ -144,9 +224,7 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
     for (int e = 0; e < 9; ++e) m[e] = a.P[9ll * row + e];
   };
   auto apply_P = [&](const float (&m)[9], const float (&v)[3], float (&o)[3]) {
-    o[0] = m[0] * v[0] + m[1] * v[1] + m[2] * v[2];
-    o[1] = m[3] * v[0] + m[4] * v[1] + m[5] * v[2];
-    o[2] = m[6] * v[0] + m[7] * v[1] + m[8] * v[2];
+    for (int c = 0; c < 3; ++c) o[c] = dot3(m[3 * c], m[3 * c + 1], m[3 * c + 2], v[0], v[1], v[2]);
   };
   // slice j's partials of the next reduction: the warp's, of all its slices in turn
   auto hand_over = [&](double v, float m0, float m1, float m2) {
@@ -172,8 +250,8 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
       rz_loc = double(b[0]) * zz[0] + double(b[1]) * zz[1] + double(b[2]) * zz[2];
       if (ONE) {
         kb = a.rowptr[row]; cnt = a.rowptr[row + 1] - kb;
-        for (int e = 0; e < 9; ++e) Pm[e] = m[e];
-        for (int e = 0; e < 3; ++e) { r[e] = b[e]; z[e] = zz[e]; x[e] = 0.f; p[e] = 0.f; }
+        if (KEEP) for (int e = 0; e < 9; ++e) Pm[e] = m[e];
+        for (int e = 0; e < 3; ++e) { r[e] = b[e]; z[e] = zz[e]; x[e] = 0.f; p[e] = 0.f; if (!KEEP) a.x[3 * row + e] = 0.f; }
       } else {
         for (int e = 0; e < 3; ++e) { a.x[3 * row + e] = 0.f; a.r[3 * row + e] = b[e]; }
       }
@@ -207,43 +285,31 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
         __syncwarp();
         held = j;
       }
-      float y[3] = {0.f, 0.f, 0.f};
-      const int lo = k0 - hk0, inbuf = max(0, min(n, cap - lo));
+      const int lo = k0 - hk0;
       const int* bc = bcol + co + lo;
+      float y[3] = {0.f, 0.f, 0.f};
+      const NewP<S> vec{a.z, pold, beta, first};
       const float* bv = bval + vo + 9 * lo;
-      auto fma3 = [&](const float* h, const float4& zz, const float4& pp) {
-        const float q0 = first ? zz.x : zz.x + beta * pp.x, q1 = first ? zz.y : zz.y + beta * pp.y, q2 = first ? zz.z : zz.z + beta * pp.z;
-        y[0] += h[0] * q0 + h[1] * q1 + h[2] * q2;
-        y[1] += h[3] * q0 + h[4] * q1 + h[5] * q2;
-        y[2] += h[6] * q0 + h[7] * q1 + h[8] * q2;
-      };
-      for (int e = 0; e < inbuf; e += U) {
-        float4 zz[U], pp[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (e + u < inbuf) {
-            const int c = bc[e + u];
-            zz[u] = ld4<S>(a.z, c);
-            pp[u] = first ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4<S>(pold, c);
-          }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (e + u < inbuf) fma3(bv + 9 * (e + u), zz[u], pp[u]);
+      if constexpr (ALL) {
+#pragma unroll 1
+        for (int h = 0; h < min(n, 2); ++h) {
+          float t[4][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+          add_parts<4>(h, n, [&](int e) { return bc[e]; }, bv, vec, t);
+          add_half(t, y);
+        }
+      } else {
+        const int held = n <= cap - lo ? n : max(0, cap - lo) & ~7;
+        add_row<ONE ? 2 : 4>(a, RowAt{row, k0, n, held, bc, bv}, vec, y);
       }
-      auto outside = [&](int c, const float* h) {
-        fma3(h, ld4<S>(a.z, c), first ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4<S>(pold, c));
-      };
-      for (int e = inbuf; e < n; ++e) outside(a.cols[k0 + e], a.val + 9ll * (k0 + e));
-      if (a.xbegin && row < V)
-        for (int e = a.xbegin[row]; e < a.xend[row]; ++e) outside(a.xcols[e], a.xval + 9ll * e);
       double pap_loc = 0.0;
       if (row < V) {
         float pv[3];
         if (ONE) {
-          for (int e = 0; e < 3; ++e) { pv[e] = p[e] = first ? z[e] : z[e] + beta * p[e]; q[e] = y[e]; }
+          for (int e = 0; e < 3; ++e) { pv[e] = p[e] = first ? z[e] : axpy(beta, p[e], z[e]); q[e] = y[e]; }
         } else {
-          const float4 zz = ld4<S>(a.z, row), pp = first ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4<S>(pold, row);
-          pv[0] = first ? zz.x : zz.x + beta * pp.x; pv[1] = first ? zz.y : zz.y + beta * pp.y; pv[2] = first ? zz.z : zz.z + beta * pp.z;
+          typename NewP<S>::Raw own;
+          vec.load(row, own);
+          vec.value(own, pv);
           for (int e = 0; e < 3; ++e) a.Ap[3 * row + e] = y[e];
         }
         st4<S>(pnew, row, pv[0], pv[1], pv[2]);
@@ -262,7 +328,12 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
       float rv[3] = {0.f, 0.f, 0.f}, zv[3];
       if (row < V) {
         if (ONE) {
-          for (int e = 0; e < 3; ++e) { x[e] += alpha * p[e]; rv[e] = r[e] -= alpha * q[e]; }
+          for (int e = 0; e < 3; ++e) {
+            float& xe = KEEP ? x[e] : a.x[3 * row + e];
+            xe = axpy(alpha, p[e], xe);
+            rv[e] = r[e] = axpy(-alpha, q[e], r[e]);
+          }
+          if (!KEEP) load_P(row, Pm);
           apply_P(Pm, rv, zv);
           for (int e = 0; e < 3; ++e) z[e] = zv[e];
         } else {
@@ -271,8 +342,8 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
           const float4 pp = ld4<S>(pnew, row);
           const float pv[3] = {pp.x, pp.y, pp.z};
           for (int e = 0; e < 3; ++e) {
-            a.x[3 * row + e] += alpha * pv[e];
-            rv[e] = a.r[3 * row + e] -= alpha * a.Ap[3 * row + e];
+            a.x[3 * row + e] = axpy(alpha, pv[e], a.x[3 * row + e]);
+            rv[e] = a.r[3 * row + e] = axpy(-alpha, a.Ap[3 * row + e], a.r[3 * row + e]);
           }
           apply_P(m, rv, zv);
         }
@@ -287,11 +358,31 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
     first = false;
     float* t = pold; pold = pnew; pnew = t;
   }
-  if (ONE) {
+  if (KEEP) {
     const int row = row_of(w);
     if (w < sn && row < V) for (int e = 0; e < 3; ++e) a.x[3 * row + e] = x[e];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) st.report(ctrl);
+}
+
+// At most WARPS to a CTA. Both copies of the loop are inlined: a call in the
+// kernel costs the common one 4 us an iteration.
+template <bool ONE, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 1) k_pcg(const __grid_constant__ PcgArgs a) {
+  if (a.ctrl->converged) return;
+  __shared__ XrSmem sh;
+  __shared__ PcgScalars st;
+  const int ns = (a.V + 31) >> 5, spc = (ns + (int)gridDim.x - 1) / (int)gridDim.x, s0 = blockIdx.x * spc;
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, cap = (((a.smem / nw) & ~15) - 64) / 40;
+  bool rest = false;
+  for (int j = threadIdx.x >> 5; j < min(spc, ns - s0); j += nw) {
+    const int row = 32 * (s0 + j) + lane, first = a.rowptr[32 * (s0 + j)];
+    if (row >= a.V) continue;
+    const int k1 = a.rowptr[row + 1];
+    rest |= k1 - first > cap || (a.xbegin && a.xend[row] > a.xbegin[row]);
+  }
+  if (__syncthreads_or(rest)) pcg_solve<ONE, false>(a, sh, st);
+  else pcg_solve<ONE, true>(a, sh, st);
 }
 
 // The same solve for a small system, as one cluster of at most 16 CTAs with
@@ -301,7 +392,7 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs a) {
 // neighbours' p stay in registers (p_new_j = z_j + beta p_j is what the
 // thread computed for them one iteration ago). 1,024 rows: 34.9 us per
 // iteration with a warp per row and two grid barriers through L2.
-constexpr int PCG_KQ = 8;
+constexpr int PCG_KQ = 8;   // one block in each of a row's eight parts
 
 __device__ inline float4 cl_ld4(unsigned addr) {
   float4 v;
@@ -309,12 +400,23 @@ __device__ inline float4 cl_ld4(unsigned addr) {
   return v;
 }
 
-__global__ void __launch_bounds__(PCG_CLUSTER_TPB, 1) k_pcg_cluster(PcgArgs a) {
-  Ctrl* ctrl = a.ctrl;
-  if (ctrl->converged) return;
+// p_new of a column from the CTA that owns it (handle: the address of its z);
+// in the first iteration p_old is not there yet, and z is read for it with beta 0
+struct ClusterP {
+  unsigned z0; int rows; unsigned pold; float beta;
+  struct Raw { float4 z, p; };
+  __device__ unsigned handle(int col) const { const int c = col / rows; return cl_map(z0 + 16u * (col - c * rows), c); }
+  __device__ unsigned held(int c) const { return (unsigned)c; }
+  __device__ void load(unsigned at, Raw& r) const { r.z = cl_ld4(at); r.p = cl_ld4(at + pold); }
+  __device__ void value(const Raw& r, float (&v)[3]) const {
+    v[0] = axpy(beta, r.p.x, r.z.x); v[1] = axpy(beta, r.p.y, r.z.y); v[2] = axpy(beta, r.p.z, r.z.z);
+  }
+};
+
+// ALL: the CTA's rows have at most PCG_KQ blocks, all in the buffers, and none elsewhere.
+template <bool ALL>
+__device__ __forceinline__ void pcg_solve_cluster(const PcgArgs& a, XrSmem& sh, PcgScalars& st) {
   extern __shared__ __align__(16) unsigned char pcg_dyn[];   // z, p, p' of the CTA's rows (float4), then each warp's matrix buffer
-  __shared__ XrSmem sh;
-  __shared__ PcgScalars st;
   const int V = a.V, rows = blockDim.x, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int row = blockIdx.x * rows + threadIdx.x;
   const bool live = row < V;
@@ -333,20 +435,18 @@ __global__ void __launch_bounds__(PCG_CLUSTER_TPB, 1) k_pcg_cluster(PcgArgs a) {
   const int co = warp_copy_async(bcol, a.cols + k0, min(nb, cap));
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncwarp();
-  const int lo = kb - k0, inbuf = max(0, min(n, cap - lo));
+  const int lo = kb - k0, held = ALL || n <= cap - lo ? n : max(0, cap - lo) & ~7;
   int* const bc = bcol + co + lo;
   const float* const bv = bval + vo + 9 * lo;
-  for (int e = 0; e < inbuf; ++e) bc[e] = (int)handle(bc[e]);   // columns -> addresses of their z
+  for (int e = 0; e < held; ++e) bc[e] = (int)handle(bc[e]);   // columns -> addresses of their z
 
-  float P[9], r[3] = {0.f, 0.f, 0.f}, z[3] = {0.f, 0.f, 0.f}, p[3] = {0.f, 0.f, 0.f}, x[3] = {0.f, 0.f, 0.f}, q[PCG_KQ][3];
+  float P[9], r[3] = {0.f, 0.f, 0.f}, z[3] = {0.f, 0.f, 0.f}, p[3] = {0.f, 0.f, 0.f}, x[3] = {0.f, 0.f, 0.f}, q[ALL ? PCG_KQ : 1][3];
   for (int e = 0; e < 9; ++e) P[e] = live ? a.P[9ll * row + e] : 0.f;
-  for (int e = 0; e < PCG_KQ; ++e) q[e][0] = q[e][1] = q[e][2] = 0.f;
+  for (int e = 0; e < (ALL ? PCG_KQ : 1); ++e) q[e][0] = q[e][1] = q[e][2] = 0.f;
   if (live) for (int e = 0; e < 3; ++e) r[e] = a.b[3 * row + e];
   auto put = [&](unsigned off, const float (&v)[3]) { *reinterpret_cast<float4*>(pcg_dyn + off + 16 * threadIdx.x) = make_float4(v[0], v[1], v[2], 0.f); };
   auto apply_P = [&]() {
-    z[0] = P[0] * r[0] + P[1] * r[1] + P[2] * r[2];
-    z[1] = P[3] * r[0] + P[4] * r[1] + P[5] * r[2];
-    z[2] = P[6] * r[0] + P[7] * r[1] + P[8] * r[2];
+    for (int c = 0; c < 3; ++c) z[c] = dot3(P[3 * c], P[3 * c + 1], P[3 * c + 2], r[0], r[1], r[2]);
     put(0, z);
     return double(r[0]) * z[0] + double(r[1]) * z[1] + double(r[2]) * z[2];
   };
@@ -364,36 +464,34 @@ __global__ void __launch_bounds__(PCG_CLUSTER_TPB, 1) k_pcg_cluster(PcgArgs a) {
   for (int it = 0; st.status == PCG_MAXIT && it < a.max_iters; ++it) {
     // ---- phase A: p_new = z + beta p_old, Ap = A p_new, p^T Ap
     float y[3] = {0.f, 0.f, 0.f};
-    auto fma3 = [&](const float* h, float q0, float q1, float q2) {
-      y[0] += h[0] * q0 + h[1] * q1 + h[2] * q2;
-      y[1] += h[3] * q0 + h[4] * q1 + h[5] * q2;
-      y[2] += h[6] * q0 + h[7] * q1 + h[8] * q2;
-    };
-    float4 zz[PCG_KQ];
+    if constexpr (ALL) {
+      float4 zz[PCG_KQ];
 #pragma unroll
-    for (int e = 0; e < PCG_KQ; ++e) if (e < inbuf) zz[e] = cl_ld4((unsigned)bc[e]);
+      for (int e = 0; e < PCG_KQ; ++e) if (e < n) zz[e] = cl_ld4((unsigned)bc[e]);
 #pragma unroll
-    for (int e = 0; e < PCG_KQ; ++e)
-      if (e < inbuf) {
-        q[e][0] = zz[e].x + beta * q[e][0]; q[e][1] = zz[e].y + beta * q[e][1]; q[e][2] = zz[e].z + beta * q[e][2];
-        fma3(bv + 9 * e, q[e][0], q[e][1], q[e][2]);
+      for (int h = 0; h < 2; ++h) {
+        float t[4][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int e = half_block(h, u);
+          if (e < n) {
+            q[e][0] = axpy(beta, q[e][0], zz[e].x); q[e][1] = axpy(beta, q[e][1], zz[e].y); q[e][2] = axpy(beta, q[e][2], zz[e].z);
+            block_product(bv + 9 * e, q[e], t[u]);
+          }
+        }
+        add_half(t, y);
       }
-    auto far = [&](unsigned at, const float* h) {
-      const float4 zf = cl_ld4(at), pf = it ? cl_ld4(at + pold) : make_float4(0.f, 0.f, 0.f, 0.f);
-      fma3(h, zf.x + beta * pf.x, zf.y + beta * pf.y, zf.z + beta * pf.z);
-    };
-    for (int e = PCG_KQ; e < inbuf; ++e) far((unsigned)bc[e], bv + 9 * e);
-    for (int e = inbuf; e < n; ++e) far(handle(a.cols[kb + e]), a.val + 9ll * (kb + e));
-    if (a.xbegin && live)
-      for (int e = a.xbegin[row]; e < a.xend[row]; ++e) far(handle(a.xcols[e]), a.xval + 9ll * e);
-    for (int e = 0; e < 3; ++e) p[e] = z[e] + beta * p[e];
+    } else {
+      add_row<4>(a, RowAt{row, kb, n, held, bc, bv}, ClusterP{pub0, rows, it ? pold : 0u, it ? beta : 0.f}, y);
+    }
+    for (int e = 0; e < 3; ++e) p[e] = axpy(beta, p[e], z[e]);
     put(pnew, p);
     reduce(2 + 2 * it, double(p[0]) * y[0] + double(p[1]) * y[1] + double(p[2]) * y[2], 0u,
            [&](bool ok, double pap, unsigned) { st.after_product(ok, pap); });
     if (st.status != PCG_MAXIT) break;
     const float alpha = st.coef;
     // ---- phase B: x, r, z, r^T z, |r|_inf
-    for (int e = 0; e < 3; ++e) { x[e] += alpha * p[e]; r[e] -= alpha * y[e]; }
+    for (int e = 0; e < 3; ++e) { x[e] = axpy(alpha, p[e], x[e]); r[e] = axpy(-alpha, y[e], r[e]); }
     rz0 = apply_P();
     reduce(3 + 2 * it, rz0, mag(), [&](bool ok, double rz, unsigned mx) { st.after_update(ok, rz, mx, a.tol, 0); });
     if (st.status != PCG_MAXIT) break;
@@ -401,8 +499,23 @@ __global__ void __launch_bounds__(PCG_CLUSTER_TPB, 1) k_pcg_cluster(PcgArgs a) {
     const unsigned t = pold; pold = pnew; pnew = t;
   }
   if (live) for (int e = 0; e < 3; ++e) a.x[3 * row + e] = x[e];
-  if (row == 0) st.report(ctrl);
+  if (row == 0) st.report(a.ctrl);
   cl_sync_shared();   // the others have read this CTA's last partial
+}
+
+__global__ void __launch_bounds__(PCG_CLUSTER_TPB, 1) k_pcg_cluster(const __grid_constant__ PcgArgs a) {
+  if (a.ctrl->converged) return;
+  __shared__ XrSmem sh;
+  __shared__ PcgScalars st;
+  const int rows = blockDim.x, nw = rows >> 5, cap = ((((a.smem - 48 * rows) / nw) & ~15) - 64) / 40;
+  const int row = blockIdx.x * rows + threadIdx.x;
+  bool rest = false;
+  if (row < a.V) {
+    const int k0 = a.rowptr[row], k1 = a.rowptr[row + 1];
+    rest = k1 - k0 > PCG_KQ || k1 - a.rowptr[row & ~31] > cap || (a.xbegin && a.xend[row] > a.xbegin[row]);
+  }
+  if (__syncthreads_or(rest)) pcg_solve_cluster<false>(a, sh, st);
+  else pcg_solve_cluster<true>(a, sh, st);
 }
 
 // ------------------------------------------------------------ scaled PCG
@@ -1079,7 +1192,10 @@ size_t pcg_scaled_partials(int V) { return 3ull * (size_t)((V + 31) / 32 + 1); }
 
 namespace {
 using PcgKernel = void (*)(PcgArgs);
-PcgKernel pcg_kernel(bool one) { return one ? k_pcg<true> : k_pcg<false>; }
+PcgKernel pcg_kernel(bool one, int warps) {
+  if (!one) return k_pcg<false, PCG_WARPS_MANY>;
+  return warps <= PCG_WARPS_MANY ? k_pcg<true, PCG_WARPS_MANY> : k_pcg<true, PCG_WARPS>;
+}
 
 // Resident kernel of a shape: threads per CTA rounded up to a compiled bound,
 // and with it the registers, which decide how many neighbours' p are kept
@@ -1303,7 +1419,7 @@ cudaError_t launch_pcg(const PcgArgs& args, cudaStream_t s) {
   const int each = one ? 1 : (spc + PCG_WARPS_MANY - 1) / PCG_WARPS_MANY, nw = (spc + each - 1) / each;
   a.smem = nw * std::min(PCG_SMEM / nw, one ? 24 * 1024 : PCG_BUF_MANY);
   void* p[] = {(void*)&a};
-  return launch_ctas((const void*)pcg_kernel(one), false, grid, 32 * nw, a.smem, PCG_SMEM, p, s);
+  return launch_ctas((const void*)pcg_kernel(one, nw), false, grid, 32 * nw, a.smem, PCG_SMEM, p, s);
 }
 
 }  // namespace ando
