@@ -167,6 +167,37 @@ __device__ inline void add_parts(int h, int n, const Col& col, const float* val,
   }
 }
 
+// Rows of more than PCG_WIDE blocks are summed by their warp, one row after
+// another with a block to each lane. By its thread alone a row of 900 blocks took
+// 220 us an iteration and one of 8,000 2.4 ms (15 and 60 so), and rows of 81
+// throughout 569 us at 90,000 rows (110 so), which their threads read from memory
+// in pieces. Rows of 27 throughout are the faster by thread, 38 us against 65
+// with a warp to a row at 8,100 rows; of 41, 103 against 50.
+constexpr int PCG_WIDE = 32;
+
+// y += the row of n blocks from k0 on, for the lanes whose n is above PCG_WIDE. Called by the whole warp.
+template <class Vec>
+__device__ inline void add_wide(int k0, int n, const int* cols, const float* val, const Vec& vec, float (&y)[3]) {
+  const int lane = threadIdx.x & 31;
+  for (unsigned left = __ballot_sync(0xffffffffu, n > PCG_WIDE); left; left &= left - 1) {
+    const int src = __ffs(left) - 1;
+    const int first = __shfl_sync(0xffffffffu, k0, src), last = first + __shfl_sync(0xffffffffu, n, src);
+    float t[3] = {0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int k = first + lane; k < last; k += 32) {
+      typename Vec::Raw raw;
+      float q[3];
+      vec.load(vec.handle(cols[k]), raw);
+      vec.value(raw, q);
+      block_product(val + 9ll * k, q, t);
+    }
+    for (int c = 0; c < 3; ++c) {
+      for (int o = 16; o; o >>= 1) t[c] += __shfl_xor_sync(0xffffffffu, t[c], o);
+      if (lane == src) y[c] += t[c];
+    }
+  }
+}
+
 // The lane's row in general: its first `held` blocks (8 | held, or all) from the
 // buffer, the others and the extra segment's from memory. One copy of the code
 // for the three: a register spilled is a store that every barrier waits for.
@@ -181,11 +212,12 @@ __device__ inline void add_row(const PcgArgs& a, const RowAt r, const Vec& vec, 
     for (int s = 0; s < (a.xbegin ? 3 : 2); ++s) {
       const int* cols = s == 0 ? r.cols : s == 1 ? a.cols + r.k0 + r.held : a.xcols + xb;
       const float* val = s == 0 ? r.val : s == 1 ? a.val + 9ll * (r.k0 + r.held) : a.xval + 9ll * xb;
-      const int n = s == 0 ? r.held : s == 1 ? r.n - r.held : xn;
+      const int n = s == 0 ? r.held : s == 1 ? (r.n > PCG_WIDE ? 0 : r.n - r.held) : xn;
       add_parts<B>(h, n, [&](int e) { return s == 0 ? vec.held(cols[e]) : vec.handle(cols[e]); }, val, vec, t);
     }
     add_half(t, y);
   }
+  if (__any_sync(0xffffffffu, r.n > PCG_WIDE)) add_wide(r.k0, r.n, a.cols, a.val, vec, y);
 }
 
 // p_new = z + beta p_old of a column: from the published rows
@@ -298,7 +330,7 @@ __device__ __forceinline__ void pcg_solve(const PcgArgs& a, XrSmem& sh, PcgScala
           add_half(t, y);
         }
       } else {
-        const int held = n <= cap - lo ? n : max(0, cap - lo) & ~7;
+        const int held = n > PCG_WIDE ? 0 : n <= cap - lo ? n : max(0, cap - lo) & ~7;
         add_row<ONE ? 2 : 4>(a, RowAt{row, k0, n, held, bc, bv}, vec, y);
       }
       double pap_loc = 0.0;
@@ -378,8 +410,8 @@ __global__ void __launch_bounds__(32 * WARPS, 1) k_pcg(const __grid_constant__ P
   for (int j = threadIdx.x >> 5; j < min(spc, ns - s0); j += nw) {
     const int row = 32 * (s0 + j) + lane, first = a.rowptr[32 * (s0 + j)];
     if (row >= a.V) continue;
-    const int k1 = a.rowptr[row + 1];
-    rest |= k1 - first > cap || (a.xbegin && a.xend[row] > a.xbegin[row]);
+    const int k0 = a.rowptr[row], k1 = a.rowptr[row + 1];
+    rest |= k1 - k0 > PCG_WIDE || k1 - first > cap || (a.xbegin && a.xend[row] > a.xbegin[row]);
   }
   if (__syncthreads_or(rest)) pcg_solve<ONE, false>(a, sh, st);
   else pcg_solve<ONE, true>(a, sh, st);
@@ -435,7 +467,7 @@ __device__ __forceinline__ void pcg_solve_cluster(const PcgArgs& a, XrSmem& sh, 
   const int co = warp_copy_async(bcol, a.cols + k0, min(nb, cap));
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncwarp();
-  const int lo = kb - k0, held = ALL || n <= cap - lo ? n : max(0, cap - lo) & ~7;
+  const int lo = kb - k0, held = ALL || n <= min(PCG_WIDE, cap - lo) ? n : n > PCG_WIDE ? 0 : max(0, cap - lo) & ~7;
   int* const bc = bcol + co + lo;
   const float* const bv = bval + vo + 9 * lo;
   for (int e = 0; e < held; ++e) bc[e] = (int)handle(bc[e]);   // columns -> addresses of their z
