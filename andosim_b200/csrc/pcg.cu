@@ -20,6 +20,7 @@
 #include <utility>
 #include <vector>
 
+#include "copy_pieces.cuh"
 #include "kernels.cuh"
 
 namespace ando {
@@ -109,17 +110,20 @@ template <int S> __device__ inline void st4(float* v, int j, float a, float b, f
 }
 
 // Asynchronous copy of n 4-byte elements from src into 16-byte aligned shared
-// memory, by the calling warp, in whole 16-byte pieces of global memory (a
-// piece holds at least one of the elements, so it is readable). Returns the
-// element offset of src[0] in dst.
+// memory, by the calling warp, in whole 16-byte pieces of global memory and the
+// elements beside them one by one (the array may be a caller's, and its
+// neighbours another's). Returns the element offset of src[0] in dst.
 __device__ inline int warp_copy_async(void* dst, const void* src, int n) {
-  const size_t a = reinterpret_cast<size_t>(src);
-  const int off = int(a & 15) >> 2;
-  const char* g = reinterpret_cast<const char*>(a & ~size_t(15));
+  const int off = int(reinterpret_cast<size_t>(src) & 15) >> 2;
+  const char* g = reinterpret_cast<const char*>(src) - 4 * off;
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int pieces = (off + n + 3) >> 2;
-  for (int q = threadIdx.x & 31; q < pieces; q += 32)
+  const CopyPieces p = copy_pieces(off, n);
+  const int lane = threadIdx.x & 31;
+  for (int q = p.q0 + lane; q < p.q1; q += 32)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16u * q), "l"(g + 16ll * q) : "memory");
+  const int e = off + (lane < 4 ? lane : n - p.tail + lane - 4);   // lanes 0 to 2: the head, 4 to 6: the tail
+  if (lane < 4 ? lane < p.head : lane - 4 < p.tail)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4u * e), "l"(g + 4ll * e) : "memory");
   return off;
 }
 
