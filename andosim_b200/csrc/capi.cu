@@ -94,10 +94,11 @@ struct ando_ctx_s {
   DevBuf<unsigned char> chol_ok;
   DevBuf<double> spart;            // per-slice partials of the scaled PCG
   double tune_ms = 0.0;            // device time spent timing launch shapes
-  // launch shape of the scaled PCG per preconditioner kind (0 Jacobi, 1 learned):
-  // autotuned on the first solve of a mesh (choice < 0) or a fixed candidate
-  PcgShape shape[2];
-  int shape_V[2] = {-1, -1}, shape_choice[2] = {-1, -1};
+  // launch shape of the scaled PCG per preconditioner kind (0 Jacobi, 1 learned),
+  // without and with contact blocks: autotuned on the first solve of a mesh
+  // (choice < 0) or a fixed candidate; the one last used is what is reported
+  PcgShape shape[2][2];
+  int shape_V[2][2] = {{-1, -1}, {-1, -1}}, shape_last[2] = {0, 0}, shape_choice[2] = {-1, -1};
   PcgShape shape_untuned;          // block-Jacobi fallback launch before its shape has been tuned
   int asm_tpb = 256, asm_V = -1, asm_choice = -1;  // scaled assembly block size (tuned like the PCG shape)
   double dt2inv = 0.0;             // of the last assembled system
@@ -934,28 +935,43 @@ int ensure_learned(ando_ctx c) {
   return ANDO_OK;
 }
 
-// Launch shape of the scaled PCG for the current mesh. On the first solve
-// of a mesh (autotune on) every candidate runs the solve at hand once more,
-// timed with CUDA events after one untimed round, and the fastest is kept.
+// Whether the launch of the current system differs from the contact-free one:
+// the looping form's does not.
+int shape_kind(ando_ctx c) { return c->nx && pcg_resident(c->V) ? 1 : 0; }
+
+int shape_candidates(ando_ctx c, bool learned, int kind, PcgShape (&cand)[16], bool* same) {
+  return pcg_scaled_shapes(c->device, c->V, c->sell_wmax, kind != 0, learned, cand, 16, same);
+}
+
+// Launch shape of the scaled PCG for the current mesh. On the first solve of a
+// mesh, and on its first with contact blocks (autotune on), every candidate runs
+// the solve at hand once more, timed with CUDA events after one untimed round,
+// and the fastest is kept; candidates that are one launch are not compared. (With
+// one choice for both, a mesh that started without contacts kept the first, the
+// second or the third by chance: 9.1, 11.1 or 12.9 us an iteration on two sheets
+// of 100^2 in contact.)
 // The solve is a pure function of its inputs and every shape gives the same
 // bits, so the solves run for timing leave exactly the state one solve leaves.
 const PcgShape& pcg_shape(ando_ctx c, bool learned, const PcgScaledArgs& sa) {
-  const int k = learned ? 1 : 0;
-  if (c->shape_V[k] == c->V) return c->shape[k];
+  const int k = learned ? 1 : 0, kind = shape_kind(c);
+  PcgShape& shape = c->shape[k][kind];
+  c->shape_last[k] = kind;
+  if (c->shape_V[k][kind] == c->V) return shape;
   PcgShape cand[16];
-  int n = pcg_scaled_shapes(c->device, c->V, learned, cand, 16);
-  c->shape[k] = n > 0 ? cand[0] : PcgShape{32, 1, 1};
-  c->shape_V[k] = c->V;
+  bool same = false;
+  int n = shape_candidates(c, learned, kind, cand, &same);
+  shape = n > 0 ? cand[0] : PcgShape{32, 1, 1};
+  c->shape_V[k][kind] = c->V;
   if (c->shape_choice[k] >= 0) {
-    if (c->shape_choice[k] < n) c->shape[k] = cand[c->shape_choice[k]];
-    return c->shape[k];
+    if (c->shape_choice[k] < n) shape = cand[c->shape_choice[k]];
+    return shape;
   }
-  if (n < 2) return c->shape[k];
+  if (n < 2) return shape;
   cudaEvent_t e0, e1;
-  if (cudaEventCreate(&e0) != cudaSuccess) return c->shape[k];
-  if (cudaEventCreate(&e1) != cudaSuccess) { cudaEventDestroy(e0); return c->shape[k]; }
+  if (cudaEventCreate(&e0) != cudaSuccess) return shape;
+  if (cudaEventCreate(&e1) != cudaSuccess) { cudaEventDestroy(e0); return shape; }
   float best = 1e30f;
-  for (int rep = 0; rep < 2; ++rep) {
+  for (int rep = 0; rep < (same ? 1 : 2); ++rep) {
     for (int i = 0; i < n; ++i) {
       if (rep == 0 && i > 0) break;  // one untimed solve warms the caches
       cudaEventRecord(e0, c->stream);
@@ -967,22 +983,23 @@ const PcgShape& pcg_shape(ando_ctx c, bool learned, const PcgScaledArgs& sa) {
         continue;
       }
       c->tune_ms += ms;
-      if (rep == 1 && ms < best) { best = ms; c->shape[k] = cand[i]; }
+      if (rep == 1 && ms < best) { best = ms; shape = cand[i]; }
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  return c->shape[k];
+  return shape;
 }
 
 // Shape of a launch that must not run the autotuner (its timing solves would
 // overwrite the solution of the solve before it): the tuned shape when there
 // is one, else the caller's choice or the first candidate.
 const PcgShape& pcg_shape_no_tuning(ando_ctx c, bool learned) {
-  const int k = learned ? 1 : 0;
-  if (c->shape_V[k] == c->V) return c->shape[k];
+  const int k = learned ? 1 : 0, kind = shape_kind(c);
+  if (c->shape_V[k][kind] == c->V) return c->shape[k][kind];
   PcgShape cand[16];
-  const int n = pcg_scaled_shapes(c->device, c->V, learned, cand, 16);
+  bool same = false;
+  const int n = shape_candidates(c, learned, kind, cand, &same);
   const int pick = c->shape_choice[k] >= 0 && c->shape_choice[k] < n ? c->shape_choice[k] : 0;
   c->shape_untuned = n > 0 ? cand[pick] : PcgShape{32, 1, 1};
   return c->shape_untuned;
@@ -1516,7 +1533,8 @@ int32_t ando_mesh_upload(ando_ctx c, const double* vertices, int32_t V, const in
   }
   cudaStream_t s = c->stream;
   c->V = V; c->T = T; c->nnzb = nnzb;
-  c->shape_V[0] = c->shape_V[1] = -1;
+  for (auto& kinds : c->shape_V) kinds[0] = kinds[1] = -1;
+  c->shape_last[0] = c->shape_last[1] = 0;
   c->asm_V = -1;
   CK(c->spart.reserve(pcg_scaled_partials(V)));
   c->S_ready = false;
@@ -2121,7 +2139,7 @@ int32_t ando_ctx_select_pcg_shape(ando_ctx c, int32_t learned, int32_t index) {
   if (rc) return rc;
   if (learned < 0 || learned > 1 || index < -1) return fail(ANDO_ERR_INVALID, "shape arguments");
   c->shape_choice[learned] = index;
-  c->shape_V[learned] = -1;
+  c->shape_V[learned][0] = c->shape_V[learned][1] = -1;
   return ANDO_OK;
 }
 
@@ -2129,15 +2147,18 @@ int32_t ando_ctx_pcg_shape(ando_ctx c, int32_t learned, int32_t* count, int32_t*
   int rc = check_ctx(c);
   if (rc) return rc;
   if (learned < 0 || learned > 1) return fail(ANDO_ERR_INVALID, "shape arguments");
+  const int kind = c->shape_last[learned];
   if (count) {
     PcgShape cand[16];
-    *count = c->mesh_ready ? pcg_scaled_shapes(c->device, c->V, learned != 0, cand, 16) : 0;
+    bool same = false;
+    *count = c->mesh_ready ? shape_candidates(c, learned != 0, kind, cand, &same) : 0;
   }
   if (shape) {
-    const bool set = c->mesh_ready && c->shape_V[learned] == c->V;
-    shape[0] = set ? c->shape[learned].tpb : 0;
-    shape[1] = set ? c->shape[learned].grid : 0;
-    shape[2] = set ? c->shape[learned].unroll : 0;
+    const bool set = c->mesh_ready && c->shape_V[learned][kind] == c->V;
+    const PcgShape& sh = c->shape[learned][kind];
+    shape[0] = set ? sh.tpb : 0;
+    shape[1] = set ? sh.grid : 0;
+    shape[2] = set ? sh.unroll : 0;
   }
   if (tune_ms) *tune_ms = c->tune_ms;
   return ANDO_OK;

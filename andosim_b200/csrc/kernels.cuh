@@ -166,7 +166,7 @@ struct PcgShape { int tpb = 0, grid = 0, unroll = 1; };
 size_t pcg_scaled_partials(int V);
 bool pcg_resident(int V);   // the scaled PCG of V rows runs in its resident form (reads xs_*)
 constexpr int PCG_NEAR_SLOTS = 7;   // static slots of a row whose neighbours' p the resident form keeps itself
-int pcg_scaled_shapes(int device, int V, bool learned, PcgShape* out, int max);
+int pcg_scaled_shapes(int device, int V, int wmax, bool contact, bool learned, PcgShape* out, int max, bool* same);
 cudaError_t launch_pcg_scaled(const PcgScaledArgs& a, bool learned, const PcgShape& sh, cudaStream_t s);
 cudaError_t launch_pcg(const PcgArgs& a, cudaStream_t s);
 

@@ -1388,19 +1388,38 @@ bool pcg_resident(int V) {
   return res_layout(V, true, cluster, ctas, spc) && res_layout(V, false, cluster, ctas, spc);
 }
 
-// Candidate launch shapes of the scaled PCG for V rows on `device`; shape 0
-// is the default. Every shape gives the same result bits. The resident form's
-// CTAs and warps follow from V and whether there are contact blocks; its
-// candidates are the shared memory (KiB) for the blocks of a system that does
-// not fit whole: all of it, or less, which leaves more to the L1 for the
-// gathers.
-int pcg_scaled_shapes(int device, int V, bool learned, PcgShape* out, int max) {
-  bool cluster; int ctas, spc;
+namespace {
+// The resident launch of a system. far: contact blocks, rows of more than RES_KQ
+// slots, or blocks that do not all fit on the chip.
+struct ResPlan { ResKernel k; bool far, cluster; int ctas, spc, pub, near; };
+ResPlan res_plan(int V, int wmax, bool contact, bool learned) {
+  ResPlan p{};
+  p.far = contact || wmax > RES_KQ;
+  while (true) {
+    res_layout(V, p.far, p.cluster, p.ctas, p.spc);
+    p.k = res_kernel(learned, p.far, p.cluster, 32 * p.spc);
+    p.near = std::max(wmax - (p.k.compact ? 1 : 0), 1);
+    p.pub = p.cluster ? 16 * 32 * p.spc * res_vectors(learned, p.far, p.k.kq) : 0;
+    if (p.far || p.pub + p.spc * res_warp_bytes(p.near) <= RES_SMEM) return p;
+    p.far = true;
+  }
+}
+}  // namespace
+
+// Candidate launch shapes of the scaled PCG for V rows of at most wmax slots,
+// with or without contact blocks, on `device`; shape 0 is the default. Every
+// shape gives the same result bits. The resident form's CTAs and warps follow
+// from those three; its candidates are the shared memory (KiB) for the blocks of
+// a system that does not fit whole: all of it, or less, which leaves more to the
+// L1 for the gathers. *same: the system fits, and they are one launch.
+int pcg_scaled_shapes(int device, int V, int wmax, bool contact, bool learned, PcgShape* out, int max, bool* same) {
+  *same = false;
   if (!pcg_resident(V)) return streamed_shapes(device, V, learned, out, max);
-  res_layout(V, false, cluster, ctas, spc);
+  const ResPlan p = res_plan(V, wmax, contact, learned);
+  *same = !p.far;
   int n = 0;
   for (int kb : {RES_SMEM / 1024, 160, 96})
-    if (n < max) out[n++] = PcgShape{32 * spc, ctas, kb};
+    if (n < max) out[n++] = PcgShape{32 * p.spc, p.ctas, kb};
   return n;
 }
 
@@ -1411,22 +1430,11 @@ cudaError_t launch_pcg_scaled(const PcgScaledArgs& args, bool learned, const Pcg
   PcgScaledArgs a = args;
   void* p[] = {(void*)&a};
   if (!pcg_resident(a.V)) return cudaLaunchCooperativeKernel((void*)scaled_kernel(learned, sh.unroll), dim3(sh.grid), dim3(sh.tpb), p, 0, s);
-  bool cluster, far = a.xbegin || a.wmax > RES_KQ;
-  int ctas, spc, pub = 0;
-  ResKernel k;
-  int near = 0;
-  while (true) {   // a mesh without contact blocks keeps all its blocks on chip, or is treated as one with
-    res_layout(a.V, far, cluster, ctas, spc);
-    k = res_kernel(learned, far, cluster, 32 * spc);
-    near = std::max(a.wmax - (k.compact ? 1 : 0), 1);
-    pub = cluster ? 16 * 32 * spc * res_vectors(learned, far, k.kq) : 0;
-    if (far || pub + spc * res_warp_bytes(near) <= RES_SMEM) break;
-    far = true;
-  }
-  const int room = std::max(std::min(sh.unroll * 1024, RES_SMEM) - pub - 128 * spc, 0);
-  a.slots = far ? std::min(room / (1280 * spc), 64) : near;
-  const int smem = pub + spc * res_warp_bytes(a.slots);
-  return launch_ctas(k.f, cluster, ctas, 32 * spc, smem, RES_SMEM, p, s);
+  const ResPlan q = res_plan(a.V, a.wmax, a.xbegin != nullptr, learned);
+  const int room = std::max(std::min(sh.unroll * 1024, RES_SMEM) - q.pub - 128 * q.spc, 0);
+  a.slots = q.far ? std::min(room / (1280 * q.spc), 64) : q.near;
+  const int smem = q.pub + q.spc * res_warp_bytes(a.slots);
+  return launch_ctas(q.k.f, q.cluster, q.ctas, 32 * q.spc, smem, RES_SMEM, p, s);
 }
 
 bool pcg_packed_rows(int V) {

@@ -346,14 +346,18 @@ ANDO_API int32_t ando_step_batch(ando_batch_item* items, int32_t count, int32_t 
 
 /* Launch shape of the scaled PCG (CORRECTED semantics) for the current mesh,
  * per preconditioner (learned = 0: block Jacobi, 1: learned). The candidates
- * (threads per CTA, CTAs, column slots loaded ahead) all give the same result
- * bits. By default (index -1) the first solve of a mesh times every candidate
- * and keeps the fastest; index >= 0 fixes candidate `index`. No reference
+ * all give the same result bits. Up to 151,552 rows they differ in the shared
+ * memory for the system's blocks, which matters when those do not fit whole
+ * (contact blocks, wide rows); above in threads per CTA, CTAs and column slots
+ * loaded ahead. By default (index -1) the first solve of a mesh, and its first
+ * with contact blocks, times every candidate that is a launch of its own and
+ * keeps the fastest; index >= 0 fixes candidate `index`. No reference
  * counterpart (the reference solves on the CPU). */
 ANDO_API int32_t ando_ctx_select_pcg_shape(ando_ctx ctx, int32_t learned, int32_t index);
-/* Number of candidates for the current mesh and the shape in use
- * (shape[0..2] = threads per CTA, CTAs, slots ahead; zeros before the first
- * solve of the mesh). `tune_ms` (may be null): device time spent timing. */
+/* Number of candidates for the current mesh and the shape of the last solve
+ * (shape[0..2] = threads per CTA, CTAs, KiB of shared memory for blocks or
+ * slots ahead; zeros before the first solve of the mesh). `tune_ms` (may be
+ * null): device time spent timing. */
 ANDO_API int32_t ando_ctx_pcg_shape(ando_ctx ctx, int32_t learned, int32_t* count, int32_t* shape, double* tune_ms);
 
 /* Capacity, in candidate pairs, of the context's broad-phase candidate
