@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from andosim_b200 import learned, scenes
+from test_gpu_pcg_forms import EPS, matvec, solve_step
 
 pytestmark = pytest.mark.gpu
 CLOSE = 0.0008        # metres between the curtains: below the activation distance everywhere
@@ -49,3 +50,75 @@ def test_a_mesh_is_tuned_again_on_its_first_contact_blocks(abi, precond):
     assert (free["tpb"], free["grid"]) == (288, 16)              # and the cluster without
     assert {k: again[k] for k in ("tpb", "grid", "unroll")} == {k: free[k] for k in ("tpb", "grid", "unroll")}
     assert again["tune_ms"] == seen[0]["tune_ms"]
+
+
+def run(abi, n, precond, spacing, index, bending=0.0, frames=2):
+    sc, S, p = scene(abi, n, precond, spacing, index, bending)
+    iters = 0
+    for f in range(frames):
+        S.apply_gravity(sc.gravity, p.dt)
+        iters += S.step(p, sc.pins_at(f), sc.walls)["pcg_iters"]
+    rows = S.last_contact_blocks()[0]
+    width = 7 + int(np.bincount(rows).max()) if len(rows) else 13 if bending else 7
+    out = (*S.download(), iters, S.pcg_shape(precond == "learned"), width)
+    S.close()
+    return out
+
+
+@pytest.mark.parametrize("precond", ["block_jacobi", "learned"])
+@pytest.mark.parametrize("n,spacing,bending,wide", [(22, CLOSE, 0.0, 25), (60, CLOSE, 0.0, 25), (60, 0.003, 1e-5, 13), (276, 0.003, 0.0, 0)])
+def test_every_shape_gives_the_same_bits(abi, n, spacing, bending, wide, precond):
+    """Cluster and grid with contact blocks, wide rows, and the looping form."""
+    x0, v0, it0, shape, width = run(abi, n, precond, spacing, 0, bending)
+    assert it0 > 0 and shape["candidates"] >= 3 and shape["tune_ms"] == 0
+    assert width >= wide        # more of a row's blocks than every candidate keeps on the chip (bending: than the smallest does)
+    used = [(shape["tpb"], shape["grid"], shape["unroll"])]
+    for k in range(1, shape["candidates"]):
+        x, v, it, s, _ = run(abi, n, precond, spacing, k, bending)
+        used.append((s["tpb"], s["grid"], s["unroll"]))
+        assert it == it0
+        np.testing.assert_array_equal(x, x0)
+        np.testing.assert_array_equal(v, v0)
+    assert len(set(used)) >= 3
+
+
+def residual(st, s, d):
+    L = np.linalg.inv(s["M"])
+    y, _ = matvec(s["rows"], s["cols"], s["vals"], np.einsum("vba,vb->va", L, d), s["V"])
+    size, _ = matvec(s["rows"], s["cols"], s["size"], np.einsum("vba,vb->va", np.abs(L), np.abs(d)), s["V"])
+    return np.abs(s["b"] - y).max(), 1e-4 * np.abs(s["b"]).max() + (st["pcg_iters"] + 8) * EPS * size.max()
+
+
+@pytest.mark.parametrize("n,precond", [(11, "learned"), (276, "learned"), (276, "block_jacobi")])
+def test_solution(abi, n, precond):
+    """A curtain the network was not trained for (whichever solve ended it), and the looping form."""
+    st, s, d = solve_step(abi, scenes.c4(n=n, size=2.0 * (n - 1) / 255.0), precond)
+    assert st["pcg_iters"] > 0 and st["pcg_not_converged"] == 0
+    r, bound = residual(st, s, d)
+    assert r <= bound
+
+
+@pytest.mark.parametrize("precond", ["block_jacobi", "learned"])
+def test_a_few_rows_with_very_many_contacts(abi, precond):
+    """A coarse sheet close under a fine one, a coarse vertex in every slice of 32: the contact blocks' copy by slices would be
+    mostly padding, so the solve walks them row by row."""
+    nf, nc, size = 62, 8, 0.3
+    fine, coarse = scenes.grid_plane(nf, size), scenes.grid_plane(nc, size)
+    rng = np.random.default_rng(4)
+    fine[:, :2] = fine[:, :2] * 0.98 + 0.003
+    v = np.concatenate([fine + [0, 0, 0.5 + CLOSE], coarse + [0, 0, 0.5]]) + rng.uniform(-2e-5, 2e-5, (nf * nf + nc * nc, 3))
+    tris = np.concatenate([scenes.grid_triangles(nf, nf), scenes.grid_triangles(nc, nc, offset=nf * nf)])
+    place = np.empty(len(v), int)                       # new index of each vertex
+    place[nf * nf:] = 32 * np.arange(nc * nc) + 5
+    place[:nf * nf] = np.setdiff1d(np.arange(len(v)), place[nf * nf:])
+    x = np.empty_like(v)
+    x[place] = v
+    sc = scenes.c1(n=4)
+    sc.vertices, sc.triangles, sc.walls = x, place[tris].astype(np.int32), []
+    sc.pins = [(int(place[nf * nf]), x[place[nf * nf]].copy())]
+    st, s, d = solve_step(abi, sc, precond)
+    count = np.bincount(s["rows"][len(s["rows"]) - s["contact_blocks"]:], minlength=-(-len(x) // 32) * 32)
+    assert 32 * count.reshape(-1, 32).max(axis=1).sum() > 6 * s["contact_blocks"] + 65536
+    assert st["pcg_iters"] > 0 and st["pcg_not_converged"] == 0
+    r, bound = residual(st, s, d)
+    assert r <= bound
