@@ -964,6 +964,7 @@ __global__ void __launch_bounds__(SCALED_MAX_TPB) k_pcg_scaled(PcgScaledArgs a) 
 // are walked row by row.
 constexpr int RES_KQ = PCG_NEAR_SLOTS;
 constexpr int RES_SMEM = 224 * 1024;   // dynamic shared memory of a CTA, at most
+constexpr int RES_CLUSTER_SLOTS = 72;  // slots of a slice of the cluster form, at most (res_layout)
 // float4 vectors that a CTA of the cluster form publishes in shared memory
 constexpr int res_vectors(bool learned, bool far, int kq) { return (learned ? 4 : 1) + (far || kq == 0 ? 2 : 0); }
 // CTAs of more than 512 threads have no room for the rows' own blocks
@@ -1361,14 +1362,17 @@ int streamed_shapes(int device, int V, bool learned, PcgShape* out, int max) {
 //  - Up to 8,192 rows without contact blocks (1,024 with): one cluster. Its
 //    barriers cost a third of the grid's, but a row of another CTA is read at
 //    an eighth of the local shared-memory rate, which many-block rows or more
-//    rows to a CTA make the longer part.
+//    rows to a CTA make the longer part. A slice as wide as a hub's row is walked
+//    slot by slot, each with a column to turn into an address: on discs about a
+//    hub of 64, 80, 128 and 512 neighbours the cluster takes 16, 24, 49 and 252 us
+//    an iteration, the grid 16, 21, 44 and 194, so wider meshes go to the grid.
 //  - Above: CTAs of 16 slices (8 with contact blocks, whose registers then
 //    hold 24 neighbours' p), so that a small system leaves SMs to other
 //    contexts' solves, and more slices once every SM has a CTA.
-bool res_layout(int V, bool far, bool& cluster, int& ctas, int& spc) {
+bool res_layout(int V, bool far, int wmax, bool& cluster, int& ctas, int& spc) {
   const PcgDevice D = pcg_device();
   const int ns = std::max(1, (V + 31) / 32), sms = std::min(D.sms, XR_MAX_CTAS);
-  cluster = D.cluster && ns <= (far ? 32 : 256);
+  cluster = D.cluster && ns <= (far ? 32 : 256) && wmax <= RES_CLUSTER_SLOTS;
   if (cluster) {
     ctas = 1;
     while (ctas < 16 && ctas * 4 < ns) ctas *= 2;   // four warps to an SM while there are CTAs left
@@ -1385,7 +1389,7 @@ bool res_layout(int V, bool far, bool& cluster, int& ctas, int& spc) {
 
 bool pcg_resident(int V) {
   bool cluster; int ctas, spc;
-  return res_layout(V, true, cluster, ctas, spc) && res_layout(V, false, cluster, ctas, spc);
+  return res_layout(V, true, 1, cluster, ctas, spc) && res_layout(V, false, 1, cluster, ctas, spc);
 }
 
 namespace {
@@ -1396,7 +1400,7 @@ ResPlan res_plan(int V, int wmax, bool contact, bool learned) {
   ResPlan p{};
   p.far = contact || wmax > RES_KQ;
   while (true) {
-    res_layout(V, p.far, p.cluster, p.ctas, p.spc);
+    res_layout(V, p.far, wmax, p.cluster, p.ctas, p.spc);
     p.k = res_kernel(learned, p.far, p.cluster, 32 * p.spc);
     p.near = std::max(wmax - (p.k.compact ? 1 : 0), 1);
     p.pub = p.cluster ? 16 * 32 * p.spc * res_vectors(learned, p.far, p.k.kq) : 0;

@@ -122,3 +122,23 @@ def test_a_few_rows_with_very_many_contacts(abi, precond):
     assert st["pcg_iters"] > 0 and st["pcg_not_converged"] == 0
     r, bound = residual(st, s, d)
     assert r <= bound
+
+
+@pytest.mark.parametrize("m,launch", [(71, (96, 1)), (72, (96, 1)), (200, (224, 1)), (900, (256, 4))])
+def test_a_hub_in_a_small_mesh(abi, m, launch):
+    """A disc of m triangles about one vertex: up to 72 slots one cluster, above the grid's launch."""
+    th = np.linspace(0, 2 * np.pi, m, endpoint=False)
+    sc = scenes.c1(n=4)
+    sc.vertices = np.concatenate([[[0, 0, 1.0]], np.stack([np.cos(th), np.sin(th), np.ones(m)], 1)])
+    i = np.arange(m)
+    sc.triangles = np.stack([np.zeros(m, int), 1 + i, 1 + (i + 1) % m], 1).astype(np.int32)
+    sc.pins, sc.walls = [(0, sc.vertices[0].copy())], []
+    st, s, d = solve_step(abi, sc, "block_jacobi")
+    assert s["width"] == m + 1 and st["pcg_iters"] > 0 and st["pcg_not_converged"] == 0
+    r, bound = residual(st, s, d)
+    assert r <= bound
+    S = abi.Scene(sc.vertices, sc.triangles, sc.material)
+    S.step(abi.make_params(sc.params, semantics="corrected"), sc.pins, [])
+    shape = S.pcg_shape(False)
+    S.close()
+    assert (shape["tpb"], shape["grid"]) == launch
