@@ -1240,9 +1240,11 @@ PcgKernel pcg_kernel(bool one, int warps) {
 struct ResKernel { const void* f; int kq; bool compact; };
 template <bool L, bool F, bool C> ResKernel res_pick(int tpb) {
   constexpr int KW = F ? 24 : RES_KQ;   // 256 threads leave registers for contact blocks' neighbours as well
-  if (tpb <= 256) return {(const void*)k_pcg_res<L, F, C, KW, F ? 8 : RES_KQ, 4, 256>, KW, res_compact(F, 256)};
-  if (tpb <= 512) return {(const void*)k_pcg_res<L, F, C, RES_KQ, 4, L ? 3 : 4, 512>, RES_KQ, res_compact(F, 512)};
-  if constexpr (!C) {   // a cluster's CTAs have at most 512
+  // a grid's CTAs have 16 slices without contact blocks (fewer only where no cluster can be had)
+  if constexpr (F || C) if (tpb <= 256) return {(const void*)k_pcg_res<L, F, C, KW, F ? 8 : RES_KQ, 4, 256>, KW, res_compact(F, 256)};
+  // a cluster's CTAs have at most 16 slices, with contact blocks 4
+  if constexpr (!(F && C)) if (tpb <= 512) return {(const void*)k_pcg_res<L, F, C, RES_KQ, 4, L ? 3 : 4, 512>, RES_KQ, res_compact(F, 512)};
+  if constexpr (!C) {
     if constexpr (!F) if (tpb <= 896) return {(const void*)k_pcg_res<L, F, C, L ? 0 : RES_KQ, 4, L ? 2 : 3, 896>, L ? 0 : RES_KQ, res_compact(F, 896)};
     return {(const void*)k_pcg_res<L, F, C, 0, 1, 2, 1024>, 0, res_compact(F, 1024)};
   }
