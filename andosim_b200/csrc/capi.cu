@@ -557,7 +557,7 @@ int prepare_contacts(ando_ctx c, const StepParams& sp, const double* g_base, con
   ph.launched();
   if (nu && sp.semantics == ANDO_SEMANTICS_CORRECTED && pcg_resident(V)) {
     CK(c->xs_width.reserve((V + 31) / 32)); CK(c->xs_off.reserve((V + 31) / 32 + 1));
-    launch_x_layout(V, c->xbegin.p, c->xend.p, 6ll * nu + 65536, c->xs_width.p, c->xs_off.p, c->ctrl.p, c->stream);
+    launch_x_layout(V, c->xbegin.p, c->xend.p, nu, c->xs_width.p, c->xs_off.p, c->ctrl.p, c->stream);
     ph.launched(2);
   }
   CK(cudaGetLastError());
@@ -940,7 +940,7 @@ int ensure_learned(ando_ctx c) {
 int shape_kind(ando_ctx c) { return c->nx && pcg_resident(c->V) ? 1 : 0; }
 
 int shape_candidates(ando_ctx c, bool learned, int kind, PcgShape (&cand)[16], bool* same) {
-  return pcg_scaled_shapes(c->device, c->V, c->sell_wmax, kind != 0, learned, cand, 16, same);
+  return pcg_scaled_shapes(c->device, c->V, c->sell_wmax, kind != 0, kind != 0 && !c->xs_ready, learned, cand, 16, same);
 }
 
 // Launch shape of the scaled PCG for the current mesh. On the first solve of a

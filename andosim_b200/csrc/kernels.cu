@@ -1056,21 +1056,30 @@ __global__ void k_extra_rows(const K* __restrict__ key, const int* __restrict__ 
 }
 // SELL-32 layout of the merged blocks for the resident PCG: a slice of 32 rows
 // is as wide as its row with the most blocks. The scan of the slice widths is
-// one CTA (a mesh of the resident form has at most 4,736 slices). A layout
-// whose padding would exceed `limit` block places (a few rows with very many
-// contacts) is reported as -1 and not used.
+// one CTA (a mesh of the resident form has at most 4,736 slices). A layout of
+// more than 6 n + 65,536 places for n blocks, or of more than 6 n where a slice is
+// wider than XS_WIDE, is mostly padding behind a few rows with very many contacts:
+// it is reported as -1 and not used, and the solve walks the blocks row by row.
+// us an iteration by the copy and walked, a coarse sheet under a fine one: at 14
+// to 16 places a block (900, 3,900 and 14,700 rows) 360 and 148, 104 and 66, 371
+// and 215, at 6.8 32 and 29, at 4.3 22 and 25. Narrow slices: two sheets of 64^2
+// that touch along a column, 25 places a block, 8.2 and 9.4.
+constexpr int XS_WIDE = 64;
 __global__ void k_x_widths(int V, const int* begin, const int* end, int* width) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = __reduce_max_sync(0xffffffffu, v < V ? end[v] - begin[v] : 0);
   if ((threadIdx.x & 31) == 0 && v < V) width[v >> 5] = n;
 }
-__global__ void __launch_bounds__(1024) k_x_scan(int ns, const int* width, long long limit, int* off, Ctrl* ctrl) {
+__global__ void __launch_bounds__(1024) k_x_scan(int ns, const int* width, long long n, int* off, Ctrl* ctrl) {
   __shared__ long long part[32];
+  const long long limit = 6 * n + 65536;
+  bool wide = false;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   long long carry = 0;
   for (int base = 0; base < ns; base += 1024) {
     const int i = base + threadIdx.x;
     const long long mine = i < ns ? 32ll * width[i] : 0;
+    wide |= mine > 32ll * XS_WIDE;
     long long v = mine;
     for (int o = 1; o < 32; o <<= 1) { const long long u = __shfl_up_sync(0xffffffffu, v, o); if (l >= o) v += u; }
     if (l == 31) part[w] = v;
@@ -1081,7 +1090,8 @@ __global__ void __launch_bounds__(1024) k_x_scan(int ns, const int* width, long 
     carry += all;
     __syncthreads();
   }
-  if (threadIdx.x == 0) { off[ns] = int(min(carry, limit)); ctrl->xs_blocks = carry <= limit ? int(carry) : -1; }
+  wide = __syncthreads_or(wide);
+  if (threadIdx.x == 0) { off[ns] = int(min(carry, limit)); ctrl->xs_blocks = carry <= (wide ? 6 * n : limit) ? int(carry) : -1; }
 }
 // The entries of a block merge into one: the FP64 sum of the per-contact blocks
 // in contact order, each value below barrier_tol dropped on its own. With Linv
@@ -1555,9 +1565,9 @@ template void launch_extra_entries(const ContactRec*, const int*, int, int, unsi
 template void launch_extra_entries(const ContactRec*, const int*, int, int, unsigned long long*, int*, cudaStream_t);
 template void launch_extra_rows(const unsigned*, const int*, int, int, int*, int*, cudaStream_t);
 template void launch_extra_rows(const unsigned long long*, const int*, int, int, int*, int*, cudaStream_t);
-void launch_x_layout(int V, const int* begin, const int* end, long long limit, int* width, int* off, Ctrl* ctrl, cudaStream_t s) {
+void launch_x_layout(int V, const int* begin, const int* end, int n, int* width, int* off, Ctrl* ctrl, cudaStream_t s) {
   k_x_widths<<<nblk(V), TPB, 0, s>>>(V, begin, end, width);
-  k_x_scan<<<1, 1024, 0, s>>>((V + 31) / 32, width, limit, off, ctrl);
+  k_x_scan<<<1, 1024, 0, s>>>((V + 31) / 32, width, n, off, ctrl);
 }
 void launch_extra_merge(const ContactRec* recs, const int* id, const int* heads, const int* xrow, const int* xcols, int nu, int n,
                         const unsigned char* fixed, const StepParams& p, const double* Linv, float* xval, float* xvalh, cudaStream_t s, XsLayout xs) {

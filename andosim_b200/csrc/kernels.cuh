@@ -71,8 +71,8 @@ void launch_extra_rows(const K* key, const int* heads, int nu, int bits, int* xr
 // (32 x width), columns (-1: padding, set by the caller) and 9 planes of 32
 // lanes per slot; begin = first block of each row
 struct XsLayout { const int* off = nullptr; const int* begin = nullptr; int* col = nullptr; float* val = nullptr; };
-// its slice widths and offsets; ctrl->xs_blocks = places in all, -1 when over `limit`
-void launch_x_layout(int V, const int* begin, const int* end, long long limit, int* width, int* off, Ctrl* ctrl, cudaStream_t s);
+// the slice widths and offsets for n blocks; ctrl->xs_blocks = places in all, -1 for a layout not worth it
+void launch_x_layout(int V, const int* begin, const int* end, int n, int* width, int* off, Ctrl* ctrl, cudaStream_t s);
 void launch_extra_merge(const ContactRec* recs, const int* id, const int* heads, const int* xrow, const int* xcols, int nu, int n,
                         const unsigned char* fixed, const StepParams& p, const double* Linv, float* xval, float* xvalh, cudaStream_t s,
                         XsLayout xs = XsLayout{});
@@ -166,7 +166,7 @@ struct PcgShape { int tpb = 0, grid = 0, unroll = 1; };
 size_t pcg_scaled_partials(int V);
 bool pcg_resident(int V);   // the scaled PCG of V rows runs in its resident form (reads xs_*)
 constexpr int PCG_NEAR_SLOTS = 7;   // static slots of a row whose neighbours' p the resident form keeps itself
-int pcg_scaled_shapes(int device, int V, int wmax, bool contact, bool learned, PcgShape* out, int max, bool* same);
+int pcg_scaled_shapes(int device, int V, int wmax, bool contact, bool walked, bool learned, PcgShape* out, int max, bool* same);
 cudaError_t launch_pcg_scaled(const PcgScaledArgs& a, bool learned, const PcgShape& sh, cudaStream_t s);
 cudaError_t launch_pcg(const PcgArgs& a, cudaStream_t s);
 

@@ -1367,7 +1367,8 @@ int streamed_shapes(int device, int V, bool learned, PcgShape* out, int max) {
 //    rows to a CTA make the longer part. A slice as wide as a hub's row is walked
 //    slot by slot, each with a column to turn into an address: on discs about a
 //    hub of 64, 80, 128 and 512 neighbours the cluster takes 16, 24, 49 and 252 us
-//    an iteration, the grid 16, 21, 44 and 194, so wider meshes go to the grid.
+//    an iteration, the grid 16, 21, 44 and 194, so wider meshes go to the grid, and
+//    so do contact blocks that are walked row by row (rows of 680 blocks: 209 and 148).
 //  - Above: CTAs of 16 slices (8 with contact blocks, whose registers then
 //    hold 24 neighbours' p), so that a small system leaves SMs to other
 //    contexts' solves, and more slices once every SM has a CTA.
@@ -1398,8 +1399,9 @@ namespace {
 // The resident launch of a system. far: contact blocks, rows of more than RES_KQ
 // slots, or blocks that do not all fit on the chip.
 struct ResPlan { ResKernel k; bool far, cluster; int ctas, spc, pub, near; };
-ResPlan res_plan(int V, int wmax, bool contact, bool learned) {
+ResPlan res_plan(int V, int wmax, bool contact, bool walked, bool learned) {
   ResPlan p{};
+  if (walked) wmax = std::max(wmax, RES_CLUSTER_SLOTS + 1);
   p.far = contact || wmax > RES_KQ;
   while (true) {
     res_layout(V, p.far, wmax, p.cluster, p.ctas, p.spc);
@@ -1413,15 +1415,15 @@ ResPlan res_plan(int V, int wmax, bool contact, bool learned) {
 }  // namespace
 
 // Candidate launch shapes of the scaled PCG for V rows of at most wmax slots,
-// with or without contact blocks, on `device`; shape 0 is the default. Every
+// with or without contact blocks (walked: row by row), on `device`; shape 0 is the default. Every
 // shape gives the same result bits. The resident form's CTAs and warps follow
 // from those three; its candidates are the shared memory (KiB) for the blocks of
 // a system that does not fit whole: all of it, or less, which leaves more to the
 // L1 for the gathers. *same: the system fits, and they are one launch.
-int pcg_scaled_shapes(int device, int V, int wmax, bool contact, bool learned, PcgShape* out, int max, bool* same) {
+int pcg_scaled_shapes(int device, int V, int wmax, bool contact, bool walked, bool learned, PcgShape* out, int max, bool* same) {
   *same = false;
   if (!pcg_resident(V)) return streamed_shapes(device, V, learned, out, max);
-  const ResPlan p = res_plan(V, wmax, contact, learned);
+  const ResPlan p = res_plan(V, wmax, contact, walked, learned);
   *same = !p.far;
   int n = 0;
   for (int kb : {RES_SMEM / 1024, 160, 96})
@@ -1436,7 +1438,7 @@ cudaError_t launch_pcg_scaled(const PcgScaledArgs& args, bool learned, const Pcg
   PcgScaledArgs a = args;
   void* p[] = {(void*)&a};
   if (!pcg_resident(a.V)) return cudaLaunchCooperativeKernel((void*)scaled_kernel(learned, sh.unroll), dim3(sh.grid), dim3(sh.tpb), p, 0, s);
-  const ResPlan q = res_plan(a.V, a.wmax, a.xbegin != nullptr, learned);
+  const ResPlan q = res_plan(a.V, a.wmax, a.xbegin != nullptr, a.xbegin && !a.xs_off, learned);
   const int room = std::max(std::min(sh.unroll * 1024, RES_SMEM) - q.pub - 128 * q.spc, 0);
   a.slots = q.far ? std::min(room / (1280 * q.spc), 64) : q.near;
   const int smem = q.pub + q.spc * res_warp_bytes(a.slots);
