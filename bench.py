@@ -170,25 +170,12 @@ class ClockSampler:
 
 
 # --------------------------------------------------------------------- ours
-def pcg_bytes(V, nnzb, prof):
-    """Algorithmic bytes of the scaled PCG over the profiled frames.
-
-    Per block-Jacobi iteration (CG on the scaled system, identity diagonal):
-      phase A  40 nnzb (scaled BSR values + column) + 40 per contact block
-               outside the mesh pattern, 12 V each for z, p_old (gathered
-               once), p_new and Ap
-      phase B  12 V p, 24 V x^ read+write (FP64), 12 V Ap, 24 V r read+write,
-               24 V L (FP32, residual norm)
-      = 40 nnzb + 40 n_extra + 144 V
-    A learned iteration adds the second product z = S r on the mesh pattern,
-    applied as S_ij = coef_ij A^_ij plus S's diagonal blocks:
-      + 44 nnzb (A^ values, column, coefficient) + 36 V (diagonal blocks)
-      + 24 V (r2, z written) + 12 V (Ap gathered)
-    plus 48 V per launch (initialisation and d = L^-T x^)."""
-    it = prof["pcg_iterations"]
-    lit = prof["pcg_learned_iterations"]
-    return (40 * nnzb + 144 * V) * it + 40 * prof["pcg_extra_block_iterations"] + (44 * nnzb + 72 * V) * lit \
-        + 48 * V * prof["phase_launches"]["pcg"]
+def pcg_dram_bytes(V, nnzb):
+    """Bytes that one learned solve of the resident PCG reads from memory; its iterations find everything on the chip.
+      the scaled blocks and their columns (40) and the coefficients of S (4)                    = 44 nnzb
+      b^ (12), the diagonal blocks of S (36) and L^-1 (FP64, 48) of a vertex                     = 96 V
+    (the solution and the published vectors, written, stay in L2)."""
+    return 44 * nnzb + 96 * V
 
 
 def assembly_bytes(V, nnzb, learned=True):
@@ -204,11 +191,13 @@ def assembly_bytes(V, nnzb, learned=True):
 
 
 # DRAM bytes (read + write) per launch of the kernel on this workload, from one ncu capture (the summaries
-# under profiles/ give the command): the PCG's matrix and vectors come from DRAM once per launch and from L2
-# for every later iteration (captured on the looping form; the resident form reads the same once per launch and
-# has no capture of its own); the assembly's figure is k_diag_factor plus k_assemble_scaled_slice (44.9 + 27.9 MB).
-PCG_TRAFFIC = 53_985_536
+# under profiles/ give the command): the resident PCG's learned solve, whatever its number of iterations;
+# k_diag_factor plus k_assemble_scaled_slice (44.9 + 27.9 MB).
+PCG_TRAFFIC = 53_516_288
 ASSEMBLY_TRAFFIC = 72_798_720
+# Two of the PCG's reductions over 148 CTAs of 896 threads with nothing between them (us): an iteration has two,
+# each waiting for every row's part of the one before.
+PCG_REDUCTIONS_US = 4.5
 
 
 class Timer:
@@ -667,14 +656,19 @@ def run_ours(args, rank, world, local, pg):
     source = "measured (MEASURED_PEAKS.json hbm_gbs)" if peaks else "fallback"
     pcg_ms = prof["phase_ms"]["pcg"]
     launches = max(1, prof["phase_launches"]["pcg"])
-    pb = pcg_bytes(V, nnzb, prof)
     roof = None
-    if pcg_ms > 0:
-        achieved = pb / (pcg_ms * 1e-3) / 1e9
-        roof = {"bound": "hbm", "kernel": "k_pcg_res (learned and block-Jacobi launches)", "achieved": round(achieved, 1),
-                "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4), "traffic": PCG_TRAFFIC,
-                "peak_source": source, "bytes_per_launch": int(pb // launches),
-                "launches": int(launches), "avg_launch_us": round(pcg_ms * 1e3 / launches, 2),
+    if pcg_ms > 0 and prof["pcg_iterations"] > 0:
+        # the matrix and the rows' state stay on the chip, so an iteration is bounded by its two dependent
+        # reductions, not by memory; the second figure says how little of the memory's rate it needs
+        us = pcg_ms * 1e3 / prof["pcg_iterations"]
+        solves = max(1, prof["newton_iterations"])
+        dram = pcg_dram_bytes(V, nnzb) * solves / (pcg_ms * 1e-3) / 1e9
+        roof = {"bound": "latency: two grid reductions per iteration", "kernel": "k_pcg_res (learned; block Jacobi where it falls back)",
+                "achieved": round(us, 2), "peak": PCG_REDUCTIONS_US, "unit": "us per iteration (peak: the two reductions alone)",
+                "frac": round(PCG_REDUCTIONS_US / us, 4), "traffic": PCG_TRAFFIC,
+                "dram": {"bytes_per_solve": pcg_dram_bytes(V, nnzb), "achieved_gbs": round(dram, 1), "peak_gbs": hbm,
+                         "frac": round(dram / hbm, 4), "peak_source": source},
+                "launches": int(launches), "avg_solve_us": round(pcg_ms * 1e3 / solves, 2),
                 "pcg_iterations": int(prof["pcg_iterations"]), "share_of_frame": round(pcg_ms / max(sum(prof["phase_ms"].values()), 1e-9), 3)}
     asm_ms = prof["phase_ms"]["assemble"]
     asm_n = max(1, prof["newton_iterations"])
