@@ -12,10 +12,10 @@
 //
 // Pipeline: scene bounds -> 30-bit Morton codes of box centres -> stable radix
 // sort (equal codes stay in index order, so code and index together are unique
-// sorted keys) -> Karras hierarchy (one thread per internal node) -> bottom-up refit in shared
-// memory (cut subtrees, then the nodes above the cut) -> one thread per query with an explicit stack; overlapping
-// leaves are queued per warp and appended in batches, and the pair list is then
-// sorted so its order does not depend on scheduling.
+// sorted keys) -> Karras hierarchy (one thread per internal node) -> boxes in
+// shared memory (cut subtrees, then the nodes above the cut) -> one descent for
+// the 32 queries of a warp, whose hits are queued and appended in batches; the
+// pair list is then sorted so its order does not depend on scheduling.
 #include <atomic>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_reduce.cuh>

@@ -67,7 +67,7 @@ def parse():
                     help="Newton iterations between evaluations of the preconditioner network (8: about once per frame; in "
                          "between, S is rebuilt from each Newton system with the last coefficients)")
     ap.add_argument("--pcg-shape", type=int, default=-1,
-                    help="learned scaled-PCG launch candidate of the timed contexts (-1: autotune on the first solve; "
+                    help="learned scaled-PCG launch candidate of the timed contexts (-1: autotune on the first solves; "
                          "a fixed candidate reproduces one shape, e.g. under a profiler)")
     ap.add_argument("--weights", default=None, help="learned preconditioner weights (.npy); default: the shipped C4 weights")
     ap.add_argument("--c3-frames", type=int, default=60, help="timed frames of the batched 64-scene comparison (0: skip)")

@@ -413,15 +413,16 @@ ANDO_API int32_t ando_last_gradient(ando_ctx ctx, double* gradient, int32_t num_
  * Device pointers: rowptr (num_rows+1), cols (sorted per row), vals (9 floats
  * per block, row-major), rhs (3*num_rows), x (3*num_rows, overwritten) and
  * work (>= 24*num_rows floats, any contents; smaller work buffers are rejected
- * with ANDO_ERR_CAPACITY, as are num_rows > ANDO_NOALLOC_MAX_ROWS). `stream` is a
- * cudaStream_t of `device` (NULL = legacy default stream). Reduction partials
- * and grid-barrier words live in a 16 KiB static device array per device
- * (partials for up to 640 CTAs; the grid is capped there); the call zeroes its
- * control words itself, so nothing has to start at zero.
+ * with ANDO_ERR_CAPACITY, as are num_rows > ANDO_NOALLOC_MAX_ROWS). Nothing
+ * outside these arrays is read. `stream` is a cudaStream_t of `device` (NULL =
+ * legacy default stream). The control block and two sets of 160 reduction slots,
+ * one slot to a CTA (one CTA to an SM), live in a 16 KiB static device array per
+ * device; the call zeroes its control block itself, so nothing has to start at
+ * zero.
  *
- * The first call on a device looks up that array's device address and the
- * kernel's grid size (which may load the module): make it before any stream
- * capture. Calls on one device share the scratch, so overlapping calls (other
+ * The first call on a device looks up that array's device address and what
+ * launches the device takes (which may load the module): make it before any
+ * stream capture. Calls on one device share the scratch, so overlapping calls (other
  * streams or threads without ordering) race; serialise them. With all three
  * outputs NULL the call is asynchronous on `stream` and reports launch errors
  * only: a grid-barrier timeout, a not-SPD stop or reaching max_iters is not
